@@ -39,6 +39,7 @@
 #include <algorithm>
 
 #include "mpm_internal.h"
+#include "mpm_scatter.cuh"
 
 namespace {
 
@@ -113,22 +114,24 @@ template<class T> __device__ __forceinline__ void node3(const AdjArgs<T>& a, con
     }
 }
 
-template<class T> __global__ void k_adj_g2p(AdjArgs<T> a)
+// Per particle: its own adjoints, and the factors of its scatter of v-bar,
+// w (Vt + B'-bar (Z - X)) + G-bar grad w; returns the first node (< 0: none).
+template<class T> __device__ __forceinline__ int64_t adj_g2p_row(const AdjArgs<T>& a, T* row)
 {
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if(p >= a.n) return;
+    if(p >= a.n) return -1;
     const T *aX1 = a.aX1 + 3 * p, *aV1 = a.aV1 + 3 * p, *aB1 = a.aB1 + 9 * p, *aF1 = a.aF1 + 9 * p;
     if(!a.valid[p]) {   // frozen particle: identity
         for(int k = 0; k < 3; k++) { a.aX0[3 * p + k] = aX1[k]; a.aV0[3 * p + k] = aV1[k]; }
         for(int k = 0; k < 9; k++) { a.aB0[9 * p + k] = aB1[k]; a.aF0[9 * p + k] = aF1[k]; }
-        return;
+        return -1;
     }
     const T* X = a.X + 3 * p;
     const T* F = a.F + 9 * p;
     Axis2<T> ax[3];
 #pragma unroll
     for(int k = 0; k < 3; k++) ax[k] = axis2<T>(X[k], (T)a.sp.dmin[k], (T)a.sp.dx[k], (T)a.sp.inv_dx[k]);
-    if(!stencil_ok(a, ax)) { atomicOr(a.flags, MPM_FLAG_DOMAIN); return; }
+    if(!stencil_ok(a, ax)) { atomicOr(a.flags, MPM_FLAG_DOMAIN); return -1; }
     // recompute G = sum v g^T
     T G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for(int q = 0; q < 27; q++) {
@@ -164,12 +167,9 @@ template<class T> __global__ void k_adj_g2p(AdjArgs<T> a)
         T w, g[3], H[9], d[3];
         node3(a, ax, X, q, i, w, g, H, d);
         const T* v = a.gv + 3 * i;
-        T vb[3], u[3], Bd[3], BTv[3];
+        T u[3], Bd[3], BTv[3];
 #pragma unroll
-        for(int r = 0; r < 3; r++) {
-            Bd[r] = aB1[r] * d[0] + aB1[r + 3] * d[1] + aB1[r + 6] * d[2];
-            vb[r] = w * Vt[r] + Gb[r] * g[0] + Gb[r + 3] * g[1] + Gb[r + 6] * g[2] + w * Bd[r];
-        }
+        for(int r = 0; r < 3; r++) Bd[r] = aB1[r] * d[0] + aB1[r + 3] * d[1] + aB1[r + 6] * d[2];
 #pragma unroll
         for(int c = 0; c < 3; c++) {
             u[c] = Gb[3 * c] * v[0] + Gb[3 * c + 1] * v[1] + Gb[3 * c + 2] * v[2];
@@ -179,13 +179,38 @@ template<class T> __global__ void k_adj_g2p(AdjArgs<T> a)
 #pragma unroll
         for(int e = 0; e < 3; e++)
             Xb[e] += s * g[e] + H[3 * e] * u[0] + H[3 * e + 1] * u[1] + H[3 * e + 2] * u[2] - w * BTv[e];
-#pragma unroll
-        for(int r = 0; r < 3; r++) atomicAdd(a.ga + 3 * i + r, vb[r]);
     }
 #pragma unroll
     for(int k = 0; k < 3; k++) a.aX0[3 * p + k] = Xb[k];
 #pragma unroll
     for(int k = 0; k < 9; k++) a.aF0[9 * p + k] = Fb[k];
+    Axis<T> wx[3];
+    int64_t first = 0;
+#pragma unroll
+    for(int e = 0; e < 3; e++) {
+        wx[e].base = ax[e].base;
+#pragma unroll
+        for(int o = 0; o < 3; o++) { wx[e].w[o] = ax[e].w[o]; wx[e].dw[o] = ax[e].dw[o]; }
+        first = first * a.gs[e] + (ax[e].base + MPM_GHOST);
+    }
+    T Bc[9];
+#pragma unroll
+    for(int e = 0; e < 9; e++) Bc[e] = aB1[e];
+    plain::scatter_row<T, 3>(row, wx, X, a.sp.dmin, a.sp.dx, Vt, Bc, Gb, (T)0);
+    return first;
+}
+
+template<class T> __global__ void __launch_bounds__(plain::kScatterThreads) k_adj_g2p(AdjArgs<T> a)
+{
+    __shared__ plain::ScatterWarp<T, 3> SW[plain::kScatterThreads / 32];
+    plain::ScatterWarp<T, 3>& S = SW[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    S.base[lane] = adj_g2p_row<T>(a, S.row[lane]);
+    __syncwarp();
+    plain::scatter_warp<T, 3, false>(S, (int64_t)a.gs[1] * a.gs[2], a.gs[2], [&](int64_t i, const T* q) {
+#pragma unroll
+        for(int r = 0; r < 3; r++) atomicAdd(a.ga + 3 * i + r, q[r]);
+    });
 }
 
 // The adjoint of a node's collision projection C(u): replay the projections
@@ -636,7 +661,7 @@ template<class T> static int backward_t(mpm_handle* h, const void* gX, const voi
     MPM_CUDA(h, cudaMemcpyAsync(a1 + 15 * n, gB, 9 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemsetAsync(t->amu, 0, n * e, h->stream));
     MPM_CUDA(h, cudaMemsetAsync(t->alam, 0, n * e, h->stream));
-    const int tb = 128;
+    const int tb = plain::kScatterThreads;
     // a full tape is one segment, recorded by the forward; otherwise each
     // checkpoint's segment is recomputed from it, keeping what the adjoint needs
     const int nck = t->full ? 1 : (t->nsteps + every - 1) / every;

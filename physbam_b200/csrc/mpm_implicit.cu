@@ -26,6 +26,7 @@
 
 #include "mpm_internal.h"
 #include "mpm_plain.cuh"
+#include "mpm_scatter.cuh"
 
 namespace {
 
@@ -209,50 +210,49 @@ template<class T, int d> __global__ void k_imp_precompute(ImpArgs<T> ia)
 
 // MPM_FINITE_ELEMENTS::Add_Forces (l.84-99) + MPM_GRAVITY::Add_Forces (l.62-68)
 // + the penalty forces of MPM_EXAMPLE::Add_Forces (MPM_EXAMPLE.cpp:139-153).
-template<class T, int d> __global__ void k_imp_forces(ImpArgs<T> ia, T* f)
+template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_imp_forces(ImpArgs<T> ia, T* f)
 {
     const PlainArgs<T>& a = ia.a;
+    __shared__ ScatterWarp<T, d> SW[kScatterThreads / 32];
+    ScatterWarp<T, d>& S = SW[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if(t >= a.n) return;
-    const int64_t p = particle_at(ia, t);
-    if(!a.valid[p]) return;
-    Stencil<T, d> s;
-    if(!make_stencil<T, d>(a, ia.X0 + p * d, s)) return;
-    T A[9];
+    int64_t first = -1;
+    if(t < a.n) {
+        const int64_t p = particle_at(ia, t);
+        Stencil<T, d> s;
+        if(a.valid[p] && make_stencil<T, d>(a, ia.X0 + p * d, s)) {
+            first = first_node<T, d>(a, s);
+            T A[d * d], c[d];
+            const T vol = a.vol[p], mp = a.mass[p];
 #pragma unroll
-    for(int e = 0; e < d * d; e++) A[e] = a.pft[p * d * d + e] * a.vol[p];
-    const T mp = a.mass[p];
-    T fp[3] = {0, 0, 0};
-    if(a.sp.npen)
-        for(int e = 0; e < d; e++) fp[e] = ia.pen[p * (d + d * d) + e];
-    const int nq = d == 3 ? 27 : 9;
-    for(int q = 0; q < nq; q++) {
-        int64_t i;
-        T w, g[3], Z[3];
-        node<T, d>(a, s, q, i, w, g, Z);
+            for(int e = 0; e < d * d; e++) A[e] = -a.pft[p * d * d + e] * vol;
 #pragma unroll
-        for(int r = 0; r < d; r++) {
-            T sum = 0;
-#pragma unroll
-            for(int c = 0; c < d; c++) sum += A[r + d * c] * g[c];
-            atomicAdd(f + i * d + r, -sum + w * mp * (T)a.sp.gravity[r] + w * fp[r]);
+            for(int e = 0; e < d; e++) c[e] = mp * (T)a.sp.gravity[e] + (a.sp.npen ? ia.pen[p * (d + d * d) + e] : (T)0);
+            scatter_row<T, d>(S.row[lane], s.ax, ia.X0 + p * d, a.sp.dmin, a.sp.dx, c, nullptr, A, (T)0);
         }
     }
+    S.base[lane] = first;
+    __syncwarp();
+    scatter_warp<T, d, false>(S, node_stride(a, d, 0), node_stride(a, d, 1), [&](int64_t i, const T* q) {
+#pragma unroll
+        for(int k = 0; k < d; k++) atomicAdd(f + i * d + k, q[k]);
+    });
 }
 
 // MPM_FINITE_ELEMENTS::Add_Hessian_Times (l.103-132): W = sum z_i grad w_i^T,
 // M = U dPhat(U^T W FV) FV^T vol, f_i += M grad w_i; with penalty objects also
 // MPM_EXAMPLE::Add_Hessian_Times' Lagrangian part (MPM_EXAMPLE.cpp:157-177):
 // z_p = sum w_i z_i, f_i += w_i H_p z_p.
-template<class T, int d> __global__ void k_imp_hessian(ImpArgs<T> ia, const T* z, T* f)
+template<class T, int d> __device__ __forceinline__ int64_t hessian_row(const ImpArgs<T>& ia, const T* z, T* row)
 {
     const PlainArgs<T>& a = ia.a;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if(t >= a.n) return;
+    if(t >= a.n) return -1;
     const int64_t p = particle_at(ia, t);
-    if(!a.valid[p]) return;
+    if(!a.valid[p]) return -1;
     Stencil<T, d> s;
-    if(!make_stencil<T, d>(a, ia.X0 + p * d, s)) return;
+    if(!make_stencil<T, d>(a, ia.X0 + p * d, s)) return -1;
     T W[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, zp[3] = {0, 0, 0};
     const bool pen = a.sp.npen != 0;
     const int nq = d == 3 ? 27 : 9;
@@ -320,18 +320,22 @@ template<class T, int d> __global__ void k_imp_hessian(ImpArgs<T> ia, const T* z
             for(int k = 0; k < d; k++) sum += UD[r + d * k] * FV[c + d * k];
             M[r + d * c] = sum * vol;
         }
-    for(int q = 0; q < nq; q++) {
-        int64_t i;
-        T w, g[3], Z[3];
-        node<T, d>(a, s, q, i, w, g, Z);
+    scatter_row<T, d>(row, s.ax, ia.X0 + p * d, a.sp.dmin, a.sp.dx, Hz, nullptr, M, (T)0);
+    return first_node<T, d>(a, s);
+}
+
+template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_imp_hessian(ImpArgs<T> ia, const T* z, T* f)
+{
+    const PlainArgs<T>& a = ia.a;
+    __shared__ ScatterWarp<T, d> SW[kScatterThreads / 32];
+    ScatterWarp<T, d>& S = SW[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    S.base[lane] = hessian_row<T, d>(ia, z, S.row[lane]);
+    __syncwarp();
+    scatter_warp<T, d, false>(S, node_stride(a, d, 0), node_stride(a, d, 1), [&](int64_t i, const T* q) {
 #pragma unroll
-        for(int r = 0; r < d; r++) {
-            T sum = 0;
-#pragma unroll
-            for(int c = 0; c < d; c++) sum += M[r + d * c] * g[c];
-            atomicAdd(f + i * d + r, sum + w * Hz[r]);
-        }
-    }
+        for(int k = 0; k < d; k++) atomicAdd(f + i * d + k, q[k]);
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -656,7 +660,7 @@ template<class T, int d> struct Solver {
         ia.order = nullptr;
         for(int k = 0; k < V_COUNT; k++) v[k] = (T*)s.vec + (size_t)k * s.gn * d;
         ia.svel = v[V_SVEL];
-        pb = pblocks(s.n, 128);
+        pb = pblocks(s.n, kScatterThreads);
         gb = gblocks(h, s.gn, 256);
     }
     static int pblocks(int64_t n, int t) { int64_t b = (n + t - 1) / t; return (int)(b < 1 ? 1 : b); }
@@ -720,7 +724,7 @@ template<class T, int d> struct Solver {
         if(e) *e = energy(dv);
         if(g) {
             zero(v[V_TMP2]);
-            k_imp_forces<T, d><<<pb, 128, 0, st>>>(ia, v[V_TMP2]);
+            k_imp_forces<T, d><<<pb, kScatterThreads, 0, st>>>(ia, v[V_TMP2]);
             k_imp_grad<T, d><<<gb, 256, 0, st>>>(ia, g, dv, v[V_TMP2]);
         }
         check("compute_unconstrained");
@@ -740,7 +744,7 @@ template<class T, int d> struct Solver {
     {
         k_imp_mult_pre<T, d><<<gb, 256, 0, st>>>(ia, v[V_STMP], x);
         zero(out);
-        k_imp_hessian<T, d><<<pb, 128, 0, st>>>(ia, v[V_STMP], out);
+        k_imp_hessian<T, d><<<pb, kScatterThreads, 0, st>>>(ia, v[V_STMP], out);
         k_imp_mult_post<T, d><<<gb, 256, 0, st>>>(ia, out, v[V_STMP], x);
     }
 

@@ -12,6 +12,7 @@
 
 #include "mpm_internal.h"
 #include "mpm_plain.cuh"
+#include "mpm_scatter.cuh"
 
 namespace {
 
@@ -33,38 +34,38 @@ template<class T> __global__ void k_clear(PlainArgs<T> a)
     }
 }
 
-// MPM_DRIVER::Particle_To_Grid scatter (MPM_DRIVER.cpp:259-271).
-template<class T, int d> __global__ void k_p2g(PlainArgs<T> a)
+// MPM_DRIVER::Particle_To_Grid scatter (MPM_DRIVER.cpp:259-271): mass and
+// momentum w m (V + B Dp^-1 (Z - X)).
+template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_p2g(PlainArgs<T> a)
 {
-    int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if(p >= a.n || !a.valid[p]) return;
-    const T* X = a.X + p * d;
-    Stencil<T, d> s;
-    if(!make_stencil<T, d>(a, X, s)) { atomicOr(a.flags, MPM_FLAG_DOMAIN); return; }
-    T Dp_inv[3];
+    __shared__ ScatterWarp<T, d> W[kScatterThreads / 32];
+    ScatterWarp<T, d>& S = W[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int64_t first = -1;
+    if(p < a.n && a.valid[p]) {
+        Stencil<T, d> s;
+        if(make_stencil<T, d>(a, a.X + p * d, s)) {
+            first = first_node<T, d>(a, s);
+            const T mp = a.mass[p];
+            T c[d], K[d * d];
 #pragma unroll
-    for(int k = 0; k < d; k++) Dp_inv[k] = 4 * (T)a.sp.inv_dx[k] * (T)a.sp.inv_dx[k];
-    const T* Bp = a.B + p * d * d;
-    T mp = a.mass[p];
-    const int nq = d == 3 ? 27 : 9;
-    for(int q = 0; q < nq; q++) {
-        int64_t i;
-        T w, g[3], Z[3];
-        node<T, d>(a, s, q, i, w, g, Z);
-        atomicAdd(a.gm + i, w * mp);
-        T Vn[3], Y[3];
+            for(int k = 0; k < d; k++) {
+                c[k] = mp * a.V[p * d + k];
+                const T D = 4 * (T)a.sp.inv_dx[k] * (T)a.sp.inv_dx[k] * mp;
 #pragma unroll
-        for(int k = 0; k < d; k++) { Vn[k] = w * a.V[p * d + k]; Y[k] = (Z[k] - X[k]) * Dp_inv[k]; }
-#pragma unroll
-        for(int r = 0; r < d; r++) {
-            T sum = 0;
-#pragma unroll
-            for(int c = 0; c < d; c++) sum += Bp[r + d * c] * Y[c];
-            Vn[r] += sum * w;
-        }
-#pragma unroll
-        for(int k = 0; k < d; k++) atomicAdd(a.gmv + i * d + k, mp * Vn[k]);
+                for(int r = 0; r < d; r++) K[r + d * k] = a.B[p * d * d + r + d * k] * D;
+            }
+            scatter_row<T, d>(S.row[lane], s.ax, a.X + p * d, a.sp.dmin, a.sp.dx, c, K, nullptr, mp);
+        } else atomicOr(a.flags, MPM_FLAG_DOMAIN);
     }
+    S.base[lane] = first;
+    __syncwarp();
+    scatter_warp<T, d, true>(S, node_stride(a, d, 0), node_stride(a, d, 1), [&](int64_t i, const T* q) {
+        atomicAdd(a.gm + i, q[d]);
+#pragma unroll
+        for(int k = 0; k < d; k++) atomicAdd(a.gmv + i * d + k, q[k]);
+    });
 }
 
 // v = mv / m on nodes with mass (MPM_DRIVER.cpp:282-305).
@@ -93,34 +94,35 @@ template<class T, int d> __global__ void k_stress(PlainArgs<T> a)
 // MPM_FINITE_ELEMENTS::Add_Forces (MPM_FINITE_ELEMENTS.cpp:84-99),
 // MPM_GRAVITY::Add_Forces (MPM_GRAVITY.cpp:62-68) and the penalty collision
 // forces of Apply_Particle_Forces (MPM_DRIVER.cpp:933-945) in one pass.
-template<class T, int d> __global__ void k_forces(PlainArgs<T> a)
+template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_forces(PlainArgs<T> a)
 {
-    int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if(p >= a.n || !a.valid[p]) return;
-    Stencil<T, d> s;
-    if(!make_stencil<T, d>(a, a.X + p * d, s)) return;
-    T A[9];
+    __shared__ ScatterWarp<T, d> W[kScatterThreads / 32];
+    ScatterWarp<T, d>& S = W[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int64_t first = -1;
+    if(p < a.n && a.valid[p]) {
+        Stencil<T, d> s;
+        if(make_stencil<T, d>(a, a.X + p * d, s)) {
+            first = first_node<T, d>(a, s);
+            T A[d * d], c[3] = {0, 0, 0};
+            const T vol = a.vol[p], mp = a.mass[p];
 #pragma unroll
-    for(int e = 0; e < d * d; e++) A[e] = a.pft[p * d * d + e] * a.vol[p];
-    T mp = a.mass[p];
-    T fp[3] = {0, 0, 0};   // the particle's penalty force
-    if(a.sp.npen)
-        penalty_particle<T, d>(a.sp.pen, a.sp.npen, (T)a.sp.pen_stiffness, (T)a.sp.pen_separation, a.X + p * d, fp,
-                               (T*)nullptr);
-    const int nq = d == 3 ? 27 : 9;
-    for(int q = 0; q < nq; q++) {
-        int64_t i;
-        T w, g[3], Z[3];
-        node<T, d>(a, s, q, i, w, g, Z);
-        T wm = w * mp;
+            for(int e = 0; e < d * d; e++) A[e] = -a.pft[p * d * d + e] * vol;
+            if(a.sp.npen)   // the particle's penalty force
+                penalty_particle<T, d>(a.sp.pen, a.sp.npen, (T)a.sp.pen_stiffness, (T)a.sp.pen_separation, a.X + p * d, c,
+                                       (T*)nullptr);
 #pragma unroll
-        for(int r = 0; r < d; r++) {
-            T sum = 0;
-#pragma unroll
-            for(int c = 0; c < d; c++) sum += A[r + d * c] * g[c];
-            atomicAdd(a.gf + i * d + r, -sum + wm * (T)a.sp.gravity[r] + w * fp[r]);
+            for(int k = 0; k < d; k++) c[k] += mp * (T)a.sp.gravity[k];
+            scatter_row<T, d>(S.row[lane], s.ax, a.X + p * d, a.sp.dmin, a.sp.dx, c, nullptr, A, (T)0);
         }
     }
+    S.base[lane] = first;
+    __syncwarp();
+    scatter_warp<T, d, false>(S, node_stride(a, d, 0), node_stride(a, d, 1), [&](int64_t i, const T* q) {
+#pragma unroll
+        for(int k = 0; k < d; k++) atomicAdd(a.gf + i * d + k, q[k]);
+    });
 }
 
 // Apply_Forces grid update: dv = dt/m f, collision projection, friction,
@@ -438,7 +440,7 @@ template<class T> int reflect_pass(mpm_handle* h, const PlainArgs<T>& a, Reflect
 template<class T> int p2g_t(mpm_handle* h, double dt)
 {
     PlainArgs<T> a = args<T>(h, dt);
-    const int t = 128;
+    const int t = kScatterThreads;
     int slot = timer_begin(h, "plain_clear");
     k_clear<T><<<gblocks(h, a.gn, t), t, 0, h->stream>>>(a);
     timer_end(h, slot);
@@ -464,7 +466,7 @@ template<class T> int p2g_t(mpm_handle* h, double dt)
 template<class T> int forces_t(mpm_handle* h, double dt)
 {
     PlainArgs<T> a = args<T>(h, dt);
-    const int t = 128;
+    const int t = kScatterThreads;
     if(a.n) {
         int slot = timer_begin(h, "plain_stress");
         if(h->sp.dim == 3) k_stress<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);

@@ -82,6 +82,22 @@ template<class T, int d> __device__ __forceinline__ void node(const PlainArgs<T>
     }
 }
 
+// Flat index of a stencil's first node, and the flat strides of axes 0 and 1.
+template<class T, int d> __device__ __forceinline__ int64_t first_node(const PlainArgs<T>& a, const Stencil<T, d>& s)
+{
+    int64_t flat = 0;
+#pragma unroll
+    for(int k = 0; k < d; k++) flat = flat * a.gs[k] + (s.base[k] + MPM_GHOST);
+    return flat;
+}
+
+template<class T> __device__ __forceinline__ int64_t node_stride(const PlainArgs<T>& a, int d, int axis)
+{
+    int64_t n = 1;
+    for(int k = axis + 1; k < d; k++) n *= a.gs[k];
+    return n;
+}
+
 template<class T> inline PlainArgs<T> args(mpm_handle* h, double dt)
 {
     PlainArgs<T> a;
