@@ -534,8 +534,7 @@ template<class T> static int record_substep(mpm_handle* h, DiffTape* t, int j, b
     const size_t e = sizeof(T), st = 24 * n * e;
     int rc;
     if((rc = state_copy(h, (char*)t->seg + j * st, t->seg_valid + j * n, true))) return rc;
-    if((rc = plain_p2g(h, t->dt, 0))) return rc;
-    if((rc = plain_forces(h, t->dt, 0))) return rc;
+    if((rc = plain_p2g_forces(h, t->dt))) return rc;
     MPM_CUDA(h, cudaMemcpyAsync((T*)t->seg_gm + j * gn, s.gm, gn * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync((T*)t->seg_gv + j * gn * 3, s.gv, gn * 3 * e, cudaMemcpyDeviceToDevice, h->stream));
     k_grid_u<T><<<blocks_for(h, gn, 256, true), 256, 0, h->stream>>>((const T*)s.gv0, (const T*)s.gf, (const T*)s.gm,
@@ -623,8 +622,7 @@ int diff_forward(mpm_handle* h, double dt, int nsteps, int every)
             int c = k / every;
             if((rc = state_copy(h, (char*)t->ckpt + c * st, t->ckpt_valid + c * s.n, true))) return rc;
         }
-        if((rc = plain_p2g(h, dt, 0))) return rc;
-        if((rc = plain_forces(h, dt, 0))) return rc;
+        if((rc = plain_p2g_forces(h, dt))) return rc;
         if((rc = plain_g2p(h, dt, 0))) return rc;
     }
     if((rc = state_copy(h, t->final_state, t->final_valid, true))) return rc;

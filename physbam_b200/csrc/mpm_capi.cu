@@ -214,8 +214,14 @@ static bool reduces_dt(const mpm_handle* h) { return h->dt_control.strong_cfl ||
 // Advance_One_Time_Step: p2g, forces, Reduce_Dt (plain path, when asked), g2p
 static int enqueue_substep(mpm_handle* h, double dt, double time)
 {
-    int rc = mpm_particle_to_grid(h, dt, time);
-    if(!rc) rc = mpm_apply_forces(h, dt, time);
+    int rc;
+    if(!fast(h) && !h->implicit.enabled) {   // plain explicit: both phases' scatters in one pass
+        rc = update_motion(h, time, dt);
+        if(!rc) rc = plain_p2g_forces(h, dt);
+    } else {
+        rc = mpm_particle_to_grid(h, dt, time);
+        if(!rc) rc = mpm_apply_forces(h, dt, time);
+    }
     double taken = dt;
     if(!rc && !fast(h) && reduces_dt(h)) rc = plain_reduce_dt(h, dt, &taken);
     if(!rc) rc = mpm_grid_to_particle(h, taken, time);
@@ -231,7 +237,7 @@ static int run_substep(mpm_handle* h, double dt, double time)
     if(h->timing || h->implicit.enabled || (h->moving && !h->motion_from_table) || (!fast(h) && reduces_dt(h)))
         return enqueue_substep(h, dt, time);
     // the fast path's full sort after new particles runs eagerly, never in a graph
-    int prc = fast(h) ? fast_prepare(h) : MPM_OK;
+    int prc = fast(h) ? fast_prepare(h) : plain_prepare(h);
     if(prc) return prc;
     const int par = fast(h) ? h->fast.cur : 0;
     cudaGraphExec_t& ge = h->graphs[par];

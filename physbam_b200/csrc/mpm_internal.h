@@ -30,6 +30,12 @@ struct PlainState {
     void *mass = nullptr, *vol = nullptr, *mu = nullptr, *lam = nullptr, *pft = nullptr;
     uint8_t* valid = nullptr;
     void *gm = nullptr, *gmv = nullptr, *gv0 = nullptr, *gf = nullptr, *gv = nullptr, *gvf = nullptr;
+    // the nodes of the last P2G, in tiles of 32 consecutive ones: a flag per tile, the list of
+    // flagged tiles and its length.  The grid arrays are zero outside the listed tiles
+    // (`grid_listed`); small grids and reflection boundaries run over every node instead.
+    uint8_t* tile_flag = nullptr;
+    uint32_t *tiles = nullptr, *tile_count = nullptr;
+    bool grid_listed = false;
     void *Fp = nullptr, *mu0 = nullptr, *lam0 = nullptr;   // plastic state (plasticity on): clamp
     void *pdef = nullptr, *rhoF = nullptr, *sigY = nullptr, *vc = nullptr;   // Drucker-Prager
     uint8_t* pmodel = nullptr;   // per-particle constitutive model (null: the handle's model)
@@ -211,7 +217,9 @@ int plain_alloc(mpm_handle* h, int64_t n);
 void plain_free(mpm_handle* h);
 int plain_set_particles(mpm_handle* h, const mpm_particles_view* v);
 int plain_get_particles(mpm_handle* h, mpm_particles_view* v);
+int plain_prepare(mpm_handle* h);
 int plain_p2g(mpm_handle* h, double dt, double time);
+int plain_p2g_forces(mpm_handle* h, double dt);
 int plain_forces(mpm_handle* h, double dt, double time);
 int plain_g2p(mpm_handle* h, double dt, double time);
 int plain_get_grid(mpm_handle* h, double* m, double* v0, double* v, double* vf);

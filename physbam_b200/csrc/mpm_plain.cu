@@ -22,29 +22,94 @@ using namespace plain;
 template<class T> struct Vec4 { T v[4]; };
 template<class T> struct Vec5 { T v[5]; };
 
-template<class T> __global__ void k_clear(PlainArgs<T> a)
+template<class T> __device__ __forceinline__ void clear_node(const PlainArgs<T>& a, int64_t i)
 {
     const int d = a.sp.dim;
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.gn; i += (int64_t)gridDim.x * blockDim.x) {
-        a.gm[i] = 0;
-        for(int k = 0; k < d; k++) {
-            a.gmv[i * d + k] = 0; a.gf[i * d + k] = 0; a.gv0[i * d + k] = 0;
-            a.gv[i * d + k] = 0; a.gvf[i * d + k] = 0;
-        }
+    a.gm[i] = 0;
+    for(int k = 0; k < d; k++) {
+        a.gmv[i * d + k] = 0; a.gf[i * d + k] = 0; a.gv0[i * d + k] = 0;
+        a.gv[i * d + k] = 0; a.gvf[i * d + k] = 0;
     }
 }
 
+// The grid arrays (and tile flags) of the last P2G's nodes back to zero.
+template<class T> __global__ void k_clear(PlainArgs<T> a)
+{
+    for_nodes(a, [&](int64_t i) {
+        clear_node(a, i);
+        if(a.tile_flag && i % kTileNodes == 0) a.tile_flag[i / kTileNodes] = 0;
+    });
+}
+
+// The flagged tiles in tile order, and their number.  A CTA lists kTileSpan
+// tiles; the flags before its own it counts itself (one byte each, 0 or 1, read
+// as 16-byte words), so the list takes one launch and no CTA waits for another.
+constexpr int kTileSpan = 1024, kTileThreads = 256;
+__global__ void __launch_bounds__(kTileThreads) k_tile_list(const uint8_t* flag, int64_t ntiles, uint32_t* tiles, uint32_t* count)
+{
+    __shared__ uint32_t s_warp[kTileThreads / 32], s_before[kTileThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t first = (int64_t)blockIdx.x * kTileSpan;
+    uint32_t before = 0;
+    const uint4* f16 = reinterpret_cast<const uint4*>(flag);
+    for(int64_t k = threadIdx.x; k < first / 16; k += kTileThreads) {
+        const uint4 v = f16[k];
+        before += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+    }
+    // this CTA's tiles, four per thread (the flags are padded to whole spans)
+    const uint32_t mine = reinterpret_cast<const uint32_t*>(flag + first)[threadIdx.x];
+    const uint32_t c = __popc(mine);
+    uint32_t x = c;
+#pragma unroll
+    for(int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if(lane >= o) x += y;
+    }
+#pragma unroll
+    for(int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if(lane == 31) s_warp[warp] = x;
+    if(lane == 0) s_before[warp] = before;
+    __syncthreads();
+    uint32_t at = x - c, total = 0;
+#pragma unroll
+    for(int w = 0; w < kTileThreads / 32; w++) {
+        at += s_before[w] + (w < warp ? s_warp[w] : 0u);
+        total += s_before[w] + s_warp[w];
+    }
+#pragma unroll
+    for(int k = 0; k < 4; k++)
+        if((mine >> (8 * k)) & 1u) tiles[at++] = (uint32_t)(first + 4 * threadIdx.x + k);
+    if(blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count = total;
+}
+
+// Factors of the particle's forces: MPM_FINITE_ELEMENTS::Add_Forces
+// (MPM_FINITE_ELEMENTS.cpp:84-99), MPM_GRAVITY::Add_Forces (MPM_GRAVITY.cpp:62-68)
+// and the penalty collision forces of Apply_Particle_Forces (MPM_DRIVER.cpp:933-945).
+template<class T, int d> __device__ __forceinline__ void force_row(const PlainArgs<T>& a, int64_t p, const Stencil<T, d>& s, T* row)
+{
+    T A[d * d], c[3] = {0, 0, 0};
+    const T vol = a.vol[p], mp = a.mass[p];
+#pragma unroll
+    for(int e = 0; e < d * d; e++) A[e] = -a.pft[p * d * d + e] * vol;
+    if(a.sp.npen)
+        penalty_particle<T, d>(a.sp.pen, a.sp.npen, (T)a.sp.pen_stiffness, (T)a.sp.pen_separation, a.X + p * d, c, (T*)nullptr);
+#pragma unroll
+    for(int k = 0; k < d; k++) c[k] += mp * (T)a.sp.gravity[k];
+    scatter_row<T, d>(row, s.ax, a.X + p * d, a.sp.dmin, a.sp.dx, c, nullptr, A, (T)0);
+}
+
 // MPM_DRIVER::Particle_To_Grid scatter (MPM_DRIVER.cpp:259-271): mass and
-// momentum w m (V + B Dp^-1 (Z - X)).
-template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_p2g(PlainArgs<T> a)
+// momentum w m (V + B Dp^-1 (Z - X)); FORCES: the forces too (a whole substep
+// then reads the particles and forms their weights once).
+template<class T, int d, bool FORCES> __global__ void __launch_bounds__(kScatterThreads) k_p2g(PlainArgs<T> a)
 {
     __shared__ ScatterWarp<T, d> W[kScatterThreads / 32];
     ScatterWarp<T, d>& S = W[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t first = -1;
+    Stencil<T, d> s;
     if(p < a.n && a.valid[p]) {
-        Stencil<T, d> s;
         if(make_stencil<T, d>(a, a.X + p * d, s)) {
             first = first_node<T, d>(a, s);
             const T mp = a.mass[p];
@@ -61,21 +126,32 @@ template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_p2
     }
     S.base[lane] = first;
     __syncwarp();
-    scatter_warp<T, d, true>(S, node_stride(a, d, 0), node_stride(a, d, 1), [&](int64_t i, const T* q) {
+    const int64_t s0 = node_stride(a, d, 0), s1 = node_stride(a, d, 1);
+    scatter_warp<T, d, true>(S, s0, s1, [&](int64_t i, const T* q) {
         atomicAdd(a.gm + i, q[d]);
 #pragma unroll
         for(int k = 0; k < d; k++) atomicAdd(a.gmv + i * d + k, q[k]);
+        if(a.tile_flag) a.tile_flag[i / kTileNodes] = 1;
     });
+    if(FORCES) {
+        __syncwarp();
+        if(first >= 0) force_row<T, d>(a, p, s, S.row[lane]);
+        __syncwarp();
+        scatter_warp<T, d, false>(S, s0, s1, [&](int64_t i, const T* q) {
+#pragma unroll
+            for(int k = 0; k < d; k++) atomicAdd(a.gf + i * d + k, q[k]);
+        });
+    }
 }
 
 // v = mv / m on nodes with mass (MPM_DRIVER.cpp:282-305).
 template<class T> __global__ void k_normalize(PlainArgs<T> a)
 {
     const int d = a.sp.dim;
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.gn; i += (int64_t)gridDim.x * blockDim.x) {
-        T m = a.gm[i];
+    for_nodes(a, [&](int64_t i) {
+        const T m = a.gm[i];
         for(int k = 0; k < d; k++) a.gv0[i * d + k] = m != 0 ? a.gmv[i * d + k] / m : (T)0;
-    }
+    });
 }
 
 // MPM_FINITE_ELEMENTS::Precompute (MPM_FINITE_ELEMENTS.cpp:47-67).
@@ -91,9 +167,7 @@ template<class T, int d> __global__ void k_stress(PlainArgs<T> a)
     for(int e = 0; e < d * d; e++) a.pft[p * d * d + e] = PFT[e];
 }
 
-// MPM_FINITE_ELEMENTS::Add_Forces (MPM_FINITE_ELEMENTS.cpp:84-99),
-// MPM_GRAVITY::Add_Forces (MPM_GRAVITY.cpp:62-68) and the penalty collision
-// forces of Apply_Particle_Forces (MPM_DRIVER.cpp:933-945) in one pass.
+// The force scatter by itself, for a P2G that did not take it along.
 template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_forces(PlainArgs<T> a)
 {
     __shared__ ScatterWarp<T, d> W[kScatterThreads / 32];
@@ -101,21 +175,10 @@ template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_fo
     const int lane = threadIdx.x & 31;
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t first = -1;
-    if(p < a.n && a.valid[p]) {
-        Stencil<T, d> s;
-        if(make_stencil<T, d>(a, a.X + p * d, s)) {
-            first = first_node<T, d>(a, s);
-            T A[d * d], c[3] = {0, 0, 0};
-            const T vol = a.vol[p], mp = a.mass[p];
-#pragma unroll
-            for(int e = 0; e < d * d; e++) A[e] = -a.pft[p * d * d + e] * vol;
-            if(a.sp.npen)   // the particle's penalty force
-                penalty_particle<T, d>(a.sp.pen, a.sp.npen, (T)a.sp.pen_stiffness, (T)a.sp.pen_separation, a.X + p * d, c,
-                                       (T*)nullptr);
-#pragma unroll
-            for(int k = 0; k < d; k++) c[k] += mp * (T)a.sp.gravity[k];
-            scatter_row<T, d>(S.row[lane], s.ax, a.X + p * d, a.sp.dmin, a.sp.dx, c, nullptr, A, (T)0);
-        }
+    Stencil<T, d> s;
+    if(p < a.n && a.valid[p] && make_stencil<T, d>(a, a.X + p * d, s)) {
+        first = first_node<T, d>(a, s);
+        force_row<T, d>(a, p, s, S.row[lane]);
     }
     S.base[lane] = first;
     __syncwarp();
@@ -126,12 +189,13 @@ template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_fo
 }
 
 // Apply_Forces grid update: dv = dt/m f, collision projection, friction,
-// assembly (MPM_DRIVER.cpp:989-1056, MPM_OBJECTIVE.cpp:150-225).
-template<class T, int d> __global__ void k_grid_update(PlainArgs<T> a)
+// assembly (MPM_DRIVER.cpp:989-1056, MPM_OBJECTIVE.cpp:150-225).  NORMALIZE: v0 =
+// mv / m first, where no k_normalize ran.
+template<class T, int d, bool NORMALIZE> __global__ void k_grid_update(PlainArgs<T> a)
 {
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.gn; i += (int64_t)gridDim.x * blockDim.x) {
+    for_nodes(a, [&](int64_t i) {
         T m = a.gm[i];
-        if(m == 0) continue;
+        if(m == 0) return;
         T dv[3], v0[3], X0[3], vn[3], vf[3];
         T s = a.dt / m;
         int64_t r = i;
@@ -140,13 +204,14 @@ template<class T, int d> __global__ void k_grid_update(PlainArgs<T> a)
 #pragma unroll
         for(int k = 0; k < d; k++) {
             dv[k] = s * a.gf[i * d + k];
-            v0[k] = a.gv0[i * d + k];
+            if(NORMALIZE) a.gv0[i * d + k] = v0[k] = a.gmv[i * d + k] / m;
+            else v0[k] = a.gv0[i * d + k];
             X0[k] = (T)a.sp.dmin[k] + ((T)idx[k] + (T).5) * (T)a.sp.dx[k];
         }
         collide_node<T, d>(a.sp.objs, a.sp.nobj, X0, v0, dv, a.dt, vn, vf, a.motion, a.moving);
 #pragma unroll
         for(int k = 0; k < d; k++) { a.gv[i * d + k] = vn[k]; a.gvf[i * d + k] = vf[k]; }
-    }
+    });
 }
 
 // MPM_DRIVER::Grid_To_Particle (MPM_DRIVER.cpp:450-515) and
@@ -437,8 +502,22 @@ template<class T> int reflect_pass(mpm_handle* h, const PlainArgs<T>& a, Reflect
     return MPM_OK;
 }
 
-template<class T> int p2g_t(mpm_handle* h, double dt)
+template<class T> int stress_t(mpm_handle* h, const PlainArgs<T>& a)
 {
+    const int t = 128, slot = timer_begin(h, "plain_stress");
+    if(h->sp.dim == 3) k_stress<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
+    else k_stress<T, 2><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
+    timer_end(h, slot);
+    MPM_LAUNCHED(h, "k_stress");
+    return MPM_OK;
+}
+
+// with_forces: the forces scattered in the same pass (plain_p2g_forces), the
+// velocities left to the grid update.
+template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
+{
+    int rc = plain_prepare(h);
+    if(rc) return rc;
     PlainArgs<T> a = args<T>(h, dt);
     const int t = kScatterThreads;
     int slot = timer_begin(h, "plain_clear");
@@ -446,16 +525,29 @@ template<class T> int p2g_t(mpm_handle* h, double dt)
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_clear");
     if(a.n) {
+        if(with_forces && (rc = stress_t<T>(h, a))) return rc;
         slot = timer_begin(h, "plain_p2g");
-        if(h->sp.dim == 3) k_p2g<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
-        else k_p2g<T, 2><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
+        const int b = pblocks(a.n, t);
+        if(h->sp.dim == 3) {
+            if(with_forces) k_p2g<T, 3, true><<<b, t, 0, h->stream>>>(a);
+            else k_p2g<T, 3, false><<<b, t, 0, h->stream>>>(a);
+        } else {
+            if(with_forces) k_p2g<T, 2, true><<<b, t, 0, h->stream>>>(a);
+            else k_p2g<T, 2, false><<<b, t, 0, h->stream>>>(a);
+        }
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_p2g");
     }
-    if(a.reflect && !h->reflect.full_reflection) {
-        int rc = reflect_pass<T>(h, a, REFLECT_MM);
-        if(rc) return rc;
+    if(a.tile_flag) {
+        const int64_t nt = (a.gn + kTileNodes - 1) / kTileNodes;
+        slot = timer_begin(h, "plain_tiles");
+        k_tile_list<<<(unsigned)((nt + kTileSpan - 1) / kTileSpan), kTileThreads, 0, h->stream>>>(a.tile_flag, nt, h->plain.tiles,
+                                                                                               h->plain.tile_count);
+        timer_end(h, slot);
+        MPM_LAUNCHED(h, "k_tile_list");
     }
+    if(a.reflect && !h->reflect.full_reflection && (rc = reflect_pass<T>(h, a, REFLECT_MM))) return rc;
+    if(with_forces) return MPM_OK;
     slot = timer_begin(h, "plain_normalize");
     k_normalize<T><<<gblocks(h, a.gn, t), t, 0, h->stream>>>(a);
     timer_end(h, slot);
@@ -463,35 +555,34 @@ template<class T> int p2g_t(mpm_handle* h, double dt)
     return MPM_OK;
 }
 
-template<class T> int forces_t(mpm_handle* h, double dt)
+// with_forces: P2G scattered the forces already.
+template<class T> int forces_t(mpm_handle* h, double dt, bool with_forces)
 {
     PlainArgs<T> a = args<T>(h, dt);
     const int t = kScatterThreads;
-    if(a.n) {
-        int slot = timer_begin(h, "plain_stress");
-        if(h->sp.dim == 3) k_stress<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
-        else k_stress<T, 2><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
-        timer_end(h, slot);
-        MPM_LAUNCHED(h, "k_stress");
-        slot = timer_begin(h, "plain_forces");
+    int rc;
+    if(a.n && !with_forces) {
+        if((rc = stress_t<T>(h, a))) return rc;
+        const int slot = timer_begin(h, "plain_forces");
         if(h->sp.dim == 3) k_forces<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
         else k_forces<T, 2><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_forces");
     }
-    if(a.reflect && !h->reflect.full_reflection) {
-        int rc = reflect_pass<T>(h, a, REFLECT_FORCE);
-        if(rc) return rc;
+    if(a.reflect && !h->reflect.full_reflection && (rc = reflect_pass<T>(h, a, REFLECT_FORCE))) return rc;
+    const int slot = timer_begin(h, "plain_grid_update"), b = gblocks(h, a.gn, t);
+    if(h->sp.dim == 3) {
+        if(with_forces) k_grid_update<T, 3, true><<<b, t, 0, h->stream>>>(a);
+        else k_grid_update<T, 3, false><<<b, t, 0, h->stream>>>(a);
+    } else {
+        if(with_forces) k_grid_update<T, 2, true><<<b, t, 0, h->stream>>>(a);
+        else k_grid_update<T, 2, false><<<b, t, 0, h->stream>>>(a);
     }
-    int slot = timer_begin(h, "plain_grid_update");
-    if(h->sp.dim == 3) k_grid_update<T, 3><<<gblocks(h, a.gn, t), t, 0, h->stream>>>(a);
-    else k_grid_update<T, 2><<<gblocks(h, a.gn, t), t, 0, h->stream>>>(a);
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_grid_update");
     if(a.reflect) {
         if(h->reflect.full_reflection) {   // no collision objects: the friction velocity is the velocity
-            int rc = reflect_pass<T>(h, a, REFLECT_FRICTION);
-            if(rc) return rc;
+            if((rc = reflect_pass<T>(h, a, REFLECT_FRICTION))) return rc;
             k_copy_vf<T><<<gblocks(h, a.gn * h->sp.dim, t), t, 0, h->stream>>>(a);
             MPM_LAUNCHED(h, "k_copy_vf");
         } else {
@@ -591,14 +682,14 @@ __global__ void k_fold(const double* partial, int count, int take_min, double* o
 template<class T> __global__ void k_scale_dt(PlainArgs<T> a, T s)
 {
     const int d = a.sp.dim;
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.gn; i += (int64_t)gridDim.x * blockDim.x) {
-        if(a.gm[i] == 0) continue;
+    for_nodes(a, [&](int64_t i) {
+        if(a.gm[i] == 0) return;
         for(int k = 0; k < d; k++) {
             const T vs = a.gv0[i * d + k];
             a.gv[i * d + k] = (a.gv[i * d + k] - vs) * s + vs;
             a.gvf[i * d + k] = (a.gvf[i * d + k] - vs) * s + vs;
         }
-    }
+    });
 }
 
 template<class T> int reduce_dt_t(mpm_handle* h, double dt, double* dt_out)
@@ -784,6 +875,16 @@ int plain_alloc(mpm_handle* h, int64_t n)
         for(int i = 1; i < 6; i++) MPM_CUDA(h, cudaMalloc(g[i], gn * d * e));
         s.gn = gn;
         for(void** p: g) MPM_CUDA(h, cudaMemsetAsync(*p, 0, (p == &s.gm ? gn : gn * d) * e, h->stream));
+        cudaFree(s.tile_flag); s.tile_flag = nullptr;
+        cudaFree(s.tiles); s.tiles = nullptr;
+        cudaFree(s.tile_count); s.tile_count = nullptr;
+        s.grid_listed = false;
+        if(gn >= kListedGrid) {
+            const int64_t nt = (gn + kTileNodes - 1) / kTileNodes, span = (nt + kTileSpan - 1) / kTileSpan * kTileSpan;
+            MPM_CUDA(h, cudaMalloc(&s.tile_flag, span));
+            MPM_CUDA(h, cudaMalloc(&s.tiles, nt * sizeof(uint32_t)));
+            MPM_CUDA(h, cudaMalloc(&s.tile_count, sizeof(uint32_t)));
+        }
     }
     if(s.n != n) {
         void** pa[] = {&s.X, &s.V, &s.F, &s.B, &s.mass, &s.vol, &s.mu, &s.lam, &s.pft, &s.Fp, &s.mu0, &s.lam0,
@@ -808,11 +909,34 @@ int plain_alloc(mpm_handle* h, int64_t n)
     return MPM_OK;
 }
 
+// Before a substep, never inside a captured one: the whole grid to zero where the
+// tile list does not describe it (new arrays, or reflection boundaries, whose
+// passes write every node, were on).
+int plain_prepare(mpm_handle* h)
+{
+    PlainState& s = h->plain;
+    if(!s.gn) return MPM_OK;
+    if(!list_tiles(h)) {
+        s.grid_listed = false;
+        return MPM_OK;
+    }
+    if(s.grid_listed) return MPM_OK;
+    const size_t e = esize(h);
+    const int d = h->sp.dim;
+    const int64_t nt = (s.gn + kTileNodes - 1) / kTileNodes;
+    void* g[] = {s.gm, s.gmv, s.gv0, s.gf, s.gv, s.gvf};
+    for(void* p: g) MPM_CUDA(h, cudaMemsetAsync(p, 0, (p == s.gm ? s.gn : s.gn * d) * e, h->stream));
+    MPM_CUDA(h, cudaMemsetAsync(s.tile_flag, 0, (nt + kTileSpan - 1) / kTileSpan * kTileSpan, h->stream));
+    MPM_CUDA(h, cudaMemsetAsync(s.tile_count, 0, sizeof(uint32_t), h->stream));
+    s.grid_listed = true;
+    return MPM_OK;
+}
+
 void plain_free(mpm_handle* h)
 {
     PlainState& s = h->plain;
     void* ps[] = {s.X, s.V, s.F, s.B, s.mass, s.vol, s.mu, s.lam, s.pft, s.valid, s.gm, s.gmv, s.gv0, s.gf, s.gv, s.gvf,
-                  s.Fp, s.mu0, s.lam0, s.pdef, s.rhoF, s.sigY, s.vc, s.pmodel, s.pmask};
+                  s.Fp, s.mu0, s.lam0, s.pdef, s.rhoF, s.sigY, s.vc, s.pmodel, s.pmask, s.tile_flag, s.tiles, s.tile_count};
     for(void* p: ps) cudaFree(p);
     s = PlainState();
 }
@@ -996,11 +1120,20 @@ int plain_get_particles(mpm_handle* h, mpm_particles_view* v)
 
 int plain_p2g(mpm_handle* h, double dt, double)
 {
-    return h->model.precision == MPM_FP64 ? p2g_t<double>(h, dt) : p2g_t<float>(h, dt);
+    return h->model.precision == MPM_FP64 ? p2g_t<double>(h, dt, false) : p2g_t<float>(h, dt, false);
+}
+// P2G and the forces of an explicit substep back to back, up to the grid
+// velocities: the phases as plain_p2g and plain_forces run them, in fewer passes.
+int plain_p2g_forces(mpm_handle* h, double dt)
+{
+    const bool fp64 = h->model.precision == MPM_FP64;
+    int rc = fp64 ? p2g_t<double>(h, dt, true) : p2g_t<float>(h, dt, true);
+    if(rc) return rc;
+    return fp64 ? forces_t<double>(h, dt, true) : forces_t<float>(h, dt, true);
 }
 int plain_forces(mpm_handle* h, double dt, double)
 {
-    return h->model.precision == MPM_FP64 ? forces_t<double>(h, dt) : forces_t<float>(h, dt);
+    return h->model.precision == MPM_FP64 ? forces_t<double>(h, dt, false) : forces_t<float>(h, dt, false);
 }
 int plain_reflect_velocity(mpm_handle* h)
 {
@@ -1031,11 +1164,15 @@ int plain_get_grid(mpm_handle* h, double* m, double* v0, double* v, double* vf)
 
 namespace {
 // Extra node forces into the grid force array of the current substep (after
-// P2G cleared it and before the grid update reads it).
-template<class T, class S> __global__ void k_add_forces(T* gf, const S* f, int64_t count)
+// P2G cleared it and before the grid update reads it), at the nodes with mass,
+// the only ones it reads.
+template<class T, class S> __global__ void k_add_forces(PlainArgs<T> a, const S* f)
 {
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
-        gf[i] += (T)f[i];
+    const int d = a.sp.dim;
+    for_nodes(a, [&](int64_t i) {
+        if(a.gm[i] == 0) return;
+        for(int k = 0; k < d; k++) a.gf[i * d + k] += (T)f[i * d + k];
+    });
 }
 }  // namespace
 
@@ -1054,11 +1191,13 @@ int plain_add_forces(mpm_handle* h, const void* f, int dtype, bool on_device)
     }
     const int blocks = gblocks(h, count, 256);
     if(h->model.precision == MPM_FP64) {
-        if(e == 8) k_add_forces<double, double><<<blocks, 256, 0, h->stream>>>((double*)s.gf, (const double*)src, count);
-        else k_add_forces<double, float><<<blocks, 256, 0, h->stream>>>((double*)s.gf, (const float*)src, count);
+        const PlainArgs<double> a = args<double>(h, 0.0);
+        if(e == 8) k_add_forces<double, double><<<blocks, 256, 0, h->stream>>>(a, (const double*)src);
+        else k_add_forces<double, float><<<blocks, 256, 0, h->stream>>>(a, (const float*)src);
     } else {
-        if(e == 8) k_add_forces<float, double><<<blocks, 256, 0, h->stream>>>((float*)s.gf, (const double*)src, count);
-        else k_add_forces<float, float><<<blocks, 256, 0, h->stream>>>((float*)s.gf, (const float*)src, count);
+        const PlainArgs<float> a = args<float>(h, 0.0);
+        if(e == 8) k_add_forces<float, double><<<blocks, 256, 0, h->stream>>>(a, (const double*)src);
+        else k_add_forces<float, float><<<blocks, 256, 0, h->stream>>>(a, (const float*)src);
     }
     MPM_LAUNCHED(h, "k_add_forces");
     if(stage) MPM_CUDA(h, cudaFreeAsync(stage, h->stream));

@@ -25,7 +25,29 @@ template<class T> struct PlainArgs {
     unsigned moving;
     const uint8_t* pmodel;     // per-particle constitutive model, or null (sp.model for all)
     const uint8_t* pmask;      // particles the plasticity acts on, or null (all)
+    uint8_t* tile_flag;        // node tiles: P2G's flags, the list and its length; null: every node
+    const uint32_t *tiles, *tile_count;
 };
+
+constexpr int kTileNodes = 32;
+
+// f(i) over the nodes of the listed tiles (a warp per tile), or over every node.
+template<class T, class FN> __device__ __forceinline__ void for_nodes(const PlainArgs<T>& a, FN&& f)
+{
+    const uint32_t nt = a.tiles ? *a.tile_count : (uint32_t)((a.gn + kTileNodes - 1) / kTileNodes);
+    const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+    for(uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < nt; t += nw) {
+        const int64_t i = (int64_t)(a.tiles ? a.tiles[t] : t) * kTileNodes + (threadIdx.x & 31);
+        if(i < a.gn) f(i);
+    }
+}
+
+// Grids of this many nodes and more are passed over by the list of tiles that
+// P2G touched.  64^2 grid (4,900 nodes): every node is the faster way, one
+// launch less; 64^3 (343,000): the list is.
+constexpr int64_t kListedGrid = 1 << 16;
+
+inline bool list_tiles(const mpm_handle* h) { return !h->reflect.enabled && h->plain.gn >= kListedGrid; }
 
 // The constitutive model of particle p: its own, or the handle's.
 template<class T> __device__ __forceinline__ int model_of(const PlainArgs<T>& a, int64_t p)
@@ -119,6 +141,10 @@ template<class T> inline PlainArgs<T> args(mpm_handle* h, double dt)
     a.pmask = s.pmask;
     a.motion = h->motion_dev;
     a.moving = h->motion_dev ? h->moving : 0u;
+    const bool listed = list_tiles(h);
+    a.tile_flag = listed ? s.tile_flag : nullptr;
+    a.tiles = listed ? s.tiles : nullptr;
+    a.tile_count = s.tile_count;
     return a;
 }
 
