@@ -465,11 +465,10 @@ int mpm_autotune_ex(mpm_handle* h, double dt, int substeps, int flags, char* rep
 
 /* The fast path's launch shape, as mpm_autotune chooses it (no reference
  * counterpart: the reference's OpenMP loops have no launch configuration).
- * p2g_variant: MPM_P2G_GROUPS128 / MPM_P2G_GROUPS256 (groups of 4 lanes
- * accumulating a cell's node values in registers, 128 or 256 threads, work
- * items of up to 512 / 1024 particles of a block), MPM_P2G_FIXED128 /
- * MPM_P2G_FIXED256 (one thread per particle into a fixed-point shared tile,
- * work items of up to 128 / 256 particles); G2P takes the same work items;
+ * p2g_variant: threads per CTA and largest work item (particles of one block)
+ * of P2G: MPM_P2G_GROUPS128 128 and 256, MPM_P2G_GROUPS256 256 and 256,
+ * MPM_P2G_FIXED128 64 and 64, MPM_P2G_FIXED256 128 and 128 (the names are of
+ * earlier kernels); G2P takes the same work items;
  * g2p_threads: 64, 128 or 256 per CTA; cta_mult: 1 or 2 times the resident
  * CTAs per SM.  A new handle starts with MPM_P2G_FIXED256, 128, 1. */
 enum { MPM_P2G_GROUPS128 = 0, MPM_P2G_GROUPS256 = 1, MPM_P2G_FIXED128 = 2, MPM_P2G_FIXED256 = 3 };

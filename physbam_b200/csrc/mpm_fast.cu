@@ -12,10 +12,10 @@
 //            block; invalid particles go to the tail).
 //   p2g      persistent CTAs over the work items: B-spline weights, the stress P(F) F^T (fused;
 //            MPM_FINITE_ELEMENTS::Precompute, .cpp:47-67), APIC momentum plus
-//            dt * force into a 6^3-node shared fixed-point tile, flushed with
-//            one float4 atomic per touched node (Particle_To_Grid l.245-306 with
-//            MPM_FINITE_ELEMENTS::Add_Forces folded in).  It marks the node
-//            blocks its tile covers.
+//            dt * force summed in registers along runs of cells and sent to the
+//            grid with one float4 reduction per node and run (Particle_To_Grid
+//            l.245-306 with MPM_FINITE_ELEMENTS::Add_Forces folded in).  It marks
+//            the node blocks its block's stencils cover.
 //   grid     one thread per node of the marked node blocks: v = (mv + dt f)/m
 //            + dt g, collision projection and friction (Apply_Forces
 //            l.959-1060); clears the accumulator for the next substep.
@@ -47,14 +47,6 @@ using namespace mpm;
 constexpr int BS = 4;                      // cells per particle-block edge
 constexpr int TE = BS + 2;                 // tile edge in nodes
 constexpr int TN = TE * TE * TE;           // 216 nodes per tile
-// P2G tile layout: node (x, y, z) of the 6^3 tile at x PSX + y PSY + z.  With
-// these strides the 32 cells of a warp-aligned half block (cell = lx << 4 |
-// ly << 2 | lz, lx in {0, 1} or {2, 3}) reach 32 distinct shared-memory banks
-// at every node offset (52 lx + 8 ly + lz is distinct mod 32), where the
-// dense 6-stride layout put up to four lanes on one bank.
-constexpr int PSY = 8, PSX = 52;
-constexpr int PTN = (TE - 1) * PSX + (TE - 1) * PSY + TE;   // 306 floats per quantity
-__host__ __device__ constexpr int ptile(int x, int y, int z) { return x * PSX + y * PSY + z; }
 constexpr uint32_t SENTINEL = 0xffffffffu;
 constexpr int NCOMP = 24;                  // x3 v3 F9 B9 floats per particle
 constexpr int C_X = 0, C_V = 3, C_F = 6, C_B = 15;
@@ -75,7 +67,7 @@ constexpr int DIR_STAY = 13, DIR_FAR = 27, DIR_INVALID = 28;
 constexpr int ROW = 32;
 constexpr int SCAN_TILE = 256;             // allocation unit of the block scan's status words (>= its tiles)
 // Largest work item (particles of one block) of each P2G launch shape.
-constexpr int kPartSize[4] = {512, 1024, 128, 256};
+constexpr int kPartSize[4] = {256, 256, 64, 128};
 
 struct FastArgs {
     int64_t n, npad;
@@ -132,6 +124,14 @@ struct FastArgs {
     const uint8_t* pmodel;    // constitutive model per caller particle index, or null (the scene's)
     const uint8_t* pmask;     // plasticity on, per caller particle index, or null (all)
 };
+
+// Stream c of an SoA buffer at slot i: a base the whole warp shares and a 32-bit
+// byte offset (fast_alloc takes fewer than 2^30 particles), so that no access
+// needs a 64-bit index of its own.
+__device__ __forceinline__ float ldg_at(const float* base, int64_t c, int64_t npad, uint32_t i)
+{
+    return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(base + c * npad) + (i << 2));
+}
 
 // The constitutive model of the particle in slot i of the current buffer.
 __device__ __forceinline__ int slot_model(const FastArgs& a, const SceneDev& sc, uint32_t i)
@@ -405,9 +405,10 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x)
     return x;
 }
 
-// Work items (P2G and G2P): part k of the `parts` parts of a block, two uint4
-// each, (block, k, parts, scene) and (block start, block count, 0, 0), so that
-// a kernel needs no other load to begin an item.  CTAs take items by ticket
+// Work items (P2G and G2P): a contiguous part of a block's particles, two uint4
+// each, (block, first sorted position, one past the last, scene) and (block x |
+// y << 16, block z, 0, 0), so that a kernel needs no other load (and no
+// division) to begin an item.  CTAs take items by ticket
 // (an atomic counter: CTAs that finish early take more) ahead of need: P2G
 // starts on the item of its CTA index, then holds the next item's descriptor
 // in flight and the ticket after it, so neither round trip falls between two
@@ -564,10 +565,14 @@ __global__ void __launch_bounds__(BIN_THREADS) k_bins(FastArgs a)
 #pragma unroll
         for(int k = 0; k < 7; k++) crow[k] = make_uint4(0u, 0u, 0u, 0u);
         a.active[ex[3]++] = make_uint4((uint32_t)b, start, cnt[u], sid[u]);
+        int bx, by, bz;
+        block_coords(sc, (uint32_t)b - sc.block_base, bx, by, bz);
         for(uint32_t k = 0; k < parts; k++, ex[2]++)
             if(ex[2] < a.chunk_cap) {
-                a.chunks[2 * (size_t)ex[2]] = make_uint4((uint32_t)b, k, parts, sid[u]);
-                a.chunks[2 * (size_t)ex[2] + 1] = make_uint4(start, cnt[u], 0u, 0u);
+                const uint32_t j0 = start + (uint32_t)((uint64_t)cnt[u] * k / parts);
+                const uint32_t j1 = start + (uint32_t)((uint64_t)cnt[u] * (k + 1) / parts);
+                a.chunks[2 * (size_t)ex[2]] = make_uint4((uint32_t)b, j0, j1, sid[u]);
+                a.chunks[2 * (size_t)ex[2] + 1] = make_uint4((uint32_t)bx | ((uint32_t)by << 16), (uint32_t)bz, 0u, 0u);
             }
     }
 }
@@ -757,15 +762,12 @@ __device__ __forceinline__ void pair_slot(const Axis<float>& wx, const Axis<floa
     }
 }
 
-// Weights and separable factors of all four node quantities of the particle
-// at sorted position j (mass: Hx = m wx, Hy = Hz = 0).  A particle whose
-// stress needs the FP64 route is listed for p2g_finish and contributes
-// mass and momentum here.
+// Weights and separable factors of the momentum of the particle at sorted
+// position j (its mass is w m).  A particle whose stress needs the FP64 route is
+// listed for p2g_finish and contributes mass and momentum here.
 struct P2GFactors {
     float w[9];            // wx[3], wy[3], wz[3]
-    float mwx[3];          // mass factor m wx
     PairSlot q[3];         // momentum components x, y, z
-    int base[3];           // first stencil node - ghost, per axis
 };
 
 // Factors from a particle state held in registers (X, V, F, B, attributes);
@@ -783,7 +785,6 @@ __device__ __forceinline__ void factors_from(const FastArgs& a, const SceneDev& 
     const Axis<float> wx = spline_axis<float>(X[0], sc.dmin[0], sc.dx[0], sc.inv[0]);
     const Axis<float> wy = spline_axis<float>(X[1], sc.dmin[1], sc.dx[1], sc.inv[1]);
     const Axis<float> wz = spline_axis<float>(X[2], sc.dmin[2], sc.dx[2], sc.inv[2]);
-    P.base[0] = wx.base; P.base[1] = wy.base; P.base[2] = wz.base;
     float dX[3][3];
     const float bx = (float)wx.base + 0.5f, by = (float)wy.base + 0.5f, bz = (float)wz.base + 0.5f;
 #pragma unroll
@@ -800,41 +801,20 @@ __device__ __forceinline__ void factors_from(const FastArgs& a, const SceneDev& 
         pair_slot(wx, wy, wz, dX, m * V[r], mBD, Sr, P.q[r]);
     }
 #pragma unroll
-    for(int o = 0; o < 3; o++) {
-        P.mwx[o] = m * wx.w[o];
-        P.w[o] = wx.w[o]; P.w[3 + o] = wy.w[o]; P.w[6 + o] = wz.w[o];
-    }
+    for(int o = 0; o < 3; o++) { P.w[o] = wx.w[o]; P.w[3 + o] = wy.w[o]; P.w[6 + o] = wz.w[o]; }
 }
 
-// i = perm[j], the slot of sorted position j (callers load it early).
-__device__ __forceinline__ void particle_factors(const FastArgs& a, const SceneDev& sc, uint32_t j, uint32_t i, P2GFactors& P)
+// i = perm[j], the slot of sorted position j.  Returns the mass.
+__device__ __forceinline__ float particle_factors(const FastArgs& a, const SceneDev& sc, uint32_t j, uint32_t i, P2GFactors& P)
 {
     float X[3], V[3], F[9], B[9];
 #pragma unroll
-    for(int r = 0; r < 3; r++) { X[r] = a.src[(C_X + r) * a.npad + i]; V[r] = a.vsrc[r * a.npad + i]; }
+    for(int r = 0; r < 3; r++) { X[r] = ldg_at(a.src, C_X + r, a.npad, i); V[r] = ldg_at(a.vsrc, r, a.npad, i); }
 #pragma unroll
-    for(int r = 0; r < 9; r++) { F[r] = a.src[(C_F + r) * a.npad + i]; B[r] = a.src[(C_B + r) * a.npad + i]; }
-    factors_from(a, sc, X, V, F, B, a.src_attr[i], j, P, slot_model(a, sc, i));   // attributes: mass, volume, mu, lambda
-}
-
-// The 27 node values of one particle: f(ii, jj, kk, mass, px, py, pz).
-template<class FN> __device__ __forceinline__ void factor_nodes(const P2GFactors& P, FN&& f)
-{
-#pragma unroll
-    for(int ii = 0; ii < 3; ii++)
-#pragma unroll
-        for(int jj = 0; jj < 3; jj++) {
-            const float wxy = P.w[ii] * P.w[3 + jj], mxy = P.mwx[ii] * P.w[3 + jj];
-            float A[3];
-#pragma unroll
-            for(int r2 = 0; r2 < 3; r2++) A[r2] = fmaf(P.q[r2].Hx[ii], P.w[3 + jj], P.w[ii] * P.q[r2].Hy[jj]);
-#pragma unroll
-            for(int kk = 0; kk < 3; kk++) {
-                const float wz = P.w[6 + kk];
-                f(ii, jj, kk, mxy * wz, fmaf(A[0], wz, wxy * P.q[0].Hz[kk]), fmaf(A[1], wz, wxy * P.q[1].Hz[kk]),
-                  fmaf(A[2], wz, wxy * P.q[2].Hz[kk]));
-            }
-        }
+    for(int r = 0; r < 9; r++) { F[r] = ldg_at(a.src, C_F + r, a.npad, i); B[r] = ldg_at(a.src, C_B + r, a.npad, i); }
+    const float4 at = a.src_attr[i];
+    factors_from(a, sc, X, V, F, B, at, j, P, slot_model(a, sc, i));   // attributes: mass, volume, mu, lambda
+    return at.x;
 }
 
 // The elastic force of the particles the P2G kernels listed for the FP64
@@ -907,461 +887,165 @@ __global__ void k_penalty_kick(FastArgs a)
 // ---------------------------------------------------------------------------
 // P2G (MPM_DRIVER::Particle_To_Grid, MPM_DRIVER.cpp:245-306, with
 // MPM_FINITE_ELEMENTS::Add_Forces, MPM_FINITE_ELEMENTS.cpp:84-99, folded in as
-// dt f): one work item is part k of a block, the particles bstart + k,
-// bstart + k + parts, ... (a strided part samples every cell of the block),
-// one thread per particle.
+// dt f): one work item is a contiguous part of a block, binned by cell in shared
+// memory.  Each thread prepares PER particles (stress, weights, separable
+// factors) and leaves them in shared memory in cell order; then groups of 9
+// lanes, a lane per (x, y) offset of the stencil, walk balanced ranges of that
+// order and sum the three nodes along z of all four quantities in registers.
+// Where the cell changes, a step to the next cell along z sends one node and
+// shifts the registers, any other step sends all three, each as one float4
+// reduction.  So a node value costs two FMAs and no atomic of its own: a cell's
+// particles share theirs, and CTA barriers only order the binning and the
+// factors (two per item).
 //
-// The part's node values are summed in a shared tile of fixed-point
-// integers: shared-memory integer adds run at three times the rate of float
-// adds to shared memory, and integer sums do not depend on their order.  Each
-// quantity (mass, momentum x, y, z) has its own power-of-two scale, chosen
-// after every particle of the part has bounded its largest node value: the
-// bounds' sum B maps below 2^21, so no node sum can overflow.  A contribution
-// goes in as its nearest integer plus its rounding residual in units of 2^-23
-// (a second 32-bit sum: at most 256 residuals of at most 2^22), both formed by
-// float adds rather than conversion instructions, so a node keeps B 2^-45
-// absolutely: nodes that only the edges of a few stencils reach, with masses
-// many orders below the part's, keep their velocities to FP32 accuracy.  The
-// tile goes out as floats (hi + lo 2^-23 combined in FP64) with one float4
-// atomic per touched node.
-//
-// Lanes must hit different nodes in each shared add, so the part's particles
-// are first binned by cell and handed out round by round (round r: the
-// (r+1)-th particle of every cell that has one), cells in index order.
+// What bounds it (4.33 M particles, 128^3 dam break, corotated): 36 issue slots
+// per particle, of which the preparation is two thirds, at 24 warps per SM; the
+// factor reads take a quarter of the shared-memory pipe.  It replaced a 6^3
+// fixed-point tile of shared integer atomics (216 per particle, 74 issue slots
+// and seven barriers per item; the float sums here are no further from FP64):
+// 540 -> 323 us there, 52 -> 32 us on the 242,752 particles of the spheres.
+// 128 threads and particles per item: 256 and 256 took 348 and 33 us (fewer
+// CTAs to fill each other's barriers), 64 and 64 331 and 33 us.
 // ---------------------------------------------------------------------------
-template<int T> struct P2GSmem {
-    int q[4][PTN];                        // fixed-point tile: mass, momentum x, y, z (units of 1 / scale)
-    int ql[4][PTN];                       // the rounding residuals, units of 2^-22 / scale
-    uint32_t ccount[64];                  // particles per cell of the part
-    uint32_t rsize[T];                    // particles in round r
-    uint32_t roff[T];                     // first list position of round r
-    unsigned long long rmask[T];          // cells with more than r particles
-    uint32_t list[T];                     // the part's sorted positions, round by round
-    float bound[4];
-    float scale[4];
-    int maxc;
-    int scene;
+// Add a node value without reading it back.  atomicAdd(float4*) becomes the
+// returning form here: 42 LSU wavefronts per warp instruction, P2G 467 us.
+__device__ __forceinline__ void red_add(float4* p, const float4& v)
+{
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :: "l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// A particle in shared memory: 9 float4 (per axis and offset the three momentum
+// factors and the weight), then mass and cell.  11 float4, an odd number, so that
+// the 8 lanes of a 128-bit store phase start on different banks.
+constexpr int FROW = 11;
+
+struct P2GSmem {
+    uint32_t ccount[2][64];               // particles per cell, this item and the next
     uint4 work[2][2];                     // this item's descriptor and the next one's
+    int scene, last;
     SceneDev sc;
 };
 
-// Largest |node value| of a particle over its 27 nodes, per quantity.
-__device__ __forceinline__ void factor_bounds(const P2GFactors& P, float* bnd)
+template<int T, int PER, int CTAS> __global__ void __launch_bounds__(T, CTAS) k_p2g(FastArgs a)
 {
-    const float mx = fmaxf(P.w[0], fmaxf(P.w[1], P.w[2]));
-    const float my = fmaxf(P.w[3], fmaxf(P.w[4], P.w[5]));
-    const float mz = fmaxf(P.w[6], fmaxf(P.w[7], P.w[8]));
-    bnd[0] = fmaxf(P.mwx[0], fmaxf(P.mwx[1], P.mwx[2])) * my * mz;
-#pragma unroll
-    for(int r = 0; r < 3; r++) {
-        const PairSlot& s = P.q[r];
-        const float hx = fmaxf(fabsf(s.Hx[0]), fmaxf(fabsf(s.Hx[1]), fabsf(s.Hx[2])));
-        const float hy = fmaxf(fabsf(s.Hy[0]), fmaxf(fabsf(s.Hy[1]), fabsf(s.Hy[2])));
-        const float hz = fmaxf(fabsf(s.Hz[0]), fmaxf(fabsf(s.Hz[1]), fabsf(s.Hz[2])));
-        bnd[1 + r] = hx * my * mz + mx * hy * mz + mx * my * hz;
-    }
-}
-
-// The factors of a particle in shared memory, one array of T per value (so the
-// thread that reads slot t reads consecutive words).
-constexpr int NFAC = 39;   // w[9], mass factor m wx[3], momentum Hx, Hy, Hz of x, y, z
-
-constexpr float kRoundMagic = 12582912.f;       // 1.5 2^23
-constexpr int kRoundMagicBits = 0x4B400000;     // its bit pattern
-
-__device__ __forceinline__ void store_factors(float* FS, int T, int pos, const P2GFactors& P)
-{
-#pragma unroll
-    for(int e = 0; e < 9; e++) FS[e * T + pos] = P.w[e];
-#pragma unroll
-    for(int o = 0; o < 3; o++) FS[(9 + o) * T + pos] = P.mwx[o];
-#pragma unroll
-    for(int r = 0; r < 3; r++)
-#pragma unroll
-        for(int o = 0; o < 3; o++) {
-            FS[(12 + 9 * r + o) * T + pos] = P.q[r].Hx[o];
-            FS[(15 + 9 * r + o) * T + pos] = P.q[r].Hy[o];
-            FS[(18 + 9 * r + o) * T + pos] = P.q[r].Hz[o];
-        }
-}
-
-__device__ __forceinline__ void load_factors(const float* FS, int T, int pos, P2GFactors& P)
-{
-#pragma unroll
-    for(int e = 0; e < 9; e++) P.w[e] = FS[e * T + pos];
-#pragma unroll
-    for(int o = 0; o < 3; o++) P.mwx[o] = FS[(9 + o) * T + pos];
-#pragma unroll
-    for(int r = 0; r < 3; r++)
-#pragma unroll
-        for(int o = 0; o < 3; o++) {
-            P.q[r].Hx[o] = FS[(12 + 9 * r + o) * T + pos];
-            P.q[r].Hy[o] = FS[(15 + 9 * r + o) * T + pos];
-            P.q[r].Hz[o] = FS[(18 + 9 * r + o) * T + pos];
-        }
-}
-
-// Each thread first prepares the particle its own slot of the part holds
-// (loads through perm stay close to consecutive), then the factors move
-// through shared memory to the thread of the particle's place in the
-// round-by-round cell order, which adds them to the tile.
-template<int T> __global__ void __launch_bounds__(T, 768 / T) k_p2g(FastArgs a)
-{
-    constexpr int NW = T / 32;
-    __shared__ P2GSmem<T> S;
-    extern __shared__ __align__(16) float FS[];    // NFAC x T factors, in place order
+    constexpr int PART = T * PER, GROUPS = T / 32 * 3;
+    __shared__ P2GSmem S;
+    extern __shared__ __align__(16) float4 FS[];   // PART rows, in cell order
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nwork = min(a.ctr[CNT_CHUNKS], a.chunk_cap);
-    // thread 0: this item and the next; the first item by CTA index (every CTA
-    // starts on one), later ones by ticket
-    uint32_t w = 0, wnext = 0;
+    for(int t = threadIdx.x; t < 128; t += T) (&S.ccount[0][0])[t] = 0u;
+    // thread 0: the next item; the first by CTA index (every CTA starts on one), later ones by ticket
+    uint32_t wnext = 0;
     if(threadIdx.x == 0) {
         S.scene = -1;
-        w = blockIdx.x;
-        work_prefetch(a, w, nwork, S.work[0]);
+        work_prefetch(a, blockIdx.x, nwork, S.work[0]);
         wnext = gridDim.x + atomicAdd(&a.ctr[CNT_P2G_WORK], 1u);
+        work_arrive(blockIdx.x, nwork, S.work[0]);
+        work_prefetch(a, wnext, nwork, S.work[1]);
     }
+    __syncthreads();
+    const int grp = warp * 3 + lane / 9, gi = lane % 9 / 3, gj = lane % 3;   // lanes 27..31 idle
     for(int cur = 0;; cur ^= 1) {
-        __syncthreads();
-        if(threadIdx.x == 0) {
-            work_arrive(w, nwork, S.work[cur]);
-            work_prefetch(a, wnext, nwork, S.work[cur ^ 1]);
-            w = wnext;
-            wnext = gridDim.x + atomicAdd(&a.ctr[CNT_P2G_WORK], 1u);
-            S.maxc = 0;
-        }
-        for(int t = threadIdx.x; t < 4 * PTN; t += T) { (&S.q[0][0])[t] = 0; (&S.ql[0][0])[t] = 0; }
-        if(threadIdx.x < 64) S.ccount[threadIdx.x] = 0u;
-        if(threadIdx.x < 4) S.bound[threadIdx.x] = 0.f;
-        __syncthreads();
         const uint4 wk = S.work[cur][0], wr = S.work[cur][1];
         if(wk.x == SENTINEL) break;
-        const uint32_t b = wk.x, part = wk.y, parts = wk.z;
-        const int sid = (int)wk.w;
-        if(sid != S.scene) stage_scene(a, sid, &S.sc);
-        const uint32_t s = wr.x, e = wr.x + wr.y;
-        const uint32_t cnt = e - s > part ? min((e - s - part + parts - 1) / parts, (uint32_t)T) : 0u;
-        // this thread's slot of the (strided) part: cell, rank in its cell, factors, bounds
-        const bool mine = threadIdx.x < cnt;
-        uint32_t cell = 0, r = 0;
-        float bnd[4] = {0.f, 0.f, 0.f, 0.f};
-        P2GFactors P;
-        uint32_t slot = 0;
-        if(mine) {   // the slot with the key: one round trip before the particle loads, not two
-            const uint32_t j = s + part + threadIdx.x * parts;
-            cell = a.sorted_keys[j] & 63u;
-            slot = a.perm[j];
-            r = atomicAdd(&S.ccount[cell], 1u);
+        const uint32_t j0 = wk.y, cnt = min(wk.z - wk.y, (uint32_t)PART);
+        const int sid = (int)wk.w, bx = (int)(wr.x & 0xffffu), by = (int)(wr.x >> 16), bz = (int)wr.y;
+        if(sid != S.scene) {
+            __syncthreads();   // the previous item's sums still read S.sc
+            stage_scene(a, sid, &S.sc);
+            if(threadIdx.x == 0) S.scene = sid;
+        }
+        uint32_t cell[PER], rank[PER], slot[PER];
+#pragma unroll
+        for(int u = 0; u < PER; u++) {
+            const uint32_t i = threadIdx.x + u * T;
+            cell[u] = rank[u] = slot[u] = 0u;
+            if(i < cnt) {
+                cell[u] = a.sorted_keys[j0 + i] & 63u;
+                slot[u] = a.perm[j0 + i];
+                rank[u] = atomicAdd(&S.ccount[cur][cell[u]], 1u);
+            }
         }
         __syncthreads();
-        if(threadIdx.x == 0) S.scene = sid;
+        if(threadIdx.x < 64) S.ccount[cur ^ 1][threadIdx.x] = 0u;
         // the block's 8 node blocks for the grid update: flags exchanged now,
-        // first touches listed after the flush (the round trip overlaps the item)
+        // first touches listed at the end (the round trip overlaps the item)
         uint32_t nb = 0, nb_prev = 1;
         if(threadIdx.x >= T - 8) {
             const int o = threadIdx.x - (T - 8);
-            int bx, by, bz;
-            block_coords(S.sc, b - S.sc.block_base, bx, by, bz);
             nb = S.sc.nb_base + ((uint32_t)(bx + (o >> 2)) * S.sc.NN[1] + by + ((o >> 1) & 1)) * S.sc.NN[2] + bz + (o & 1);
             nb_prev = atomicExch(&a.nb_flag[nb], 1u);
         }
-        // the part's rounds: every warp reduces the 64 cell counts itself (no
-        // barrier) and writes the masks of its rounds
-        const uint32_t cc0 = S.ccount[lane], cc1 = S.ccount[lane + 32];
-        uint32_t mc = max(cc0, cc1);
+        // every warp scans the 64 cell counts itself (no barrier): lane k holds cells 2k, 2k + 1
+        const uint32_t c0 = S.ccount[cur][2 * lane], c1 = S.ccount[cur][2 * lane + 1];
+        const uint32_t ex = warp_incl_scan(c0 + c1) - c0 - c1;
 #pragma unroll
-        for(int o = 16; o; o >>= 1) mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o));
-        const int maxc = (int)mc;
-        for(int rr = warp; rr < maxc; rr += NW) {
-            const unsigned lo = __ballot_sync(0xffffffffu, cc0 > (uint32_t)rr);
-            const unsigned hi = __ballot_sync(0xffffffffu, cc1 > (uint32_t)rr);
-            if(lane == 0) {
-                S.rmask[rr] = lo | ((unsigned long long)hi << 32);
-                S.rsize[rr] = __popc(lo) + __popc(hi);
-            }
-        }
-        if(mine) {
-            particle_factors(a, S.sc, s + part + threadIdx.x * parts, slot, P);
-            factor_bounds(P, bnd);
-        }
-#pragma unroll
-        for(int q = 0; q < 4; q++) {
-            float v = bnd[q];
-#pragma unroll
-            for(int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if(lane == 0 && v != 0.f) atomicAdd(&S.bound[q], v);
-        }
-        __syncthreads();
-        if(threadIdx.x >= T - 4) {   // the scale of each quantity
-            const int q = threadIdx.x - (T - 4);
-            const float B = S.bound[q];
-            float sc = 0.f;
-            if(!isfinite(B)) atomicOr(a.flags, MPM_FLAG_NAN);
-            else if(B > 0.f) {
-                int ex;
-                frexpf(B, &ex);                      // B < 2^ex
-                sc = ldexpf(1.f, 21 - max(ex, -90));
-            }
-            S.scale[q] = sc;
-        }
-        if(warp == 0) {   // exclusive scan of the round sizes
-            uint32_t carry = 0;
-            for(int r0 = 0; r0 < maxc; r0 += 32) {
-                const uint32_t x = r0 + lane < maxc ? S.rsize[r0 + lane] : 0u;
-                const uint32_t xi = warp_incl_scan(x);
-                if(r0 + lane < maxc) S.roff[r0 + lane] = carry + xi - x;
-                carry += __shfl_sync(0xffffffffu, xi, 31);
-            }
-        }
-        __syncthreads();
-        if(mine) {
-            const int pos = (int)(S.roff[r] + __popcll(S.rmask[r] & ((1ull << cell) - 1ull)));
-            store_factors(FS, T, pos, P);
-            S.list[pos] = cell;
-        }
-        __syncthreads();
-        if(mine) {   // the particle at place threadIdx.x of the round-by-round order
-            load_factors(FS, T, threadIdx.x, P);
-            const int pc = (int)S.list[threadIdx.x];
-            const float s0 = S.scale[0], s1 = S.scale[1], s2 = S.scale[2], s3 = S.scale[3];
-            const int t0 = ptile(pc >> 4, (pc >> 2) & 3, pc & 3);
-            // y = rint(y) + residual, both as integers without a conversion
-            // instruction: for |x| <= 2^22, x + 1.5 2^23 rounds x to an integer
-            // held in the low mantissa bits (|y| < 2^21 by the scale; the
-            // residual, |y - rint(y)| <= 1/2, goes in units of 2^-23, and
-            // y - rint(y) is exact in float)
-            auto add = [&](int q, int t, float y) {
-                const float m1 = y + kRoundMagic;
-                const float r = y - (m1 - kRoundMagic);
-                atomicAdd(&S.q[q][t], __float_as_int(m1) - kRoundMagicBits);
-                atomicAdd(&S.ql[q][t], __float_as_int(fmaf(r, 8388608.f, kRoundMagic)) - kRoundMagicBits);
-            };
-            factor_nodes(P, [&](int ii, int jj, int kk, float m, float px, float py, float pz) {
-                const int t = t0 + ptile(ii, jj, kk);
-                add(0, t, m * s0);
-                add(1, t, px * s1);
-                add(2, t, py * s2);
-                add(3, t, pz * s3);
-            });
-        }
-        __syncthreads();
-        // out: one float4 atomic per touched node, and the node blocks for the grid update
-        const SceneDev& sc = S.sc;
-        int bx, by, bz;
-        block_coords(sc, b - sc.block_base, bx, by, bz);
-        double inv[4];
-#pragma unroll
-        for(int q = 0; q < 4; q++) inv[q] = S.scale[q] > 0.f ? 1.0 / S.scale[q] : 0.0;
-        for(int t = threadIdx.x; t < TN; t += T) {
-            const int tx = t / (TE * TE), ty = (t / TE) % TE, tz = t % TE, u = ptile(tx, ty, tz);
-            float v[4];
-            bool any = false;
-#pragma unroll
-            for(int q = 0; q < 4; q++) {
-                const int hi = S.q[q][u], lo = S.ql[q][u];
-                any |= (hi | lo) != 0;
-                v[q] = (float)(((double)hi + (double)lo * 1.1920928955078125e-07) * inv[q]);
-            }
-            if(any)
-                atomicAdd(&a.acc[node_index(sc, 4 * bx + tx, 4 * by + ty, 4 * bz + tz)], make_float4(v[1], v[2], v[3], v[0]));
-        }
-        if(nb_prev == 0u) a.nb_list[atomicAdd(&a.ctr[CNT_NODE_BLOCKS], 1u)] = nb;
-    }
-    p2g_finish(a, &S.maxc);
-}
-
-// ---------------------------------------------------------------------------
-// P2G by lane groups: a work item is a contiguous part of a block (at most
-// 4 T particles for T threads), binned by cell in shared memory; groups of 4
-// lanes walk balanced ranges of the cell-sorted part.  Per round each lane of
-// a group prepares one particle (stress, weights, the separable factors of
-// all four node quantities); in four rotating sub-steps lane k takes from the
-// group's lane (k + p) mod 4 that particle's weights and the factors of
-// quantity k (mass, momentum x, y, z) and adds its 27 node values into 27
-// registers.  A lane writes its registers to the shared float tile only when
-// its particles move to another cell, so a cell of ~8 particles costs 27
-// shared atomics per quantity instead of 27 per particle; the tile goes out
-// with one float4 atomic per touched node.
-// ---------------------------------------------------------------------------
-template<int T> struct P2GGroupSmem {
-    float q[4][PTN];                      // node sums: mass, momentum + dt force x, y, z
-    uint32_t ccount[64], cstart[64];
-    uint32_t list[4 * T];                 // the part's sorted positions, cell by cell
-    uint8_t lcell[4 * T];
-    int scene;
-    uint4 work[2][2];                     // this item's descriptor and the next one's
-};
-
-// The 9 separable factors of quantity `qn` (0 mass, 1-3 momentum) of P.
-__device__ __forceinline__ void quantity_factors(const P2GFactors& P, int qn, float* h)
-{
-#pragma unroll
-    for(int o = 0; o < 3; o++) {
-        const float m = P.mwx[o];
-        const float x0 = P.q[0].Hx[o], x1 = P.q[1].Hx[o], x2 = P.q[2].Hx[o];
-        const float y0 = P.q[0].Hy[o], y1 = P.q[1].Hy[o], y2 = P.q[2].Hy[o];
-        const float z0 = P.q[0].Hz[o], z1 = P.q[1].Hz[o], z2 = P.q[2].Hz[o];
-        h[o] = qn == 0 ? m : (qn == 1 ? x0 : (qn == 2 ? x1 : x2));
-        h[3 + o] = qn == 0 ? 0.f : (qn == 1 ? y0 : (qn == 2 ? y1 : y2));
-        h[6 + o] = qn == 0 ? 0.f : (qn == 1 ? z0 : (qn == 2 ? z1 : z2));
-    }
-}
-
-template<int T> __global__ void __launch_bounds__(T, 512 / T) k_p2g_groups(FastArgs a)
-{
-    constexpr int G = T / 4;              // lane groups
-    __shared__ P2GGroupSmem<T> S;
-    __shared__ SceneDev s_sc;
-    const int lane = threadIdx.x & 31, k = threadIdx.x & 3, g = threadIdx.x >> 2;
-    const unsigned gmask = 0xfu << (lane & ~3);
-    const uint32_t nwork = min(a.ctr[CNT_CHUNKS], a.chunk_cap);
-    // thread 0: this item and the next; the first item by CTA index (every CTA
-    // starts on one), later ones by ticket
-    uint32_t w = 0, wnext = 0;
-    if(threadIdx.x == 0) {
-        S.scene = -1;
-        w = blockIdx.x;
-        work_prefetch(a, w, nwork, S.work[0]);
-        wnext = gridDim.x + atomicAdd(&a.ctr[CNT_P2G_WORK], 1u);
-    }
-    for(int cur = 0;; cur ^= 1) {
-        __syncthreads();
-        if(threadIdx.x == 0) {
-            work_arrive(w, nwork, S.work[cur]);
-            work_prefetch(a, wnext, nwork, S.work[cur ^ 1]);
-            w = wnext;
-            wnext = gridDim.x + atomicAdd(&a.ctr[CNT_P2G_WORK], 1u);
-        }
-        for(int t = threadIdx.x; t < 4 * PTN; t += T) (&S.q[0][0])[t] = 0.f;
-        if(threadIdx.x < 64) S.ccount[threadIdx.x] = 0u;
-        __syncthreads();
-        const uint4 wk = S.work[cur][0], wr = S.work[cur][1];
-        if(wk.x == SENTINEL) break;
-        const uint32_t b = wk.x, part = wk.y, parts = wk.z;
-        const int sid = (int)wk.w;
-        if(sid != S.scene) stage_scene(a, sid, &s_sc);
-        const uint32_t s = wr.x, c = wr.y;
-        const uint32_t j0 = s + (uint32_t)((uint64_t)c * part / parts);
-        const uint32_t cnt = min((uint32_t)((uint64_t)c * (part + 1) / parts) + s - j0, (uint32_t)(4 * T));
-        // bin by cell: up to 4 particles per thread
-        uint32_t cl[4], rk[4];
-#pragma unroll
-        for(int u = 0; u < 4; u++) {
-            const uint32_t i = threadIdx.x + u * T;
-            cl[u] = i < cnt ? a.sorted_keys[j0 + i] & 63u : 0u;
-            rk[u] = i < cnt ? atomicAdd(&S.ccount[cl[u]], 1u) : 0u;
-        }
-        __syncthreads();
-        if(threadIdx.x == 0) S.scene = sid;
-        // the block's 8 node blocks for the grid update: flags exchanged now,
-        // first touches listed after the flush (the round trip overlaps the item)
-        uint32_t nb = 0, nb_prev = 1;
-        if(threadIdx.x >= T - 8) {
-            const int o = threadIdx.x - (T - 8);
-            int bx, by, bz;
-            block_coords(s_sc, b - s_sc.block_base, bx, by, bz);
-            nb = s_sc.nb_base + ((uint32_t)(bx + (o >> 2)) * s_sc.NN[1] + by + ((o >> 1) & 1)) * s_sc.NN[2] + bz + (o & 1);
-            nb_prev = atomicExch(&a.nb_flag[nb], 1u);
-        }
-        if(threadIdx.x < 32) {   // exclusive scan of the 64 cell counts
-            const uint32_t c0 = S.ccount[2 * lane], c1 = S.ccount[2 * lane + 1];
-            const uint32_t x = warp_incl_scan(c0 + c1);
-            S.cstart[2 * lane] = x - c0 - c1;
-            S.cstart[2 * lane + 1] = x - c1;
-        }
-        __syncthreads();
-#pragma unroll
-        for(int u = 0; u < 4; u++) {
+        for(int u = 0; u < PER; u++) {
+            const uint32_t pair = __shfl_sync(0xffffffffu, ex, cell[u] >> 1), even = __shfl_sync(0xffffffffu, c0, cell[u] >> 1);
             const uint32_t i = threadIdx.x + u * T;
             if(i < cnt) {
-                const uint32_t pos = S.cstart[cl[u]] + rk[u];
-                S.list[pos] = j0 + i;
-                S.lcell[pos] = (uint8_t)cl[u];
-            }
-        }
-        __syncthreads();
-        // this group's balanced range of the cell-sorted part
-        const uint32_t r0 = (uint32_t)((uint64_t)cnt * g / G), r1 = (uint32_t)((uint64_t)cnt * (g + 1) / G);
-        const SceneDev& sc = s_sc;
-        float acc[27];
-#pragma unroll
-        for(int q = 0; q < 27; q++) acc[q] = 0.f;
-        int cell = -1;
-        float* const tq = S.q[k];
-        auto flush = [&]() {
-            const int t0 = ptile(cell >> 4, (cell >> 2) & 3, cell & 3);
-#pragma unroll
-            for(int q = 0; q < 27; q++) {
-                atomicAdd(&tq[t0 + ptile(q / 9, (q / 3) % 3, q % 3)], acc[q]);
-                acc[q] = 0.f;
-            }
-        };
-        for(uint32_t rb = r0; rb < r1; rb += 4) {   // a round: one particle per lane of the group
-            const uint32_t mine = rb + k;
-            P2GFactors P;
-            int pc = -1;
-            if(mine < r1) {
-                pc = S.lcell[mine];
-                particle_factors(a, sc, S.list[mine], a.perm[S.list[mine]], P);
-            } else {
-#pragma unroll
-                for(int e = 0; e < 9; e++) P.w[e] = 0.f;
+                P2GFactors P;
+                const float m = particle_factors(a, S.sc, j0 + i, slot[u], P);
+                float4* row = FS + (size_t)(pair + ((cell[u] & 1u) ? even : 0u) + rank[u]) * FROW;
 #pragma unroll
                 for(int o = 0; o < 3; o++) {
-                    P.mwx[o] = 0.f;
-#pragma unroll
-                    for(int r = 0; r < 3; r++) P.q[r].Hx[o] = P.q[r].Hy[o] = P.q[r].Hz[o] = 0.f;
+                    row[o] = make_float4(P.q[0].Hx[o], P.q[1].Hx[o], P.q[2].Hx[o], P.w[o]);
+                    row[3 + o] = make_float4(P.q[0].Hy[o], P.q[1].Hy[o], P.q[2].Hy[o], P.w[3 + o]);
+                    row[6 + o] = make_float4(P.q[0].Hz[o], P.q[1].Hz[o], P.q[2].Hz[o], P.w[6 + o]);
                 }
-            }
-#pragma unroll
-            for(int p = 0; p < 4; p++) {
-                // lane k reads lane (k + p) mod 4, which sends the factors of quantity (its index - p) mod 4
-                const int src = (lane & ~3) | ((k + p) & 3);
-                float h[9];
-                quantity_factors(P, (k - p) & 3, h);
-                float w[9], f[9];
-#pragma unroll
-                for(int e = 0; e < 9; e++) {
-                    w[e] = __shfl_sync(gmask, P.w[e], src);
-                    f[e] = __shfl_sync(gmask, h[e], src);
-                }
-                const int rc = __shfl_sync(gmask, pc, src);
-                if(rc < 0) continue;                  // past the group's range
-                if(rc != cell) {
-                    if(cell >= 0) flush();
-                    cell = rc;
-                }
-                // node (i, j, l): Hx[i] wy[j] wz[l] + wx[i] Hy[j] wz[l] + wx[i] wy[j] Hz[l]
-#pragma unroll
-                for(int ii = 0; ii < 3; ii++)
-#pragma unroll
-                    for(int jj = 0; jj < 3; jj++) {
-                        const float wxy = w[ii] * w[3 + jj];
-                        const float A = fmaf(f[ii], w[3 + jj], w[ii] * f[3 + jj]);
-#pragma unroll
-                        for(int ll = 0; ll < 3; ll++) {
-                            const int q = (ii * 3 + jj) * 3 + ll;
-                            acc[q] = fmaf(A, w[6 + ll], fmaf(wxy, f[6 + ll], acc[q]));
-                        }
-                    }
+                *reinterpret_cast<float2*>(row + 9) = make_float2(m, __int_as_float((int)cell[u]));
             }
         }
-        if(cell >= 0) flush();
+        if(threadIdx.x == 0) {
+            work_arrive(wnext, nwork, S.work[cur ^ 1]);
+            wnext = gridDim.x + atomicAdd(&a.ctr[CNT_P2G_WORK], 1u);
+        }
         __syncthreads();
-        // out: one float4 atomic per touched node, and the node blocks for the grid update
-        int bx, by, bz;
-        block_coords(sc, b - sc.block_base, bx, by, bz);
-        for(int t = threadIdx.x; t < TN; t += T) {
-            const int tx = t / (TE * TE), ty = (t / TE) % TE, tz = t % TE, u = ptile(tx, ty, tz);
-            const float m = S.q[0][u];
-            if(m != 0.f)
-                atomicAdd(&a.acc[node_index(sc, 4 * bx + tx, 4 * by + ty, 4 * bz + tz)],
-                          make_float4(S.q[1][u], S.q[2][u], S.q[3][u], m));
+        if(threadIdx.x == 0) work_prefetch(a, wnext, nwork, S.work[cur]);
+        if(lane < 27) {
+            const int sy = S.sc.GA[2], sx = S.sc.GA[1] * S.sc.GA[2];
+            float4* const base = a.acc + node_index(S.sc, 4 * bx + gi, 4 * by + gj, 4 * bz);
+            const uint32_t r0 = cnt * (uint32_t)grp / GROUPS, r1 = cnt * (uint32_t)(grp + 1) / GROUPS;
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 A0 = zero, A1 = zero, A2 = zero;
+            int run = -1;                  // the cell being summed
+            float4* at = base;             // its first node along z
+            for(uint32_t p = r0; p < r1; p++) {
+                const float4* row = FS + (size_t)p * FROW;
+                const float4 fx = row[gi], fy = row[3 + gj], z0 = row[6], z1 = row[7], z2 = row[8];
+                const float2 mc = *reinterpret_cast<const float2*>(row + 9);
+                const int pc = __float_as_int(mc.y);
+                if(pc != run) {
+                    if(pc == run + 1 && (pc & 3)) {        // the next cell along z
+                        red_add(at, A0);
+                        A0 = A1; A1 = A2; A2 = zero;
+                        at++;
+                    } else {
+                        if(run >= 0) { red_add(at, A0); red_add(at + 1, A1); red_add(at + 2, A2); }
+                        A0 = A1 = A2 = zero;
+                        at = base + (pc >> 4) * sx + ((pc >> 2) & 3) * sy + (pc & 3);
+                    }
+                    run = pc;
+                }
+                // node k: (Hx wy + wx Hy) wz[k] + wx wy Hz[k]
+                const float wxy = fx.w * fy.w, mw = mc.x * wxy;
+                const float P0 = fmaf(fx.x, fy.w, fx.w * fy.x), P1 = fmaf(fx.y, fy.w, fx.w * fy.y), P2 = fmaf(fx.z, fy.w, fx.w * fy.z);
+                auto add = [&](float4& A, const float4& z) {
+                    A.x = fmaf(P0, z.w, fmaf(wxy, z.x, A.x));
+                    A.y = fmaf(P1, z.w, fmaf(wxy, z.y, A.y));
+                    A.z = fmaf(P2, z.w, fmaf(wxy, z.z, A.z));
+                    A.w = fmaf(mw, z.w, A.w);
+                };
+                add(A0, z0);
+                add(A1, z1);
+                add(A2, z2);
+            }
+            if(run >= 0) { red_add(at, A0); red_add(at + 1, A1); red_add(at + 2, A2); }
         }
         if(nb_prev == 0u) a.nb_list[atomicAdd(&a.ctr[CNT_NODE_BLOCKS], 1u)] = nb;
     }
-    __shared__ int s_last;
-    p2g_finish(a, &s_last);
+    p2g_finish(a, &S.last);
 }
 
 // One thread per node of the listed node blocks (4^3 nodes each, 64
@@ -1814,9 +1498,7 @@ __device__ __forceinline__ bool g2p_take(const FastArgs& a, uint32_t nwork, uint
         return false;
     }
     const uint4 wk = a.chunks[2 * (size_t)w], wr = a.chunks[2 * (size_t)w + 1];
-    const SceneDev& sc = a.scenes[wk.w];
-    int bx, by, bz;
-    block_coords(sc, wk.x - sc.block_base, bx, by, bz);
+    const int bx = (int)(wr.x & 0xffffu), by = (int)(wr.x >> 16), bz = (int)wr.y;
     fence_async_shared();   // the CTA's reads of this buffer come before the copy's writes
     mbar_expect_tx(bar, TILE_BYTES);
     tma_tile(dst, a.tmaps + wk.w, bar, 4 * bx, 4 * by, 4 * bz);
@@ -1858,16 +1540,14 @@ template<int THREADS, int PK> __global__ void __launch_bounds__(THREADS) k_g2p(F
             const bool more = g2p_take(a, nwork, s_work[buf ^ 1], tv[buf ^ 1], &s_bar[buf ^ 1]);
             issued = (issued & ~(1u << buf)) | (more ? 1u << (buf ^ 1) : 0u);
         }
-        const uint32_t b = wk.x, part = wk.y, parts = wk.z;
-        const int sid = (int)wk.w;
+        const uint32_t b = wk.x, j0 = wk.y, j1 = wk.z;
+        const int sid = (int)wk.w, bx = (int)(wr.x & 0xffffu), by = (int)(wr.x >> 16), bz = (int)wr.y;
         if(sid != s_scene) {
             stage_scene(a, sid, &s_sc);
             __syncthreads();
             if(threadIdx.x == 0) s_scene = sid;
         }
         const SceneDev& sc = s_sc;
-        int bx, by, bz;
-        block_coords(sc, b - sc.block_base, bx, by, bz);
         const int ox = 4 * bx, oy = 4 * by, oz = 4 * bz;
         // the tile: wait for its copy, then note nodes whose friction velocity differs
         const bool arrived = mbar_wait(&s_bar[buf], (uint32_t)(k >> 1) & 1u);
@@ -1882,9 +1562,6 @@ template<int THREADS, int PK> __global__ void __launch_bounds__(THREADS) k_g2p(F
             break;
         }
         const bool anti = __syncthreads_or(differs) != 0;
-        // a contiguous part of the block (coalesced slots)
-        const uint32_t s = wr.x, c = wr.y;
-        const uint32_t j0 = s + (uint32_t)((uint64_t)c * part / parts), j1 = s + (uint32_t)((uint64_t)c * (part + 1) / parts);
         for(uint32_t j = j0 + threadIdx.x; j < j1; j += THREADS) {
             G2PState o;
             g2p_particle<PK>(a, sc, t4, anti, ox, oy, oz, j, o);
@@ -2116,11 +1793,10 @@ int grid_stride_blocks(mpm_handle* h, int64_t n, int t)
     return (int)(b < 1 ? 1 : b);
 }
 
-// Launch shapes the autotuner chooses among.  P2G: lane groups with 128 or
-// 256 threads (work items of up to 512 / 1024 particles), or the fixed-point
-// tile with 128 or 256 threads (one particle per thread).
+// Launch shapes the autotuner chooses among.  P2G: threads and largest work item.
 const int kG2PThreads[] = {64, 128, 256};
-const char* const kP2GNames[] = {"groups128", "groups256", "fixed128", "fixed256"};
+const char* const kP2GNames[] = {"128 threads, 256 particles", "256 threads, 256 particles", "64 threads, 64 particles",
+                                 "128 threads, 128 particles"};
 
 int occupancy_ctas(mpm_handle* h, const void* fn, int threads, int mult)
 {
@@ -2685,22 +2361,13 @@ static int fast_route(mpm_handle* h)
     return MPM_OK;
 }
 
-template<int T> static void launch_p2g(mpm_handle* h, const FastArgs& a)
+template<int T, int PER, int CTAS> static void launch_p2g(mpm_handle* h, const FastArgs& a)
 {
-    const int smem = NFAC * T * (int)sizeof(float);
-    static bool attr = false;
-    if(!attr) {
-        cudaFuncSetAttribute((const void*)k_p2g<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr = true;
-    }
+    const int smem = T * PER * FROW * (int)sizeof(float4);
+    static_assert(T * PER * FROW * sizeof(float4) + sizeof(P2GSmem) <= 48 * 1024, "opt-in shared memory");
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)k_p2g<T>, T, smem);
-    k_p2g<T><<<h->sm_count * (occ > 0 ? occ : 1) * h->fast.cta_mult, T, smem, h->stream>>>(a);
-}
-
-template<int T> static void launch_p2g_groups(mpm_handle* h, const FastArgs& a)
-{
-    k_p2g_groups<T><<<occupancy_ctas(h, (const void*)k_p2g_groups<T>, T, h->fast.cta_mult), T, 0, h->stream>>>(a);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)k_p2g<T, PER, CTAS>, T, smem);
+    k_p2g<T, PER, CTAS><<<h->sm_count * (occ > 0 ? occ : 1) * h->fast.cta_mult, T, smem, h->stream>>>(a);
 }
 
 int fast_p2g(mpm_handle* h, double dt, double)
@@ -2728,10 +2395,10 @@ int fast_p2g(mpm_handle* h, double dt, double)
     }
     int slot = timer_begin(h, "fast_p2g");
     switch(f.route_variant) {
-        case MPM_P2G_GROUPS256: launch_p2g_groups<256>(h, a); break;
-        case MPM_P2G_FIXED128: launch_p2g<128>(h, a); break;
-        case MPM_P2G_FIXED256: launch_p2g<256>(h, a); break;
-        default: launch_p2g_groups<128>(h, a); break;
+        case MPM_P2G_GROUPS128: launch_p2g<128, 2, 5>(h, a); break;
+        case MPM_P2G_GROUPS256: launch_p2g<256, 1, 3>(h, a); break;
+        case MPM_P2G_FIXED128: launch_p2g<64, 1, 12>(h, a); break;
+        default: launch_p2g<128, 1, 6>(h, a); break;
     }
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_p2g");
