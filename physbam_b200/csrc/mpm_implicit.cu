@@ -11,7 +11,8 @@
 // does every grid and particle pass (the force and Hessian scatters are those
 // of MPM_FINITE_ELEMENTS, Add_Forces / Add_Hessian_Times, l.84-132); the host
 // runs the Newton / CG / line-search control flow, reading back one or two
-// reduced scalars per step (deterministic two-stage reductions in FP64).
+// reduced scalars per step (deterministic two-stage reductions in FP64).  The
+// node passes visit the tiles of the grid that P2G touched.
 //
 // Collision objects are the static boxes, planes and spheres of the explicit
 // path; the curvature terms of the projection use the Hessian of the signed
@@ -19,6 +20,7 @@
 // in object order (the reference appends them per node in that order).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -33,13 +35,16 @@ namespace {
 using namespace mpm;
 using namespace plain;
 
-constexpr int kRedBlocks = 256, kRedThreads = 256;
+constexpr int kRedBlocks = 1024, kRedThreads = 256;   // CTAs of a reduction at most
+constexpr int kSoundBlocks = 256;
 constexpr double kCollisionThickness = 1e-15;   // MPM_OBJECTIVE::collision_thickness
 
 template<class T> struct ImpArgs {
     PlainArgs<T> a;
     T *F0, *X0;                 // particle state at the start of the step (Fn = F0)
-    T *U, *FV, *sig, *dP;       // SVD of the current F: U, Fn V, singular values, stress derivative (9 + 3 + 3)
+    // SVD of the current F: U, Fn V, singular values, stress derivative (9 + 3 + 3),
+    // component e of the pass's t-th particle at e n + t (coalesced)
+    T *U, *FV, *sig, *dP;
     double* pe;                 // per-particle potential energy
     uint8_t *cmask, *stuck;     // per node: collision objects (bit j), stuck flag
     T* cdat;                    // per node and object: phi, n_dE, normal, position, H g (2 + 3d)
@@ -72,8 +77,6 @@ template<class T, int d> __global__ void k_imp_keys(ImpArgs<T> ia, uint32_t* key
         keys[p] = k;
     }
 }
-
-template<class T, int d> __device__ __forceinline__ bool node_valid(const ImpArgs<T>& ia, int64_t i) { return ia.a.gm[i] != 0; }
 
 template<class T, int d> __device__ __forceinline__ void node_position(const ImpArgs<T>& ia, int64_t i, T* X)
 {
@@ -199,10 +202,14 @@ template<class T, int d> __global__ void k_imp_precompute(ImpArgs<T> ia)
         }
     T H[9], Bv[3], Cv[3];
     stress_derivative<T, d>(model, S, mu, la, H, Bv, Cv);
-    for(int e = 0; e < d * d; e++) { ia.U[p * d * d + e] = U[e]; ia.FV[p * d * d + e] = FV[e]; }
-    for(int e = 0; e < d; e++) ia.sig[p * d + e] = S[e];
-    for(int e = 0; e < 9; e++) ia.dP[p * 15 + e] = H[e];
-    for(int e = 0; e < 3; e++) { ia.dP[p * 15 + 9 + e] = Bv[e]; ia.dP[p * 15 + 12 + e] = Cv[e]; }
+#pragma unroll
+    for(int e = 0; e < d * d; e++) { ia.U[e * a.n + t] = U[e]; ia.FV[e * a.n + t] = FV[e]; }
+#pragma unroll
+    for(int e = 0; e < d; e++) ia.sig[e * a.n + t] = S[e];
+#pragma unroll
+    for(int e = 0; e < 9; e++) ia.dP[e * a.n + t] = H[e];
+#pragma unroll
+    for(int e = 0; e < 3; e++) { ia.dP[(9 + e) * a.n + t] = Bv[e]; ia.dP[(12 + e) * a.n + t] = Cv[e]; }
     double e = (double)a.vol[p] * (double)energy_density<T, d>(model, S, mu, la);
     for(int k = 0; k < d; k++) e -= (double)a.mass[p] * (double)a.X[p * d + k] * a.sp.gravity[k];
     ia.pe[p] = e + epen;
@@ -278,8 +285,11 @@ template<class T, int d> __device__ __forceinline__ int64_t hessian_row(const Im
             Hz[r] = sum;
         }
     }
-    const T* U = ia.U + p * d * d;
-    const T* FV = ia.FV + p * d * d;
+    T U[9], FV[9], blk[15];
+#pragma unroll
+    for(int e = 0; e < d * d; e++) { U[e] = ia.U[e * a.n + t]; FV[e] = ia.FV[e * a.n + t]; }
+#pragma unroll
+    for(int e = 0; e < 15; e++) blk[e] = ia.dP[e * a.n + t];
     T WF[9], G[9], dPh[9], UD[9], M[9];
 #pragma unroll
     for(int c = 0; c < d; c++)
@@ -299,7 +309,6 @@ template<class T, int d> __device__ __forceinline__ int64_t hessian_row(const Im
             for(int k = 0; k < d; k++) sum += U[k + d * r] * WF[k + d * c];
             G[r + d * c] = sum;
         }
-    const T* blk = ia.dP + p * 15;
     stress_differential<T, d>(blk, blk + 9, blk + 12, G, dPh);
 #pragma unroll
     for(int c = 0; c < d; c++)
@@ -341,25 +350,129 @@ template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_im
 // ---------------------------------------------------------------------------
 // node passes (nodes with mass: MPM_EXAMPLE::valid_grid_indices)
 // ---------------------------------------------------------------------------
-#define NODE_LOOP(ia) \
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (ia).a.gn; i += (int64_t)gridDim.x * blockDim.x) \
-        if(node_valid<T, d>(ia, i))
+// f(i) over them.  Every node vector of the solve is zero on the other nodes of
+// the listed tiles, and the particle passes read and write no node outside.
+template<class T, class FN> __device__ __forceinline__ void mass_nodes(const ImpArgs<T>& ia, FN&& f)
+{
+    for_nodes(ia.a, [&](int64_t i) {
+        if(ia.a.gm[i] != 0) f(i);
+    });
+}
+
+// `count` vectors of `stride` scalars each to zero
+template<class T, int d> __global__ void k_imp_zero(ImpArgs<T> ia, T* x, int64_t stride, int count)
+{
+    for_nodes(ia.a, [&](int64_t i) {
+        for(int v = 0; v < count; v++)
+            for(int k = 0; k < d; k++) x[v * stride + i * d + k] = 0;
+    });
+}
 
 // MPM_KRYLOV_VECTOR::Copy: out = c x + y (y may be null)
 template<class T, int d> __global__ void k_imp_copy(ImpArgs<T> ia, T* out, T c, const T* x, const T* y)
 {
-    NODE_LOOP(ia) {
+    mass_nodes(ia, [&](int64_t i) {
         for(int k = 0; k < d; k++) out[i * d + k] = c * x[i * d + k] + (y ? y[i * d + k] : (T)0);
-    }
+    });
 }
 
 // gradient of MPM_OBJECTIVE::Compute_Unconstrained (l.71-91): g = dv - dt/m f
 template<class T, int d> __global__ void k_imp_grad(ImpArgs<T> ia, T* g, const T* dv, const T* f)
 {
-    NODE_LOOP(ia) {
+    mass_nodes(ia, [&](int64_t i) {
         const T s = ia.a.dt / ia.a.gm[i];
         for(int k = 0; k < d; k++) g[i * d + k] = dv[i * d + k] - s * f[i * d + k];
+    });
+}
+
+// Reductions: a CTA sums its values by a fixed tree and leaves a partial; the CTA
+// that finishes last adds the partials in CTA order, so the result does not
+// depend on scheduling.  It goes to the device (the next kernel's coefficient)
+// and to pinned host memory, which the host reads after one synchronize: no
+// second launch and no copy.
+__device__ __forceinline__ double block_sum(double v)
+{
+    __shared__ double sh[kRedThreads];
+    __syncthreads();                     // an earlier sum's readers
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    for(int s = kRedThreads / 2; s > 0; s >>= 1) {
+        if(threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+        __syncthreads();
     }
+    return sh[0];
+}
+
+// One result of a reduction: its partials (kRedBlocks), count of finished CTAs, and where it goes.
+struct Reduction {
+    double* partial;
+    unsigned* done;
+    double *dev, *host;
+};
+
+__device__ __forceinline__ void grid_sum(double v, const Reduction& r)
+{
+    __shared__ bool last;
+    v = block_sum(v);
+    if(threadIdx.x == 0) {
+        r.partial[blockIdx.x] = v;
+        __threadfence();
+        last = atomicAdd(r.done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if(!last) return;
+    __threadfence();
+    double t = 0;
+    for(int b = threadIdx.x; b < (int)gridDim.x; b += kRedThreads) t += *(volatile double*)(r.partial + b);
+    t = block_sum(t);
+    if(threadIdx.x == 0) {
+        *r.dev = t;
+        *r.host = t;
+        *r.done = 0u;
+    }
+}
+
+// MPM_KRYLOV_SYSTEM::Inner_Product (l.82-95), the term of node i: m x.y
+template<class T, int d> __device__ __forceinline__ double node_dot(const ImpArgs<T>& ia, int64_t i, const T* x, const T* y)
+{
+    double s = 0;
+#pragma unroll
+    for(int k = 0; k < d; k++) s += (double)x[k] * (double)y[k];
+    return (double)ia.a.gm[i] * s;
+}
+
+template<class T, int d> __global__ void __launch_bounds__(kRedThreads) k_imp_dot(ImpArgs<T> ia, const T* x, const T* y, Reduction r)
+{
+    double acc = 0;
+    mass_nodes(ia, [&](int64_t i) { acc += node_dot<T, d>(ia, i, x + i * d, y + i * d); });
+    grid_sum(acc, r);
+}
+
+__global__ void __launch_bounds__(kRedThreads) k_imp_sum_particles(const double* pe, int64_t n, Reduction r)
+{
+    double acc = 0;
+    for(int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) acc += pe[p];
+    grid_sum(acc, r);
+}
+
+__device__ double block_max(double v)
+{
+    __shared__ double sh[kRedThreads];
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    for(int s = kRedThreads / 2; s > 0; s >>= 1) {
+        if(threadIdx.x < s) sh[threadIdx.x] = fmax(sh[threadIdx.x], sh[threadIdx.x + s]);
+        __syncthreads();
+    }
+    return sh[0];
+}
+
+__global__ void k_imp_max_final(const double* partial, int count, double* out)
+{
+    if(threadIdx.x) return;
+    double r = partial[0];
+    for(int b = 1; b < count; b++) r = fmax(r, partial[b]);
+    *out = r;
 }
 
 // MPM_OBJECTIVE::Adjust_For_Collision (l.180-222) with Test_Add_Collision
@@ -369,7 +482,7 @@ template<class T, int d> __global__ void k_imp_grad(ImpArgs<T> ia, T* g, const T
 // test.  A moving object is tested at its frames of the substep's start and end.
 template<class T, int d> __global__ void k_imp_adjust(ImpArgs<T> ia, T* dv)
 {
-    NODE_LOOP(ia) {
+    mass_nodes(ia, [&](int64_t i) {
         const PlainArgs<T>& a = ia.a;
         uint8_t mask = 0, stuck = 0;
         T X0[3];
@@ -402,7 +515,7 @@ template<class T, int d> __global__ void k_imp_adjust(ImpArgs<T> ia, T* dv)
         }
         ia.cmask[i] = mask;
         ia.stuck[i] = stuck;
-    }
+    });
 }
 
 // MPM_OBJECTIVE::Project_Gradient_And_Prune_Constraints (l.226-248): the
@@ -411,9 +524,9 @@ template<class T, int d> __global__ void k_imp_adjust(ImpArgs<T> ia, T* dv)
 // dropped, else the normal part of the gradient is removed.
 template<class T, int d> __global__ void k_imp_project(ImpArgs<T> ia, T* g, int allow_sep)
 {
-    NODE_LOOP(ia) {
+    mass_nodes(ia, [&](int64_t i) {
         uint8_t mask = ia.cmask[i];
-        if(!mask && !ia.stuck[i]) continue;
+        if(!mask && !ia.stuck[i]) return;
         if(ia.stuck[i])
             for(int k = 0; k < d; k++) g[i * d + k] = 0;
         for(int j = ia.nobj - 1; j >= 0; j--) {
@@ -439,16 +552,31 @@ template<class T, int d> __global__ void k_imp_project(ImpArgs<T> ia, T* g, int 
             for(int k = 0; k < d; k++) g[i * d + k] -= ndE * cd[2 + k] + cd[0] * cd[2 + 2 * d + k];
         }
         ia.cmask[i] = mask;
-    }
+    });
 }
 
-// MPM_KRYLOV_SYSTEM::Multiply (l.40-78), before the Hessian: tmp = v with the
-// stuck nodes zeroed and the colliding nodes' normal parts removed.
-template<class T, int d> __global__ void k_imp_mult_pre(ImpArgs<T> ia, T* tmp, const T* v)
+// The node passes of a CG iteration (CONJUGATE_GRADIENT.cpp:20-85), three
+// kernels around the Hessian's: each reads and writes a node once for all it
+// does there.  spheres 128^3 (84,924 nodes with mass of 2.4 M): one pass over
+// the listed tiles is 3 to 5 us; the copies, clears and products as passes of
+// their own over the whole grid were nine of 10 to 25 us.
+
+// s = r + beta s (first: s = r), then MPM_KRYLOV_SYSTEM::Multiply (l.40-78) up to
+// the Hessian: tmp = s with the stuck nodes zeroed and the colliding nodes'
+// normal parts removed, and the Hessian's product cleared.
+template<class T, int d> __global__ void k_cg_direction(ImpArgs<T> ia, T* s, const T* r, T beta, bool first, T* tmp, T* f)
 {
-    NODE_LOOP(ia) {
+    for_nodes(ia.a, [&](int64_t i) {
+#pragma unroll
+        for(int k = 0; k < d; k++) f[i * d + k] = 0;
+        if(ia.a.gm[i] == 0) return;
         T x[3];
-        for(int k = 0; k < d; k++) x[k] = ia.stuck[i] ? (T)0 : v[i * d + k];
+#pragma unroll
+        for(int k = 0; k < d; k++) {
+            const T v = first ? r[i * d + k] : beta * s[i * d + k] + r[i * d + k];
+            s[i * d + k] = v;
+            x[k] = ia.stuck[i] ? (T)0 : v;
+        }
         const uint8_t mask = ia.cmask[i];
         for(int j = 0; j < ia.nobj; j++) {
             if(!(mask & (1u << j))) continue;
@@ -457,16 +585,20 @@ template<class T, int d> __global__ void k_imp_mult_pre(ImpArgs<T> ia, T* tmp, c
             for(int k = 0; k < d; k++) dn += x[k] * n[k];
             for(int k = 0; k < d; k++) x[k] -= dn * n[k];
         }
+#pragma unroll
         for(int k = 0; k < d; k++) tmp[i * d + k] = x[k];
-    }
+    });
 }
 
 // ... and after it: f = (dt^2/m) H tmp + tmp, with the stuck nodes zeroed and
 // per collision f -= n (n.f) + dt (Hc v n_dE + (n.v) H_dE + (H_dE.v) n), v the
-// unprojected input (the curvature terms of MPM_KRYLOV_SYSTEM::Multiply).
-template<class T, int d> __global__ void k_imp_mult_post(ImpArgs<T> ia, T* f, const T* tmp, const T* v)
+// unprojected input (the curvature terms of MPM_KRYLOV_SYSTEM::Multiply); and
+// the product v.f.
+template<class T, int d> __global__ void __launch_bounds__(kRedThreads) k_cg_product(ImpArgs<T> ia, T* f, const T* tmp, const T* v,
+    Reduction red)
 {
-    NODE_LOOP(ia) {
+    double acc = 0;
+    mass_nodes(ia, [&](int64_t i) {
         const T s = ia.a.dt * ia.a.dt / ia.a.gm[i];
         T x[3];
         for(int k = 0; k < d; k++) x[k] = s * f[i * d + k] + tmp[i * d + k];
@@ -490,7 +622,30 @@ template<class T, int d> __global__ void k_imp_mult_post(ImpArgs<T> ia, T* f, co
                 x[k] -= n[k] * dn + ia.a.dt * (Hv[k] * cd[1] + nv * hde[k] + hv * n[k]);
         }
         for(int k = 0; k < d; k++) f[i * d + k] = x[k];
+        acc += node_dot<T, d>(ia, i, x, v + i * d);
+    });
+    grid_sum(acc, red);
+}
+
+// The step alpha = rho / s.q along s (none where s.q <= 0: the host ends there),
+// and the next rho = r.r.
+template<class T, int d> __global__ void __launch_bounds__(kRedThreads) k_cg_step(ImpArgs<T> ia, T* x, T* r, const T* s, const T* q,
+    double rho, const double* sq, Reduction red)
+{
+    double acc = 0;
+    if(!(*sq <= 0)) {
+        const T alpha = (T)(rho / *sq);
+        mass_nodes(ia, [&](int64_t i) {
+            T rn[3];
+#pragma unroll
+            for(int k = 0; k < d; k++) {
+                x[i * d + k] = alpha * s[i * d + k] + x[i * d + k];
+                r[i * d + k] = rn[k] = -alpha * q[i * d + k] + r[i * d + k];
+            }
+            acc += node_dot<T, d>(ia, i, rn, rn);
+        });
     }
+    grid_sum(acc, red);
 }
 
 // MPM_DRIVER::Apply_Friction, implicit branch (MPM_DRIVER.cpp:1064-1094):
@@ -499,7 +654,7 @@ template<class T, int d> __global__ void k_imp_mult_post(ImpArgs<T> ia, T* f, co
 // velocity_friction_save relative to v0.
 template<class T, int d> __global__ void k_imp_friction(ImpArgs<T> ia, const T* dv, const T* tmp0, const T* tmp1, T* vfs)
 {
-    NODE_LOOP(ia) {
+    mass_nodes(ia, [&](int64_t i) {
         const PlainArgs<T>& a = ia.a;
         T v[3];
         for(int k = 0; k < d; k++) {
@@ -526,90 +681,20 @@ template<class T, int d> __global__ void k_imp_friction(ImpArgs<T> ia, const T* 
             else for(int k = 0; k < d; k++) v[k] -= kf * t[k];
             for(int k = 0; k < d; k++) vfs[i * d + k] = v[k] - a.gv0[i * d + k];
         }
-    }
+    });
 }
 
 // The end of Apply_Forces (MPM_DRIVER.cpp:1049-1056): velocity = dv + v0,
 // velocity_friction_save += v0, stuck nodes at the object's velocity.
 template<class T, int d> __global__ void k_imp_finish(ImpArgs<T> ia, const T* dv, const T* vfs)
 {
-    NODE_LOOP(ia) {
+    mass_nodes(ia, [&](int64_t i) {
         const PlainArgs<T>& a = ia.a;
         for(int k = 0; k < d; k++) {
             a.gv[i * d + k] = dv[i * d + k] + a.gv0[i * d + k];
             a.gvf[i * d + k] = ia.stuck[i] ? ia.svel[i * d + k] : vfs[i * d + k] + a.gv0[i * d + k];
         }
-    }
-}
-
-// Deterministic reductions: a fixed grid writes one partial per block, one
-// block sums them in order.
-template<class T> __device__ double block_sum(double v)
-{
-    __shared__ double sh[kRedThreads];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for(int s = kRedThreads / 2; s > 0; s >>= 1) {
-        if(threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
-    }
-    return sh[0];
-}
-
-// MPM_KRYLOV_SYSTEM::Inner_Product (l.82-95): sum over nodes with mass of m x.y
-template<class T, int d> __global__ void k_imp_dot(ImpArgs<T> ia, const T* x, const T* y, double* partial)
-{
-    double acc = 0;
-    NODE_LOOP(ia) {
-        double s = 0;
-        for(int k = 0; k < d; k++) s += (double)x[i * d + k] * (double)y[i * d + k];
-        acc += (double)ia.a.gm[i] * s;
-    }
-    const double t = block_sum<T>(acc);
-    if(threadIdx.x == 0) partial[blockIdx.x] = t;
-}
-
-template<class T> __global__ void k_imp_sum_particles(const double* pe, int64_t n, double* partial)
-{
-    double acc = 0;
-    for(int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) acc += pe[p];
-    const double t = block_sum<T>(acc);
-    if(threadIdx.x == 0) partial[blockIdx.x] = t;
-}
-
-__device__ double block_sum_max(double v)
-{
-    __shared__ double sh[kRedThreads];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for(int s = kRedThreads / 2; s > 0; s >>= 1) {
-        if(threadIdx.x < s) sh[threadIdx.x] = fmax(sh[threadIdx.x], sh[threadIdx.x + s]);
-        __syncthreads();
-    }
-    return sh[0];
-}
-
-__global__ void k_imp_max_final(const double* partial, int count, double* out)
-{
-    if(threadIdx.x) return;
-    double r = partial[0];
-    for(int b = 1; b < count; b++) r = fmax(r, partial[b]);
-    *out = r;
-}
-
-// one block per result slot; the partials (count == blockDim.x) summed by a
-// fixed tree, so the result does not depend on scheduling
-__global__ void k_imp_final(const double* partial, int count, int slots, double* out)
-{
-    __shared__ double sh[kRedThreads];
-    const int s = blockIdx.x;
-    sh[threadIdx.x] = threadIdx.x < count ? partial[s * count + threadIdx.x] : 0.0;
-    __syncthreads();
-    for(int st = kRedThreads / 2; st > 0; st >>= 1) {
-        if(threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-        __syncthreads();
-    }
-    if(threadIdx.x == 0) out[s] = sh[0];
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -630,8 +715,9 @@ struct ImplicitState {
     uint8_t* stuck = nullptr;
     void* cdat = nullptr;
     double* partial = nullptr;     // 2 * kRedBlocks
+    unsigned* done = nullptr;      // finished CTAs of the 2 reductions
     double* dout = nullptr;        // 2 results
-    double* hout = nullptr;        // pinned copy
+    double* hout = nullptr;        // the same in pinned host memory
     uint32_t *keys = nullptr, *sorted = nullptr, *perm = nullptr, *alt_k = nullptr, *alt_v = nullptr, *scratch = nullptr;
     int key_bits = 1;
 };
@@ -643,7 +729,7 @@ template<class T, int d> struct Solver {
     ImpArgs<T> ia;
     T* v[V_COUNT];
     cudaStream_t st;
-    int pb, gb;
+    int pb, gb, rb;
     const mpm_implicit_desc& prm;
     int rc = MPM_OK;
     int krylov_total = 0;
@@ -662,6 +748,7 @@ template<class T, int d> struct Solver {
         ia.svel = v[V_SVEL];
         pb = pblocks(s.n, kScatterThreads);
         gb = gblocks(h, s.gn, 256);
+        rb = std::min(gb, kRedBlocks);
     }
     static int pblocks(int64_t n, int t) { int64_t b = (n + t - 1) / t; return (int)(b < 1 ? 1 : b); }
     static int gblocks(mpm_handle* h, int64_t n, int t)
@@ -677,12 +764,15 @@ template<class T, int d> struct Solver {
     }
 
     // reductions ----------------------------------------------------------
+    Reduction reduction(int slot)
+    {
+        ImplicitState& s = *h->imp;
+        return {s.partial + slot * kRedBlocks, s.done + slot, s.dout + slot, s.hout + slot};
+    }
     double dot(const T* x, const T* y)
     {
         ImplicitState& s = *h->imp;
-        k_imp_dot<T, d><<<kRedBlocks, kRedThreads, 0, st>>>(ia, x, y, s.partial);
-        k_imp_final<<<1, kRedThreads, 0, st>>>(s.partial, kRedBlocks, 1, s.dout);
-        cudaMemcpyAsync(s.hout, s.dout, sizeof(double), cudaMemcpyDeviceToHost, st);
+        k_imp_dot<T, d><<<rb, kRedThreads, 0, st>>>(ia, x, y, reduction(0));
         cudaStreamSynchronize(st);
         check("implicit dot");
         return s.hout[0];
@@ -691,10 +781,8 @@ template<class T, int d> struct Solver {
     double energy(const T* x)
     {
         ImplicitState& s = *h->imp;
-        k_imp_dot<T, d><<<kRedBlocks, kRedThreads, 0, st>>>(ia, x, x, s.partial);
-        k_imp_sum_particles<T><<<kRedBlocks, kRedThreads, 0, st>>>(s.pe, s.n, s.partial + kRedBlocks);
-        k_imp_final<<<2, kRedThreads, 0, st>>>(s.partial, kRedBlocks, 2, s.dout);
-        cudaMemcpyAsync(s.hout, s.dout, 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
+        k_imp_dot<T, d><<<rb, kRedThreads, 0, st>>>(ia, x, x, reduction(0));
+        k_imp_sum_particles<<<rb, kRedThreads, 0, st>>>(s.pe, s.n, reduction(1));
         cudaStreamSynchronize(st);
         check("implicit energy");
         return s.hout[0] / 2 + s.hout[1];
@@ -702,7 +790,7 @@ template<class T, int d> struct Solver {
 
     // vector ops on nodes with mass ---------------------------------------
     void copy(T* out, T c, const T* x, const T* y = nullptr) { k_imp_copy<T, d><<<gb, 256, 0, st>>>(ia, out, c, x, y); }
-    void zero(T* x) { cudaMemsetAsync(x, 0, (size_t)ia.a.gn * d * sizeof(T), st); }
+    void zero(T* x, int count = 1) { k_imp_zero<T, d><<<gb, 256, 0, st>>>(ia, x, ia.a.gn * d, count); }
 
     // MPM_OBJECTIVE ----------------------------------------------------------
     void adjust(T* x)
@@ -739,15 +827,6 @@ template<class T, int d> struct Solver {
     }
     void make_feasible(T* x) { adjust(x); }
 
-    // MPM_KRYLOV_SYSTEM::Multiply
-    void multiply(const T* x, T* out)
-    {
-        k_imp_mult_pre<T, d><<<gb, 256, 0, st>>>(ia, v[V_STMP], x);
-        zero(out);
-        k_imp_hessian<T, d><<<pb, kScatterThreads, 0, st>>>(ia, v[V_STMP], out);
-        k_imp_mult_post<T, d><<<gb, 256, 0, st>>>(ia, out, v[V_STMP], x);
-    }
-
     // CONJUGATE_GRADIENT::Solve with relative tolerance and
     // finish_before_indefiniteness; x = 0 on entry.
     bool cg(T* x, const T* b, double tolerance, int max_iterations, int& used)
@@ -755,27 +834,29 @@ template<class T, int d> struct Solver {
         T *q = v[V_Q], *s = v[V_S], *r = v[V_R];
         double rho_old = FLT_MAX;
         copy(r, 1, b);                // r = b - A 0
+        double rho = dot(r, r);       // no preconditioner: rho = |r|^2
         int it;
         for(it = 0;; it++) {
-            const double rho = dot(r, r);      // no preconditioner: rho = |r|^2
             const double cn = sqrt(rho);
             if(failed()) return false;
             if(it == 0) tolerance *= cn;
             if(cn <= tolerance) { used = it; return true; }   // min_iterations 0
             if(it == max_iterations) break;
-            if(it == 0) copy(s, 1, r);
-            else copy(s, (T)(rho / rho_old), s, r);
-            multiply(s, q);
-            const double sq = dot(s, q);
+            ImplicitState& is = *h->imp;
+            k_cg_direction<T, d><<<gb, 256, 0, st>>>(ia, s, r, it ? (T)(rho / rho_old) : (T)0, it == 0, v[V_STMP], q);
+            k_imp_hessian<T, d><<<pb, kScatterThreads, 0, st>>>(ia, v[V_STMP], q);
+            k_cg_product<T, d><<<rb, kRedThreads, 0, st>>>(ia, q, v[V_STMP], s, reduction(0));
+            k_cg_step<T, d><<<rb, kRedThreads, 0, st>>>(ia, x, r, s, q, rho, is.dout, reduction(1));
+            cudaStreamSynchronize(st);
+            check("implicit cg");
+            const double sq = is.hout[0];
             if(sq <= 0) {
                 if(it == 0) copy(x, 1, b);
                 used = it;
                 return true;
             }
-            const double alpha = sq ? rho / sq : (double)FLT_MAX;
-            copy(x, (T)alpha, s, x);
-            copy(r, (T)-alpha, q, r);
             rho_old = rho;
+            rho = is.hout[1];
         }
         used = it;
         return false;
@@ -906,7 +987,7 @@ template<class T, int d> struct Solver {
             ia.order = s.perm;
             k_imp_save<T, d><<<pb, 128, 0, st>>>(ia);
         }
-        for(int k = 0; k < V_COUNT; k++) zero(v[k]);
+        zero(v[0], V_COUNT);
         if(ia.nobj) {
             cudaMemsetAsync(s.cmask, 0, s.gn, st);
             cudaMemsetAsync(s.stuck, 0, s.gn, st);
@@ -960,6 +1041,8 @@ template<class T> int ensure_state(mpm_handle* h)
     MPM_CUDA(h, cudaMemset(t.stuck, 0, (size_t)t.gn));
     if(t.nobj) MPM_CUDA(h, cudaMalloc(&t.cdat, (size_t)t.gn * t.nobj * (2 + 3 * d) * e));
     MPM_CUDA(h, cudaMalloc(&t.partial, 2 * kRedBlocks * sizeof(double)));
+    MPM_CUDA(h, cudaMalloc(&t.done, 2 * sizeof(unsigned)));
+    MPM_CUDA(h, cudaMemset(t.done, 0, 2 * sizeof(unsigned)));
     MPM_CUDA(h, cudaMalloc(&t.dout, 2 * sizeof(double)));
     MPM_CUDA(h, cudaMallocHost(&t.hout, 2 * sizeof(double)));
     uint32_t** sb[] = {&t.keys, &t.sorted, &t.perm, &t.alt_k, &t.alt_v};
@@ -992,12 +1075,15 @@ template<class T, int d> __global__ void k_imp_sound(ImpArgs<T> ia, double* part
 {
     const PlainArgs<T>& a = ia.a;
     double smax = 0;
-    for(int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n; p += (int64_t)gridDim.x * blockDim.x) {
+    for(int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < a.n; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = particle_at(ia, t);
         if(!a.valid[p]) continue;
-        const T* blk = ia.dP + p * 15;
-        smax = fmax(smax, (double)sound_speed<T, d>(ia.sig + p * d, blk, blk + 9, a.mass[p] / a.vol[p]));
+        T sig[3], blk[12];
+        for(int e = 0; e < d; e++) sig[e] = ia.sig[e * a.n + t];
+        for(int e = 0; e < 12; e++) blk[e] = ia.dP[e * a.n + t];
+        smax = fmax(smax, (double)sound_speed<T, d>(sig, blk, blk + 9, a.mass[p] / a.vol[p]));
     }
-    const double r = block_sum_max(smax);
+    const double r = block_max(smax);
     if(threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
@@ -1006,12 +1092,14 @@ template<class T> int implicit_sound_t(mpm_handle* h, double* partial, double* o
     if(!h->imp) return set_error(h, MPM_ERR_STATE, "no implicit solve yet");
     if(h->sp.dim == 3) {
         Solver<T, 3> sv(h, 0.0);
-        k_imp_sound<T, 3><<<kRedBlocks, kRedThreads, 0, h->stream>>>(sv.ia, partial);
+        sv.ia.order = h->imp->perm;
+        k_imp_sound<T, 3><<<kSoundBlocks, kRedThreads, 0, h->stream>>>(sv.ia, partial);
     } else {
         Solver<T, 2> sv(h, 0.0);
-        k_imp_sound<T, 2><<<kRedBlocks, kRedThreads, 0, h->stream>>>(sv.ia, partial);
+        sv.ia.order = h->imp->perm;
+        k_imp_sound<T, 2><<<kSoundBlocks, kRedThreads, 0, h->stream>>>(sv.ia, partial);
     }
-    k_imp_max_final<<<1, 32, 0, h->stream>>>(partial, kRedBlocks, out);
+    k_imp_max_final<<<1, 32, 0, h->stream>>>(partial, kSoundBlocks, out);
     return MPM_OK;
 }
 }  // namespace
@@ -1026,7 +1114,7 @@ void implicit_free(mpm_handle* h)
     if(!h->imp) return;
     ImplicitState& s = *h->imp;
     cudaFree(s.vec); cudaFree(s.part); cudaFree(s.pe); cudaFree(s.cmask); cudaFree(s.stuck); cudaFree(s.cdat);
-    cudaFree(s.partial); cudaFree(s.dout);
+    cudaFree(s.partial); cudaFree(s.done); cudaFree(s.dout);
     cudaFree(s.keys); cudaFree(s.sorted); cudaFree(s.perm); cudaFree(s.alt_k); cudaFree(s.alt_v); cudaFree(s.scratch);
     if(s.hout) cudaFreeHost(s.hout);
     delete h->imp;
