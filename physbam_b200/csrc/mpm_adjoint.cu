@@ -29,7 +29,11 @@
 //   adj_p2g  (per particle; the adjoint of the scatter is a gather), incl. the stress.
 // The forward is recomputed segment by segment from checkpoints taken every k
 // substeps; inside a segment each substep's particle state, grid mass and
-// velocity and P F^T are kept.
+// velocity and P F^T are kept, and the list of its grid tiles (the adjoint's node
+// passes visit those).  The substep writes them into the tape itself (PlainRecord):
+// G2P moves the particles from one slot's state to the next, the grid update
+// writes the slot's mass and velocities.  Eight copies and a pass over the grid
+// per substep did before, and a third of a rollout's time was launches.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -39,6 +43,7 @@
 #include <algorithm>
 
 #include "mpm_internal.h"
+#include "mpm_plain.cuh"
 #include "mpm_scatter.cuh"
 
 namespace {
@@ -59,6 +64,8 @@ template<class T> struct AdjArgs {
     T *aX0, *aV0, *aB0, *aF0;       // adjoints of its inputs
     T *amu, *alam;                  // accumulated over substeps
     T* ga;                          // grid: v-bar, then p-bar in place
+    T* ga_next;                     // ... of the substep before, to be cleared (null: none)
+    const uint32_t *tiles, *tile_count, *next_tiles, *next_count;   // the two substeps' node tiles (null: every node)
     T* gma;                         // grid: m-bar
     T dt;
     unsigned* flags;
@@ -261,9 +268,9 @@ template<class T> __device__ void adj_collide(const AdjArgs<T>& a, int64_t i, co
 
 template<class T> __global__ void k_adj_grid(AdjArgs<T> a)
 {
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.gn; i += (int64_t)gridDim.x * blockDim.x) {
+    plain::for_tiles(a.gn, a.tiles, a.tile_count, [&](int64_t i) {
         T m = a.gm[i];
-        if(m == 0) { a.gma[i] = 0; continue; }
+        if(m == 0) { a.gma[i] = 0; return; }
         T vb[3] = {a.ga[3 * i], a.ga[3 * i + 1], a.ga[3 * i + 2]};
         const T* u = a.gu + 3 * i;
         if(a.sp.nobj) adj_collide<T>(a, i, u, vb);
@@ -274,18 +281,12 @@ template<class T> __global__ void k_adj_grid(AdjArgs<T> a)
             a.ga[3 * i + k] = vb[k] * im;
         }
         a.gma[i] = -s * im;
-    }
-}
-
-// The grid velocity before the collision projection, as the grid update forms
-// it: u = v0 + (dt / m) f.
-template<class T> __global__ void k_grid_u(const T* gv0, const T* gf, const T* gm, T dt, int64_t gn, T* u)
-{
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < gn; i += (int64_t)gridDim.x * blockDim.x) {
-        const T m = gm[i];
-        const T s = m != 0 ? dt / m : (T)0;
-        for(int k = 0; k < 3; k++) u[3 * i + k] = gv0[3 * i + k] + s * gf[3 * i + k];
-    }
+    });
+    if(a.ga_next)
+        plain::for_tiles(a.gn, a.next_tiles, a.next_count, [&](int64_t i) {
+#pragma unroll
+            for(int k = 0; k < 3; k++) a.ga_next[3 * i + k] = 0;
+        });
 }
 
 // Stress blocks in the SVD frame (the reference's Isotropic_Stress_Derivative_Helper)
@@ -452,9 +453,13 @@ template<class T> __global__ void k_adj_p2g(AdjArgs<T> a)
     a.alam[p] += (T)bla;
 }
 
-template<class T> __global__ void k_zero(T* p, int64_t n)
+// v-bar of a segment's last substep to zero (k_adj_grid clears the others')
+template<class T> __global__ void k_adj_clear(T* ga, int64_t gn, const uint32_t* tiles, const uint32_t* count)
 {
-    for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = 0;
+    plain::for_tiles(gn, tiles, count, [&](int64_t i) {
+#pragma unroll
+        for(int k = 0; k < 3; k++) ga[3 * i + k] = 0;
+    });
 }
 
 int blocks_for(mpm_handle* h, int64_t n, int t, bool cap)
@@ -479,10 +484,12 @@ struct DiffTape {
     void* seg = nullptr;             // every (or, full, nsteps) states
     uint8_t* seg_valid = nullptr;
     void *seg_gm = nullptr, *seg_gv = nullptr, *seg_gu = nullptr, *seg_pft = nullptr;
+    int64_t ntiles = 0;                             // node tiles of the grid; 0: not listed
+    uint32_t *seg_tiles = nullptr, *seg_count = nullptr;
     void* final_state = nullptr;
     uint8_t* final_valid = nullptr;
     void *adj[2] = {nullptr, nullptr};   // X V F B adjoints, double-buffered
-    void *amu = nullptr, *alam = nullptr, *ga = nullptr, *gma = nullptr;
+    void *amu = nullptr, *alam = nullptr, *ga[2] = {nullptr, nullptr}, *gma = nullptr;
 };
 
 static DiffTape* tape(mpm_handle* h) { return reinterpret_cast<DiffTape*>(h->diff); }
@@ -500,7 +507,8 @@ void diff_free(mpm_handle* h)
     DiffTape* t = tape(h);
     if(!t) return;
     void* ps[] = {t->ckpt, t->ckpt_valid, t->seg, t->seg_valid, t->seg_gm, t->seg_gv, t->seg_gu, t->seg_pft, t->final_state,
-                  t->final_valid, t->adj[0], t->adj[1], t->amu, t->alam, t->ga, t->gma};
+                  t->final_valid, t->adj[0], t->adj[1], t->amu, t->alam, t->ga[0], t->ga[1], t->gma, t->seg_tiles,
+                  t->seg_count};
     for(void* p: ps) cudaFree(p);
     delete t;
     h->diff = nullptr;
@@ -524,25 +532,30 @@ static int state_copy(mpm_handle* h, void* dst, uint8_t* dvalid, bool to_tape)
     return MPM_OK;
 }
 
-// One substep of the rollout with its intermediates into tape slot j: the
-// state before it, the node masses and velocities after the forces, the grid
-// update's velocity map (k_grid_u) and P F^T; `advance`: the G2P that ends it.
-template<class T> static int record_substep(mpm_handle* h, DiffTape* t, int j, bool advance)
+// One substep of the rollout from the state in tape slot j, its intermediates
+// (node masses, velocities after the forces and before the collision
+// projection, P F^T, tile list) into the slot; `advance`: the G2P that ends it, into
+// slot j + 1 or, `leave`, into the handle's particles.
+template<class T> static int record_substep(mpm_handle* h, DiffTape* t, int j, bool advance, bool leave)
 {
-    PlainState& s = h->plain;
     const int64_t n = t->n, gn = t->gn;
-    const size_t e = sizeof(T), st = 24 * n * e;
-    int rc;
-    if((rc = state_copy(h, (char*)t->seg + j * st, t->seg_valid + j * n, true))) return rc;
-    if((rc = plain_p2g_forces(h, t->dt))) return rc;
-    MPM_CUDA(h, cudaMemcpyAsync((T*)t->seg_gm + j * gn, s.gm, gn * e, cudaMemcpyDeviceToDevice, h->stream));
-    MPM_CUDA(h, cudaMemcpyAsync((T*)t->seg_gv + j * gn * 3, s.gv, gn * 3 * e, cudaMemcpyDeviceToDevice, h->stream));
-    k_grid_u<T><<<blocks_for(h, gn, 256, true), 256, 0, h->stream>>>((const T*)s.gv0, (const T*)s.gf, (const T*)s.gm,
-                                                                   (T)t->dt, gn, (T*)t->seg_gu + j * gn * 3);
-    MPM_LAUNCHED(h, "k_grid_u");
-    MPM_CUDA(h, cudaMemcpyAsync((T*)t->seg_pft + j * 9 * n, s.pft, 9 * n * e, cudaMemcpyDeviceToDevice, h->stream));
-    if(advance && (rc = plain_g2p(h, t->dt, 0))) return rc;
-    return MPM_OK;
+    const size_t st = 24 * n * sizeof(T);
+    PlainRecord r;
+    r.in = (char*)t->seg + j * st;
+    r.valid = t->seg_valid + j * n;
+    r.out = advance && !leave ? (char*)r.in + st : nullptr;
+    r.out_valid = r.out ? r.valid + n : nullptr;
+    r.pft = (T*)t->seg_pft + j * 9 * n;
+    r.gm = (T*)t->seg_gm + j * gn;
+    r.gv = (T*)t->seg_gv + j * gn * 3;
+    r.gu = (T*)t->seg_gu + j * gn * 3;
+    r.tiles = t->ntiles ? t->seg_tiles + j * t->ntiles : nullptr;
+    r.tile_count = t->ntiles ? t->seg_count + j : nullptr;
+    h->plain.record = &r;
+    int rc = plain_p2g_forces(h, t->dt);
+    if(!rc && advance) rc = plain_g2p(h, t->dt, 0);
+    h->plain.record = nullptr;
+    return rc;
 }
 
 // Tape slots for `slots` substeps (the segment buffers the backward reads).
@@ -556,11 +569,19 @@ static int alloc_segments(mpm_handle* h, DiffTape* t, int slots)
     MPM_CUDA(h, cudaMalloc(&t->seg_gv, slots * gn * 3 * e));
     MPM_CUDA(h, cudaMalloc(&t->seg_gu, slots * gn * 3 * e));
     MPM_CUDA(h, cudaMalloc(&t->seg_pft, slots * 9 * n * e + 1));
+    t->ntiles = plain_listed(h) ? (gn + plain::kTileNodes - 1) / plain::kTileNodes : 0;
+    if(t->ntiles) {
+        MPM_CUDA(h, cudaMalloc(&t->seg_tiles, slots * t->ntiles * sizeof(uint32_t)));
+        MPM_CUDA(h, cudaMalloc(&t->seg_count, slots * sizeof(uint32_t)));
+    }
     return MPM_OK;
 }
 
 // Bytes of the tape slots of one substep.
-static size_t slot_bytes(int64_t n, int64_t gn, size_t e) { return (24 * n + 9 * n) * e + n + 7 * gn * e; }
+static size_t slot_bytes(int64_t n, int64_t gn, size_t e)
+{
+    return (24 * n + 9 * n) * e + n + 7 * gn * e + (gn / plain::kTileNodes + 2) * sizeof(uint32_t);
+}
 
 int diff_forward(mpm_handle* h, double dt, int nsteps, int every)
 {
@@ -614,7 +635,9 @@ int diff_forward(mpm_handle* h, double dt, int nsteps, int every)
     int rc;
     for(int k = 0; k < nsteps; k++) {
         if(t->full) {
-            rc = esz == 8 ? record_substep<double>(h, t, k, true) : record_substep<float>(h, t, k, true);
+            if(k == 0 && (rc = state_copy(h, t->seg, t->seg_valid, true))) return rc;
+            rc = esz == 8 ? record_substep<double>(h, t, k, true, k + 1 == nsteps)
+                          : record_substep<float>(h, t, k, true, k + 1 == nsteps);
             if(rc) return rc;
             continue;
         }
@@ -647,7 +670,7 @@ template<class T> static int backward_t(mpm_handle* h, const void* gX, const voi
         for(int k = 0; k < 2; k++) MPM_CUDA(h, cudaMalloc(&t->adj[k], st + 1));
         MPM_CUDA(h, cudaMalloc(&t->amu, n * e + 1));
         MPM_CUDA(h, cudaMalloc(&t->alam, n * e + 1));
-        MPM_CUDA(h, cudaMalloc(&t->ga, gn * 3 * e));
+        for(int k = 0; k < 2; k++) MPM_CUDA(h, cudaMalloc(&t->ga[k], gn * 3 * e));
         MPM_CUDA(h, cudaMalloc(&t->gma, gn * e));
     }
     // seed: adjoint of the final state (device arrays of T)
@@ -668,10 +691,18 @@ template<class T> static int backward_t(mpm_handle* h, const void* gX, const voi
     for(int c = nck - 1; c >= 0; c--) {
         int k0 = c * span, k1 = k0 + span < t->nsteps ? k0 + span : t->nsteps;
         if(!t->full) {
-            if((rc = state_copy(h, (char*)t->ckpt + c * st, t->ckpt_valid + c * n, false))) return rc;
+            MPM_CUDA(h, cudaMemcpyAsync(t->seg, (char*)t->ckpt + c * st, st, cudaMemcpyDeviceToDevice, h->stream));
+            MPM_CUDA(h, cudaMemcpyAsync(t->seg_valid, t->ckpt_valid + c * n, n, cudaMemcpyDeviceToDevice, h->stream));
             for(int k = k0; k < k1; k++)
-                if((rc = record_substep<T>(h, t, k - k0, k + 1 < k1))) return rc;
+                if((rc = record_substep<T>(h, t, k - k0, k + 1 < k1, false))) return rc;
         }
+        auto list = [&](int j) { return t->ntiles ? t->seg_tiles + j * t->ntiles : nullptr; };
+        auto count = [&](int j) { return t->ntiles ? t->seg_count + j : nullptr; };
+        int cur = 0;
+        const int slot = timer_begin(h, "adj_clear");
+        k_adj_clear<T><<<blocks_for(h, gn, 256, true), 256, 0, h->stream>>>((T*)t->ga[0], gn, list(k1 - 1 - k0), count(k1 - 1 - k0));
+        timer_end(h, slot);
+        MPM_LAUNCHED(h, "k_adj_clear");
         for(int k = k1 - 1; k >= k0; k--) {
             int j = k - k0;
             const T* base = (const T*)((char*)t->seg + j * st);
@@ -689,14 +720,14 @@ template<class T> static int backward_t(mpm_handle* h, const void* gX, const voi
             a.aX1 = a1; a.aV1 = a1 + 3 * n; a.aF1 = a1 + 6 * n; a.aB1 = a1 + 15 * n;
             a.aX0 = a0; a.aV0 = a0 + 3 * n; a.aF0 = a0 + 6 * n; a.aB0 = a0 + 15 * n;
             a.amu = (T*)t->amu; a.alam = (T*)t->alam;
-            a.ga = (T*)t->ga; a.gma = (T*)t->gma;
+            a.ga = (T*)t->ga[cur]; a.gma = (T*)t->gma;
+            a.ga_next = j ? (T*)t->ga[cur ^ 1] : nullptr;
+            a.tiles = list(j); a.tile_count = count(j);
+            a.next_tiles = j ? list(j - 1) : nullptr; a.next_count = j ? count(j - 1) : nullptr;
+            cur ^= 1;
             a.dt = (T)t->dt;
             a.flags = h->d_flags;
-            int slot = timer_begin(h, "adj_zero");
-            k_zero<T><<<blocks_for(h, gn * 3, 256, true), 256, 0, h->stream>>>(a.ga, gn * 3);
-            timer_end(h, slot);
-            MPM_LAUNCHED(h, "k_zero");
-            slot = timer_begin(h, "adj_g2p");
+            int slot = timer_begin(h, "adj_g2p");
             k_adj_g2p<T><<<blocks_for(h, n, tb, false), tb, 0, h->stream>>>(a);
             timer_end(h, slot);
             MPM_LAUNCHED(h, "k_adj_g2p");

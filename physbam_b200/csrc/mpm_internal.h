@@ -24,6 +24,16 @@ struct SceneParams {
 };
 
 // Reference-layout device arrays for the plain path (one thread per particle).
+// One substep of a recorded rollout (mpm_adjoint.cu, 3D): the particles are read from
+// `in` (X 3n, V 3n, F 9n, B 9n scalars) and G2P writes them to `out` (null: to the
+// handle's own arrays); P F^T, node mass, velocity and velocity before the
+// collision projection and the tile list go into the record.
+struct PlainRecord {
+    void *in, *out, *pft, *gm, *gv, *gu;
+    uint8_t *valid, *out_valid;
+    uint32_t *tiles, *tile_count;
+};
+
 struct PlainState {
     int64_t n = 0, gn = 0;
     void *X = nullptr, *V = nullptr, *F = nullptr, *B = nullptr;
@@ -36,6 +46,7 @@ struct PlainState {
     uint8_t* tile_flag = nullptr;
     uint32_t *tiles = nullptr, *tile_count = nullptr;
     bool grid_listed = false;
+    const PlainRecord* record = nullptr;   // set while a rollout's substep is recorded
     void *Fp = nullptr, *mu0 = nullptr, *lam0 = nullptr;   // plastic state (plasticity on): clamp
     void *pdef = nullptr, *rhoF = nullptr, *sigY = nullptr, *vc = nullptr;   // Drucker-Prager
     uint8_t* pmodel = nullptr;   // per-particle constitutive model (null: the handle's model)
@@ -218,6 +229,7 @@ void plain_free(mpm_handle* h);
 int plain_set_particles(mpm_handle* h, const mpm_particles_view* v);
 int plain_get_particles(mpm_handle* h, mpm_particles_view* v);
 int plain_prepare(mpm_handle* h);
+bool plain_listed(const mpm_handle* h);
 int plain_p2g(mpm_handle* h, double dt, double time);
 int plain_p2g_forces(mpm_handle* h, double dt);
 int plain_forces(mpm_handle* h, double dt, double time);

@@ -45,7 +45,8 @@ template<class T> __global__ void k_clear(PlainArgs<T> a)
 // tiles; the flags before its own it counts itself (one byte each, 0 or 1, read
 // as 16-byte words), so the list takes one launch and no CTA waits for another.
 constexpr int kTileSpan = 1024, kTileThreads = 256;
-__global__ void __launch_bounds__(kTileThreads) k_tile_list(const uint8_t* flag, int64_t ntiles, uint32_t* tiles, uint32_t* count)
+__global__ void __launch_bounds__(kTileThreads) k_tile_list(const uint8_t* flag, int64_t ntiles, uint32_t* tiles, uint32_t* count,
+    uint32_t* rec_tiles, uint32_t* rec_count)   // and the same into a rollout's record, or null
 {
     __shared__ uint32_t s_warp[kTileThreads / 32], s_before[kTileThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -78,8 +79,16 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_list(const uint8_t* flag,
     }
 #pragma unroll
     for(int k = 0; k < 4; k++)
-        if((mine >> (8 * k)) & 1u) tiles[at++] = (uint32_t)(first + 4 * threadIdx.x + k);
-    if(blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count = total;
+        if((mine >> (8 * k)) & 1u) {
+            const uint32_t t = (uint32_t)(first + 4 * threadIdx.x + k);
+            tiles[at] = t;
+            if(rec_tiles) rec_tiles[at] = t;
+            at++;
+        }
+    if(blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        *count = total;
+        if(rec_count) *rec_count = total;
+    }
 }
 
 // Factors of the particle's forces: MPM_FINITE_ELEMENTS::Add_Forces
@@ -195,6 +204,11 @@ template<class T, int d, bool NORMALIZE> __global__ void k_grid_update(PlainArgs
 {
     for_nodes(a, [&](int64_t i) {
         T m = a.gm[i];
+        if(a.rm) {
+            a.rm[i] = m;
+            if(m == 0)
+                for(int k = 0; k < d; k++) a.rv[i * d + k] = 0;
+        }
         if(m == 0) return;
         T dv[3], v0[3], X0[3], vn[3], vf[3];
         T s = a.dt / m;
@@ -206,12 +220,25 @@ template<class T, int d, bool NORMALIZE> __global__ void k_grid_update(PlainArgs
             dv[k] = s * a.gf[i * d + k];
             if(NORMALIZE) a.gv0[i * d + k] = v0[k] = a.gmv[i * d + k] / m;
             else v0[k] = a.gv0[i * d + k];
+            if(a.rm) a.ru[i * d + k] = v0[k] + dv[k];   // collide_node changes dv
             X0[k] = (T)a.sp.dmin[k] + ((T)idx[k] + (T).5) * (T)a.sp.dx[k];
         }
         collide_node<T, d>(a.sp.objs, a.sp.nobj, X0, v0, dv, a.dt, vn, vf, a.motion, a.moving);
 #pragma unroll
         for(int k = 0; k < d; k++) { a.gv[i * d + k] = vn[k]; a.gvf[i * d + k] = vf[k]; }
+        if(a.rm)
+#pragma unroll
+            for(int k = 0; k < d; k++) a.rv[i * d + k] = vn[k];
     });
+}
+
+// A particle that G2P leaves as it is, where G2P does not write in place.
+template<class T, int d> __device__ __forceinline__ void keep_particle(const PlainArgs<T>& a, int64_t p)
+{
+    if(a.oX == a.X) return;
+    for(int k = 0; k < d; k++) { a.oX[p * d + k] = a.X[p * d + k]; a.oV[p * d + k] = a.V[p * d + k]; }
+    for(int k = 0; k < d * d; k++) { a.oF[p * d * d + k] = a.F[p * d * d + k]; a.oB[p * d * d + k] = a.B[p * d * d + k]; }
+    a.ovalid[p] = a.valid[p];
 }
 
 // MPM_DRIVER::Grid_To_Particle (MPM_DRIVER.cpp:450-515) and
@@ -219,10 +246,13 @@ template<class T, int d, bool NORMALIZE> __global__ void k_grid_update(PlainArgs
 template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
 {
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if(p >= a.n || !a.valid[p]) return;
-    T* X = a.X + p * d;
+    if(p >= a.n) return;
+    const T* X = a.X + p * d;
     Stencil<T, d> s;
-    if(!make_stencil<T, d>(a, X, s)) return;
+    if(!a.valid[p] || !make_stencil<T, d>(a, X, s)) {
+        keep_particle<T, d>(a, p);
+        return;
+    }
     T Vpic[3] = {0, 0, 0}, Vpf[3] = {0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, Bh[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     const int nq = d == 3 ? 27 : 9;
     for(int q = 0; q < nq; q++) {
@@ -250,7 +280,7 @@ template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
 #pragma unroll
             for(int r = 0; r < d; r++) Bh[r + d * c] += hw * (vf[r] * Zp[c] + Zm[r] * vf[c]);
     }
-    T* Fp = a.F + p * d * d;
+    const T* Fp = a.F + p * d * d;
     T A[9], Fn[9];
 #pragma unroll
     for(int e = 0; e < d * d; e++) A[e] = a.dt * G[e];
@@ -269,14 +299,14 @@ template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
     bool finite = true;
 #pragma unroll
     for(int k = 0; k < d; k++) xn[k] = X[k] + a.dt * Vpic[k];
-    T* Bp = a.B + p * d * d;
+    T* Bp = a.oB + p * d * d;
 #pragma unroll
     for(int c = 0; c < d; c++)
 #pragma unroll
         for(int r = 0; r < d; r++)
             Bp[r + d * c] = Bh[r + d * c] - (T).5 * (Vpf[r] * (X[c] + xn[c]) + (X[r] - xn[r]) * Vpf[c]);
 #pragma unroll
-    for(int e = 0; e < d * d; e++) { Fp[e] = Fn[e]; finite = finite && isfinite(Fn[e]); }
+    for(int e = 0; e < d * d; e++) { a.oF[p * d * d + e] = Fn[e]; finite = finite && isfinite(Fn[e]); }
     // Reflect_Or_Invalidate_Particle (l.1219-1239): mirrored back across a
     // non-free face, invalidated across a free one
     bool keep = true;
@@ -293,13 +323,14 @@ template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
             if(a.side[2 * k + 1] != MPM_BC_FREE) { x = 2 * B - x; v = -v; }
             else keep = false;
         }
-        X[k] = x;
-        a.V[p * d + k] = v;
+        a.oX[p * d + k] = x;
+        a.oV[p * d + k] = v;
     }
     if(!finite) { atomicOr(a.flags, MPM_FLAG_NAN); keep = false; }
     // a particle that leaves is marked 2 while plasticity still has to see it
     // (the reference updates every particle simulated in this substep)
-    if(!keep) a.valid[p] = a.mark_left ? 2 : 0;
+    if(!keep) a.ovalid[p] = a.mark_left ? 2 : 0;
+    else if(a.ovalid != a.valid) a.ovalid[p] = a.valid[p];
 }
 
 template<class T> __global__ void k_count_valid(const uint8_t* valid, int64_t n, unsigned long long* out)
@@ -541,8 +572,9 @@ template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
     if(a.tile_flag) {
         const int64_t nt = (a.gn + kTileNodes - 1) / kTileNodes;
         slot = timer_begin(h, "plain_tiles");
-        k_tile_list<<<(unsigned)((nt + kTileSpan - 1) / kTileSpan), kTileThreads, 0, h->stream>>>(a.tile_flag, nt, h->plain.tiles,
-                                                                                               h->plain.tile_count);
+        const PlainRecord* r = h->plain.record;
+        k_tile_list<<<(unsigned)((nt + kTileSpan - 1) / kTileSpan), kTileThreads, 0, h->stream>>>(
+            a.tile_flag, nt, h->plain.tiles, h->plain.tile_count, r ? r->tiles : nullptr, r ? r->tile_count : nullptr);
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_tile_list");
     }
@@ -931,6 +963,8 @@ int plain_prepare(mpm_handle* h)
     s.grid_listed = true;
     return MPM_OK;
 }
+
+bool plain_listed(const mpm_handle* h) { return list_tiles(h); }
 
 void plain_free(mpm_handle* h)
 {

@@ -16,6 +16,12 @@ template<class T> struct PlainArgs {
     T* pft;
     uint8_t* valid;
     T *gm, *gmv, *gv0, *gf, *gv, *gvf;
+    // where G2P writes the particles (their own arrays, or a recorded rollout's next
+    // state), and the grid update's record of mass, velocity and velocity before the
+    // collision projection (null: none)
+    T *oX, *oV, *oF, *oB;
+    uint8_t* ovalid;
+    T *rm, *rv, *ru;
     T dt;
     unsigned* flags;
     int mark_left;
@@ -31,15 +37,20 @@ template<class T> struct PlainArgs {
 
 constexpr int kTileNodes = 32;
 
-// f(i) over the nodes of the listed tiles (a warp per tile), or over every node.
-template<class T, class FN> __device__ __forceinline__ void for_nodes(const PlainArgs<T>& a, FN&& f)
+// f(i) over the nodes of the listed tiles (a warp per tile), or over all gn nodes.
+template<class FN> __device__ __forceinline__ void for_tiles(int64_t gn, const uint32_t* tiles, const uint32_t* count, FN&& f)
 {
-    const uint32_t nt = a.tiles ? *a.tile_count : (uint32_t)((a.gn + kTileNodes - 1) / kTileNodes);
+    const uint32_t nt = tiles ? *count : (uint32_t)((gn + kTileNodes - 1) / kTileNodes);
     const uint32_t nw = gridDim.x * (blockDim.x >> 5);
     for(uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < nt; t += nw) {
-        const int64_t i = (int64_t)(a.tiles ? a.tiles[t] : t) * kTileNodes + (threadIdx.x & 31);
-        if(i < a.gn) f(i);
+        const int64_t i = (int64_t)(tiles ? tiles[t] : t) * kTileNodes + (threadIdx.x & 31);
+        if(i < gn) f(i);
     }
+}
+
+template<class T, class FN> __device__ __forceinline__ void for_nodes(const PlainArgs<T>& a, FN&& f)
+{
+    for_tiles(a.gn, a.tiles, a.tile_count, f);
 }
 
 // Grids of this many nodes and more are passed over by the list of tiles that
@@ -131,6 +142,19 @@ template<class T> inline PlainArgs<T> args(mpm_handle* h, double dt)
     a.X = (T*)s.X; a.V = (T*)s.V; a.F = (T*)s.F; a.B = (T*)s.B;
     a.mass = (const T*)s.mass; a.vol = (const T*)s.vol; a.mu = (const T*)s.mu; a.lam = (const T*)s.lam;
     a.pft = (T*)s.pft; a.valid = s.valid;
+    a.oX = a.X; a.oV = a.V; a.oF = a.F; a.oB = a.B; a.ovalid = a.valid;
+    a.rm = a.rv = a.ru = nullptr;
+    if(s.record) {
+        const PlainRecord& r = *s.record;
+        a.X = (T*)r.in; a.V = a.X + 3 * s.n; a.F = a.X + 6 * s.n; a.B = a.X + 15 * s.n;
+        a.valid = r.valid;
+        a.pft = (T*)r.pft;
+        if(r.out) {
+            a.oX = (T*)r.out; a.oV = a.oX + 3 * s.n; a.oF = a.oX + 6 * s.n; a.oB = a.oX + 15 * s.n;
+            a.ovalid = r.out_valid;
+        }
+        a.rm = (T*)r.gm; a.rv = (T*)r.gv; a.ru = (T*)r.gu;
+    }
     a.gm = (T*)s.gm; a.gmv = (T*)s.gmv; a.gv0 = (T*)s.gv0; a.gf = (T*)s.gf; a.gv = (T*)s.gv; a.gvf = (T*)s.gvf;
     a.dt = (T)dt;
     a.flags = h->d_flags;
