@@ -348,6 +348,8 @@ int mpm_destroy(mpm_handle* h)
     cudaFree(h->motion_table_f);
     cudaFree(h->motion_slot);
     cudaFree(h->d_flags);
+    cudaFree(h->speed_state);
+    if(h->speed_host) cudaFreeHost(h->speed_host);
     if(h->own_stream) cudaStreamDestroy(h->stream);
     delete h;
     return MPM_OK;
@@ -917,15 +919,25 @@ int mpm_grid_totals(mpm_handle* h, mpm_totals* out)
 int mpm_compute_dt(mpm_handle* h, double cfl, double max_dt, double* dt)
 {
     if(!h || !dt || !(cfl > 0) || !(max_dt > 0)) return MPM_ERR_ARG;
-    mpm_totals t;
-    int rc = mpm_particle_totals(h, &t);
-    if(rc) return rc;
+    double v = 0;
+    if(h->have_particles) {
+        if(!h->speed_host) MPM_CUDA(h, cudaMallocHost(&h->speed_host, sizeof(double)));
+        if(!h->speed_state) {
+            MPM_CUDA(h, cudaMalloc(&h->speed_state, 2 * sizeof(unsigned long long)));
+            MPM_CUDA(h, cudaMemsetAsync(h->speed_state, 0, 2 * sizeof(unsigned long long), h->stream));
+        }
+        *h->speed_host = 0;
+        int rc = fast(h) ? fast_affine_speed(h) : plain_affine_speed(h);
+        if(rc) return rc;
+        MPM_CUDA(h, cudaStreamSynchronize(h->stream));
+        v = *h->speed_host;
+    }
     double dx_min = h->sp.dx[0];
     for(int k = 1; k < h->sp.dim; k++) dx_min = std::min(dx_min, h->sp.dx[k]);
     if(fast(h) && h->fast.batch)   // smallest cell of any scene
         for(const SceneDev& s: h->fast.scenes_h)
             for(int k = 0; k < 3; k++) dx_min = std::min(dx_min, (double)s.dx[k]);
-    double critical = cfl * dx_min / max_dt, v = t.max_affine_speed;
+    double critical = cfl * dx_min / max_dt;
     *dt = v > critical ? cfl * dx_min / v : max_dt;
     return MPM_OK;
 }

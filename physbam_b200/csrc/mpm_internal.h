@@ -180,6 +180,9 @@ struct mpm_handle {
     int64_t n = 0;
     bool have_particles = false;
     unsigned* d_flags = nullptr;
+    // Compute_Dt's speed bound: reduction state (2 words), and the result in pinned memory
+    unsigned long long* speed_state = nullptr;
+    double* speed_host = nullptr;
     PlainState plain;
     FastState fast;
     mpm_plasticity_desc plastic{};   // kind MPM_PLASTICITY_NONE: off
@@ -267,6 +270,8 @@ int sort_keys_device(mpm_handle* h, const uint32_t* keys, int64_t n, int bits, u
     uint32_t* alt_keys, uint32_t* alt_vals, uint32_t* scratch);
 int fast_prepare(mpm_handle* h);
 int fast_particle_totals(mpm_handle* h, mpm_totals* out);
+int fast_affine_speed(mpm_handle* h);
+int plain_affine_speed(mpm_handle* h);
 int fast_grid_totals(mpm_handle* h, mpm_totals* out);
 int plain_particle_totals(mpm_handle* h, mpm_totals* out);
 int plain_plastic_init(mpm_handle* h);

@@ -11,6 +11,7 @@
 #include <cstring>
 
 #include "mpm_internal.h"
+#include "mpm_launch.cuh"
 #include "mpm_plain.cuh"
 #include "mpm_scatter.cuh"
 
@@ -1314,6 +1315,22 @@ template<class T> __global__ void k_plain_particle_totals(PlainArgs<T> a, double
     pwarp_max(mx + 1, amax);
 }
 
+// Compute_Dt's bound alone (the totals' max_affine_speed).
+template<class T> __global__ void __launch_bounds__(256) k_affine_speed(PlainArgs<T> a, unsigned long long* state, double* host)
+{
+    const int d = a.sp.dim;
+    double amax = 0, inv_min = a.sp.inv_dx[0];
+    for(int k = 1; k < d; k++) inv_min = fmin(inv_min, a.sp.inv_dx[k]);
+    for(int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n; p += (int64_t)gridDim.x * blockDim.x) {
+        if(!a.valid[p]) continue;
+        double v2 = 0, bf = 0;
+        for(int k = 0; k < d; k++) { const double v = a.V[p * d + k]; v2 += v * v; }
+        for(int k = 0; k < d * d; k++) { const double b = a.B[p * d * d + k]; bf += b * b; }
+        amax = fmax(amax, sqrt(v2) + sqrt(bf) * 6.0 * sqrt((double)d) * inv_min);
+    }
+    grid_max(amax, state, host);
+}
+
 template<class T> __global__ void k_plain_grid_totals(PlainArgs<T> a, double* acc)
 {
     const int d = a.sp.dim;
@@ -1374,6 +1391,17 @@ static int plain_totals(mpm_handle* h, bool grid, mpm_totals* out)
     memcpy(&out->max_speed, &mx[0], 8);
     memcpy(&out->max_affine_speed, &mx[1], 8);
     if(grid) out->max_speed = out->max_affine_speed = 0;
+    return MPM_OK;
+}
+
+int plain_affine_speed(mpm_handle* h)
+{
+    const int64_t n = h->plain.n;
+    if(!n) return MPM_OK;
+    if(h->model.precision == MPM_FP64)
+        k_affine_speed<double><<<gblocks(h, n, 256), 256, 0, h->stream>>>(args<double>(h, 0.0), h->speed_state, h->speed_host);
+    else k_affine_speed<float><<<gblocks(h, n, 256), 256, 0, h->stream>>>(args<float>(h, 0.0), h->speed_state, h->speed_host);
+    MPM_LAUNCHED(h, "k_affine_speed");
     return MPM_OK;
 }
 
