@@ -432,6 +432,7 @@ constexpr int BIN_THREADS = 512, BIN_PER = 2, BIN_TILE = BIN_THREADS * BIN_PER;
 
 __global__ void __launch_bounds__(BIN_THREADS) k_bins(FastArgs a)
 {
+    chain_begin();
     constexpr int NW = BIN_THREADS / 32;
     __shared__ uint32_t s_warp[NW][4];
     __shared__ uint32_t s_pre[4];         // prefixes of the tile: count, invalid (look-back); parts, active (bases)
@@ -591,6 +592,7 @@ __device__ __forceinline__ void copy_slot(const FastArgs& a, uint32_t j, uint32_
 // group synchronises on its own named barrier, never the whole CTA.
 __global__ void __launch_bounds__(256) k_route(FastArgs a)
 {
+    chain_begin();
     constexpr int W = 8, RW = 4, CS = 33;       // warps per CTA, rounds per warp and batch, padded row
     __shared__ uint32_t s_cnt[W * RW][CS];      // per warp and round: count per direction, then rank
     __shared__ uint32_t s_tot[W][32];           // per warp: its batch's count per direction
@@ -913,6 +915,7 @@ struct P2GSmem {
 
 template<int T, int PER, int CTAS> __global__ void __launch_bounds__(T, CTAS) k_p2g(FastArgs a)
 {
+    chain_begin();
     constexpr int PART = T * PER, GROUPS = T / 32 * 3;
     __shared__ P2GSmem S;
     extern __shared__ __align__(16) float4 FS[];   // PART rows, in cell order
@@ -1040,6 +1043,7 @@ template<int T, int PER, int CTAS> __global__ void __launch_bounds__(T, CTAS) k_
 // (collide_node).
 __global__ void __launch_bounds__(256) k_grid(FastArgs a)
 {
+    chain_begin();
     constexpr int kGroups = 4;   // node blocks per CTA pass
     __shared__ SceneDev s_sc[kGroups];
     __shared__ DevObject s_obj[kGroups][MPM_MAX_OBJECTS];
@@ -1493,6 +1497,7 @@ __device__ __forceinline__ bool g2p_take(const FastArgs& a, uint32_t nwork, uint
 
 template<int THREADS, int PK> __global__ void __launch_bounds__(THREADS) k_g2p(FastArgs a)
 {
+    chain_begin();
     // the previous order's counters are read by nothing after the routing: they
     // become the next substep's, cleared here (no memset node between substeps)
     if(blockIdx.x == 0 && threadIdx.x < CNT_COUNT) a.nctr[threadIdx.x] = 0u;
@@ -2364,11 +2369,11 @@ static int fast_route(mpm_handle* h)
     int slot = timer_begin(h, "fast_bins");
     FastArgs a = make_args(h, 0.0);   // a.ctr: cleared by the last G2P or by fast_prepare
     const int64_t tiles = (f.total_blocks + BIN_TILE - 1) / BIN_TILE;
-    k_bins<<<(unsigned)tiles, BIN_THREADS, 0, h->stream>>>(a);
+    launch_chained(k_bins, (unsigned)tiles, BIN_THREADS, 0, h->stream, a);
     MPM_LAUNCHED(h, "k_bins");
     timer_end(h, slot);
     slot = timer_begin(h, "fast_route");
-    k_route<<<occupancy_ctas(h, (const void*)k_route, 256, 1), 256, 0, h->stream>>>(a);   // resident CTAs only
+    launch_chained(k_route, occupancy_ctas(h, (const void*)k_route, 256, 1), 256, 0, h->stream, a);   // resident CTAs only
     MPM_LAUNCHED(h, "k_route");
     timer_end(h, slot);
     f.sorted_now = true;
@@ -2381,7 +2386,7 @@ template<int T, int PER, int CTAS> static void launch_p2g(mpm_handle* h, const F
     static_assert(T * PER * FROW * sizeof(float4) + sizeof(P2GSmem) <= 48 * 1024, "opt-in shared memory");
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)k_p2g<T, PER, CTAS>, T, smem);
-    k_p2g<T, PER, CTAS><<<h->sm_count * (occ > 0 ? occ : 1) * h->fast.cta_mult, T, smem, h->stream>>>(a);
+    launch_chained(k_p2g<T, PER, CTAS>, h->sm_count * (occ > 0 ? occ : 1) * h->fast.cta_mult, T, smem, h->stream, a);
 }
 
 int fast_p2g(mpm_handle* h, double dt, double)
@@ -2428,7 +2433,7 @@ int fast_forces(mpm_handle* h, double dt, double)
     FastArgs a = make_args(h, dt);
     f.grid_set = f.cur;
     int slot = timer_begin(h, "fast_grid");
-    k_grid<<<h->sm_count * 8, 256, 0, h->stream>>>(a);
+    launch_chained(k_grid, h->sm_count * 8, 256, 0, h->stream, a);
     f.grid_dirty = false;
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_grid");
@@ -2439,9 +2444,9 @@ template<int PK> static void launch_g2p(mpm_handle* h, const FastArgs& a)
 {
     const FastState& f = h->fast;
     switch(f.g2p_threads) {
-        case 64: k_g2p<64, PK><<<occupancy_ctas(h, (const void*)k_g2p<64, PK>, 64, f.cta_mult), 64, 0, h->stream>>>(a); break;
-        case 256: k_g2p<256, PK><<<occupancy_ctas(h, (const void*)k_g2p<256, PK>, 256, f.cta_mult), 256, 0, h->stream>>>(a); break;
-        default: k_g2p<128, PK><<<occupancy_ctas(h, (const void*)k_g2p<128, PK>, 128, f.cta_mult), 128, 0, h->stream>>>(a); break;
+        case 64: launch_chained(k_g2p<64, PK>, occupancy_ctas(h, (const void*)k_g2p<64, PK>, 64, f.cta_mult), 64, 0, h->stream, a); break;
+        case 256: launch_chained(k_g2p<256, PK>, occupancy_ctas(h, (const void*)k_g2p<256, PK>, 256, f.cta_mult), 256, 0, h->stream, a); break;
+        default: launch_chained(k_g2p<128, PK>, occupancy_ctas(h, (const void*)k_g2p<128, PK>, 128, f.cta_mult), 128, 0, h->stream, a); break;
     }
 }
 

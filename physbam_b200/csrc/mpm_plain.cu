@@ -36,6 +36,7 @@ template<class T> __device__ __forceinline__ void clear_node(const PlainArgs<T>&
 // The grid arrays (and tile flags) of the last P2G's nodes back to zero.
 template<class T> __global__ void k_clear(PlainArgs<T> a)
 {
+    chain_begin();
     for_nodes(a, [&](int64_t i) {
         clear_node(a, i);
         if(a.tile_flag && i % kTileNodes == 0) a.tile_flag[i / kTileNodes] = 0;
@@ -49,6 +50,7 @@ constexpr int kTileSpan = 1024, kTileThreads = 256;
 __global__ void __launch_bounds__(kTileThreads) k_tile_list(const uint8_t* flag, int64_t ntiles, uint32_t* tiles, uint32_t* count,
     uint32_t* rec_tiles, uint32_t* rec_count)   // and the same into a rollout's record, or null
 {
+    chain_begin();
     __shared__ uint32_t s_warp[kTileThreads / 32], s_before[kTileThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t first = (int64_t)blockIdx.x * kTileSpan;
@@ -113,6 +115,7 @@ template<class T, int d> __device__ __forceinline__ void force_row(const PlainAr
 // then reads the particles and forms their weights once).
 template<class T, int d, bool FORCES> __global__ void __launch_bounds__(kScatterThreads) k_p2g(PlainArgs<T> a)
 {
+    chain_begin();
     __shared__ ScatterWarp<T, d> W[kScatterThreads / 32];
     ScatterWarp<T, d>& S = W[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -157,6 +160,7 @@ template<class T, int d, bool FORCES> __global__ void __launch_bounds__(kScatter
 // v = mv / m on nodes with mass (MPM_DRIVER.cpp:282-305).
 template<class T> __global__ void k_normalize(PlainArgs<T> a)
 {
+    chain_begin();
     const int d = a.sp.dim;
     for_nodes(a, [&](int64_t i) {
         const T m = a.gm[i];
@@ -167,6 +171,7 @@ template<class T> __global__ void k_normalize(PlainArgs<T> a)
 // MPM_FINITE_ELEMENTS::Precompute (MPM_FINITE_ELEMENTS.cpp:47-67).
 template<class T, int d> __global__ void k_stress(PlainArgs<T> a)
 {
+    chain_begin();
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if(p >= a.n || !a.valid[p]) return;
     T F[9], PFT[9];
@@ -180,6 +185,7 @@ template<class T, int d> __global__ void k_stress(PlainArgs<T> a)
 // The force scatter by itself, for a P2G that did not take it along.
 template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_forces(PlainArgs<T> a)
 {
+    chain_begin();
     __shared__ ScatterWarp<T, d> W[kScatterThreads / 32];
     ScatterWarp<T, d>& S = W[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -203,6 +209,7 @@ template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_fo
 // mv / m first, where no k_normalize ran.
 template<class T, int d, bool NORMALIZE> __global__ void k_grid_update(PlainArgs<T> a)
 {
+    chain_begin();
     for_nodes(a, [&](int64_t i) {
         T m = a.gm[i];
         if(a.rm) {
@@ -246,6 +253,7 @@ template<class T, int d> __device__ __forceinline__ void keep_particle(const Pla
 // Reflect_Or_Invalidate_Particle (l.1219-1239, all sides free).
 template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
 {
+    chain_begin();
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if(p >= a.n) return;
     const T* X = a.X + p * d;
@@ -537,8 +545,8 @@ template<class T> int reflect_pass(mpm_handle* h, const PlainArgs<T>& a, Reflect
 template<class T> int stress_t(mpm_handle* h, const PlainArgs<T>& a)
 {
     const int t = 128, slot = timer_begin(h, "plain_stress");
-    if(h->sp.dim == 3) k_stress<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
-    else k_stress<T, 2><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
+    if(h->sp.dim == 3) launch_chained(k_stress<T, 3>, pblocks(a.n, t), t, 0, h->stream, a);
+    else launch_chained(k_stress<T, 2>, pblocks(a.n, t), t, 0, h->stream, a);
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_stress");
     return MPM_OK;
@@ -553,7 +561,7 @@ template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
     PlainArgs<T> a = args<T>(h, dt);
     const int t = kScatterThreads;
     int slot = timer_begin(h, "plain_clear");
-    k_clear<T><<<gblocks(h, a.gn, t), t, 0, h->stream>>>(a);
+    launch_chained(k_clear<T>, gblocks(h, a.gn, t), t, 0, h->stream, a);
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_clear");
     if(a.n) {
@@ -561,11 +569,11 @@ template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
         slot = timer_begin(h, "plain_p2g");
         const int b = pblocks(a.n, t);
         if(h->sp.dim == 3) {
-            if(with_forces) k_p2g<T, 3, true><<<b, t, 0, h->stream>>>(a);
-            else k_p2g<T, 3, false><<<b, t, 0, h->stream>>>(a);
+            if(with_forces) launch_chained(k_p2g<T, 3, true>, b, t, 0, h->stream, a);
+            else launch_chained(k_p2g<T, 3, false>, b, t, 0, h->stream, a);
         } else {
-            if(with_forces) k_p2g<T, 2, true><<<b, t, 0, h->stream>>>(a);
-            else k_p2g<T, 2, false><<<b, t, 0, h->stream>>>(a);
+            if(with_forces) launch_chained(k_p2g<T, 2, true>, b, t, 0, h->stream, a);
+            else launch_chained(k_p2g<T, 2, false>, b, t, 0, h->stream, a);
         }
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_p2g");
@@ -574,7 +582,7 @@ template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
         const int64_t nt = (a.gn + kTileNodes - 1) / kTileNodes;
         slot = timer_begin(h, "plain_tiles");
         const PlainRecord* r = h->plain.record;
-        k_tile_list<<<(unsigned)((nt + kTileSpan - 1) / kTileSpan), kTileThreads, 0, h->stream>>>(
+        launch_chained(k_tile_list, (unsigned)((nt + kTileSpan - 1) / kTileSpan), kTileThreads, 0, h->stream,
             a.tile_flag, nt, h->plain.tiles, h->plain.tile_count, r ? r->tiles : nullptr, r ? r->tile_count : nullptr);
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_tile_list");
@@ -582,7 +590,7 @@ template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
     if(a.reflect && !h->reflect.full_reflection && (rc = reflect_pass<T>(h, a, REFLECT_MM))) return rc;
     if(with_forces) return MPM_OK;
     slot = timer_begin(h, "plain_normalize");
-    k_normalize<T><<<gblocks(h, a.gn, t), t, 0, h->stream>>>(a);
+    launch_chained(k_normalize<T>, gblocks(h, a.gn, t), t, 0, h->stream, a);
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_normalize");
     return MPM_OK;
@@ -597,19 +605,19 @@ template<class T> int forces_t(mpm_handle* h, double dt, bool with_forces)
     if(a.n && !with_forces) {
         if((rc = stress_t<T>(h, a))) return rc;
         const int slot = timer_begin(h, "plain_forces");
-        if(h->sp.dim == 3) k_forces<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
-        else k_forces<T, 2><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
+        if(h->sp.dim == 3) launch_chained(k_forces<T, 3>, pblocks(a.n, t), t, 0, h->stream, a);
+        else launch_chained(k_forces<T, 2>, pblocks(a.n, t), t, 0, h->stream, a);
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_forces");
     }
     if(a.reflect && !h->reflect.full_reflection && (rc = reflect_pass<T>(h, a, REFLECT_FORCE))) return rc;
     const int slot = timer_begin(h, "plain_grid_update"), b = gblocks(h, a.gn, t);
     if(h->sp.dim == 3) {
-        if(with_forces) k_grid_update<T, 3, true><<<b, t, 0, h->stream>>>(a);
-        else k_grid_update<T, 3, false><<<b, t, 0, h->stream>>>(a);
+        if(with_forces) launch_chained(k_grid_update<T, 3, true>, b, t, 0, h->stream, a);
+        else launch_chained(k_grid_update<T, 3, false>, b, t, 0, h->stream, a);
     } else {
-        if(with_forces) k_grid_update<T, 2, true><<<b, t, 0, h->stream>>>(a);
-        else k_grid_update<T, 2, false><<<b, t, 0, h->stream>>>(a);
+        if(with_forces) launch_chained(k_grid_update<T, 2, true>, b, t, 0, h->stream, a);
+        else launch_chained(k_grid_update<T, 2, false>, b, t, 0, h->stream, a);
     }
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_grid_update");
@@ -861,8 +869,8 @@ template<class T> int g2p_t(mpm_handle* h, double dt)
     if(!a.n) return MPM_OK;
     const int t = 128;
     int slot = timer_begin(h, "plain_g2p");
-    if(h->sp.dim == 3) k_g2p<T, 3><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
-    else k_g2p<T, 2><<<pblocks(a.n, t), t, 0, h->stream>>>(a);
+    if(h->sp.dim == 3) launch_chained(k_g2p<T, 3>, pblocks(a.n, t), t, 0, h->stream, a);
+    else launch_chained(k_g2p<T, 2>, pblocks(a.n, t), t, 0, h->stream, a);
     timer_end(h, slot);
     MPM_LAUNCHED(h, "k_g2p");
     if(h->plastic.kind == MPM_PLASTICITY_CLAMP) {
