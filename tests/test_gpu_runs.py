@@ -1,0 +1,166 @@
+"""GPU tests of the kernels that sum runs of particles and visit lists of grid tiles, at the
+sizes where they can go wrong, against the C oracle.
+
+* Particle counts around a warp (plain, adjoint and implicit scatters), a work item and a
+  block (fast P2G and G2P, every launch shape), in shuffled order, some invalid, one without
+  mass.
+* Grids past the size from which the plain path lists the tiles that P2G touched: explicit and
+  implicit substeps, a rollout recorded in place.
+* The hand-over and read-back of particles, and Compute_Dt's speed bound, around a warp.
+
+Tolerances: FP64 sums of at most 27 x 60 terms in another order, some 1e-13 of the largest
+value, over ten substeps; FP32 as in test_gpu_parity.py.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from physbam_b200 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [1, 2, 31, 33, 97, 257]
+
+
+def D():
+    from physbam_b200 import driver
+    return driver
+
+
+def pick(scene, n, seed=3):
+    """n particles of the scene in no order at all."""
+    return scene.subset(np.random.default_rng(seed).permutation(scene.n)[:n])
+
+
+def run_oracle(scene, steps, valid=None):
+    st = oracle.State(scene)
+    if valid is not None:
+        st.valid[:] = valid
+    oracle.run(st, steps)
+    return st
+
+
+def run_gpu(scene, steps, precision, path, valid=None, shape=None):
+    drv = D().MPM_DRIVER(scene, precision=precision, path=path)
+    if shape is not None:
+        drv.set_launch_shape(*shape)
+    drv.set_particles(scene.X, scene.V, scene.F, scene.B, scene.mass, scene.volume, scene.mu, scene.lam, valid=valid)
+    drv.advance(steps)
+    drv.synchronize()
+    got = drv.get_particles()
+    drv.close()
+    return got
+
+
+def check(got, st, tol):
+    keep = st.valid.astype(bool)
+    np.testing.assert_array_equal(got["valid"], keep)
+    vmax = max(np.abs(st.V).max(), 1e-12)
+    for k, ref, scale in (("X", st.X, 1.0), ("V", st.V, vmax), ("F", st.F_rowmajor(), 1.0),
+                          ("B", st.B_rowmajor(), vmax / st.scene.dx)):
+        assert np.abs(got[k] - ref)[keep].max() <= tol[k] * scale, k
+
+
+TOL64 = {"X": 1e-12, "V": 1e-9, "F": 1e-10, "B": 1e-8}
+TOL32 = {"X": 2e-6, "V": 2e-3, "F": 1e-4, "B": 2e-3}
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", COUNTS)
+def test_plain_scatter_counts(cuda_device, dim, n):
+    scene = pick(S.small_2d() if dim == 2 else S.small_3d(), n)
+    valid = np.ones(scene.n, np.uint8)
+    valid[::5] = 0
+    if n < 3:
+        valid[:] = 1
+    check(run_gpu(scene, 10, D().FP64, D().PATH_PLAIN, valid), run_oracle(scene, 10, valid), TOL64)
+
+
+@pytest.mark.parametrize("variant,threads", [(0, 64), (1, 256), (2, 64), (3, 128), (0, 256), (3, 64)])
+@pytest.mark.parametrize("n", [1, 63, 65, 127, 129, 257, 600])
+def test_fast_item_counts(cuda_device, variant, threads, n):
+    """All particles in one block and its neighbours: items of every size up to the largest."""
+    base = S.small_3d()
+    scene = pick(base, n)
+    h = 1.0 / 16
+    rng = np.random.default_rng(n)
+    scene.X[:] = 0.25 + 0.05 * h + rng.random((scene.n, 3)) * np.array([0.9, 0.9, 3.9]) * h
+    scene.mass[-1] *= 1e-3
+    check(run_gpu(scene, 10, D().FP32, D().PATH_FAST, shape=(variant, threads, 1)), run_oracle(scene, 10), TOL32)
+
+
+def test_fast_particle_without_mass(cuda_device):
+    """A particle of zero mass takes part with its force alone, as on the plain path."""
+    scene = pick(S.small_3d(), 700)
+    scene.mass[::50] = 0.0
+    check(run_gpu(scene, 5, D().FP32, D().PATH_FAST), run_oracle(scene, 5), TOL32)
+
+
+def big(scene_fn, **kw):
+    """A small body on a 40^3 grid: 46^3 nodes, past the size from which tiles are listed."""
+    return scene_fn(G=40, **kw)
+
+
+@pytest.mark.parametrize("n", [1, 97, 3000])
+def test_plain_listed_tiles(cuda_device, n):
+    scene = pick(big(S.small_3d, ppc=4), n)
+    check(run_gpu(scene, 10, D().FP64, D().PATH_PLAIN), run_oracle(scene, 10), TOL64)
+
+
+def test_implicit_listed_tiles(cuda_device):
+    """On a grid with listed tiles, over a sticking floor: the solve agrees with itself to the
+    Newton tolerance and, at a small step, with the explicit substep.  Backward and symplectic
+    Euler differ by (dt omega)^2 of the velocity per step, omega^2 = 12 (c / h)^2 the grid's
+    highest."""
+    dt = 2e-5
+    scene = S.small_3d(G=40, with_walls=False, dt=dt)
+    scene.objects = S.walls(3, scene.counts, scene.domain_min, scene.domain_max, 1 << 3, S.STICK, 0.0, 0.15)
+    st = run_oracle(scene, 2)
+    scene.implicit = S.Implicit()
+    got = run_gpu(scene, 2, D().FP64, D().PATH_PLAIN)
+    again = run_gpu(scene, 2, D().FP64, D().PATH_PLAIN)
+    vmax = np.abs(st.V).max()
+    assert np.abs(got["X"] - again["X"]).max() < 2e-9 and np.abs(got["V"] - again["V"]).max() < 1e-6 * vmax
+    c = np.sqrt((scene.lam + 2 * scene.mu).max() * scene.volume[0] / scene.mass[0])
+    assert np.abs(got["V"] - st.V).max() < 2 * 12 * (dt * c / scene.dx) ** 2 * vmax
+
+
+@pytest.mark.parametrize("G,budget", [(16, -1), (16, 0), (40, -1), (40, 0)])
+def test_recorded_rollout_state(cuda_device, G, budget):
+    """The rollout's G2P writes from one tape slot to the next; the particles it ends with are
+    those of the plain substeps, frozen and leaving ones among them, with the tape whole or in
+    segments, and a backward pass leaves them there."""
+    import torch
+    scene = S.small_3d(G=G, ppc=2, with_walls=False)
+    scene.X[:7] = 1.0 - 1e-5                       # leave in the first substeps
+    scene.V[:7] = 5.0
+    st = run_oracle(scene, 11)
+    drv = D().MPM_DRIVER(scene, precision=D().FP64, path=D().PATH_PLAIN)
+    drv.set_diff_tape_budget(budget)
+    drv.set_scene_particles(scene)
+    drv.diff_forward(11, 4)
+    check(drv.get_particles(), st, TOL64)
+    one = [torch.ones((scene.n, k), dtype=torch.float64, device="cuda") for k in (3, 3, 9, 9)]
+    g = drv.diff_backward(*one)
+    check(drv.get_particles(), st, TOL64)
+    assert all(bool(torch.isfinite(x).all()) for x in g)
+    drv.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", COUNTS)
+def test_hand_over_and_back(cuda_device, n, dtype):
+    """Particles come back as they went in (rounded to float), in the caller's order, after a
+    substep of no length to speak of has sorted them; the speed bound equals the totals'."""
+    scene = pick(S.small_3d(), n)
+    drv = D().MPM_DRIVER(scene)
+    drv.set_scene_particles(scene, dtype=dtype)
+    got = drv.get_particles(dtype=dtype)
+    for k in ("X", "V", "F", "B"):
+        np.testing.assert_array_equal(got[k], getattr(scene, k).astype(np.float32).astype(dtype))
+    drv.advance(1, 1e-12)
+    got = drv.get_particles(dtype=dtype)
+    np.testing.assert_allclose(got["X"], scene.X, atol=1e-6)
+    v = drv.particle_totals()["max_affine_speed"]
+    assert drv.compute_dt(cfl=1e-3, max_dt=1e3) == pytest.approx(1e-3 * scene.dx / v, rel=1e-15)
+    drv.close()
