@@ -2922,7 +2922,7 @@ __global__ void k_particle_totals(FastArgs a, double* acc, unsigned long long* m
 
 // Compute_Dt's bound alone: max |V| + |B| 6 sqrt(d) / dx, the max_affine_speed of
 // the totals.  Those sum eleven more values with an atomic per warp each: 165 us of a
-// 290 us adaptive substep at 301,840 particles; a maximum per CTA instead, this pass
+// 290 us adaptive substep at 444,528 particles; a maximum per CTA instead, this pass
 // reads 13 floats per particle, and the frame of 25 such substeps takes 3.1 ms, not 6.9.
 __global__ void __launch_bounds__(256) k_affine_speed(FastArgs a, unsigned long long* state, double* host)
 {

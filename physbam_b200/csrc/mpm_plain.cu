@@ -251,6 +251,12 @@ template<class T, int d> __device__ __forceinline__ void keep_particle(const Pla
 
 // MPM_DRIVER::Grid_To_Particle (MPM_DRIVER.cpp:450-515) and
 // Reflect_Or_Invalidate_Particle (l.1219-1239, all sides free).
+// The sums over the nodes are taken axis by axis, the last first, so a node costs
+// its loads and 4 d products; B of l.482-485 and l.503-508 in the form
+//   sum w v_fric (Z - X)^T + dt/2 [sum w (v_fric v^T - v v_fric^T) - (V_fric V^T - V V_fric^T)],
+// equal to it and without the cancellation of terms in Z against terms in X.
+// FP64, 242,752 particles (8 substeps): 2.38 -> 2.21 ms per call; errors against 64
+// bits 100 times smaller in FP64 (1.8e-14), 28 times in an FP32 gradient.
 template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
 {
     chain_begin();
@@ -262,33 +268,60 @@ template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
         keep_particle<T, d>(a, p);
         return;
     }
-    T Vpic[3] = {0, 0, 0}, Vpf[3] = {0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, Bh[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const int nq = d == 3 ? 27 : 9;
-    for(int q = 0; q < nq; q++) {
-        int64_t i;
-        T w, g[3], Z[3];
-        node<T, d>(a, s, q, i, w, g, Z);
-        T vn[3], vf[3], Zp[3], Zm[3];
+    T Vpic[3] = {0, 0, 0}, Vpf[3] = {0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, Bv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    T K01 = 0, K02 = 0, K12 = 0, off[3][3];
 #pragma unroll
-        for(int k = 0; k < d; k++) {
-            vn[k] = a.gv[i * d + k];
-            vf[k] = a.gvf[i * d + k];
-            Vpic[k] += w * vn[k];
-            Vpf[k] += w * vf[k];
-            T xi = Z[k] + a.dt * vn[k];
-            Zp[k] = Z[k] + xi;
-            Zm[k] = Z[k] - xi;
+    for(int k = 0; k < d; k++)
+#pragma unroll
+        for(int o = 0; o < 3; o++)
+            off[k][o] = (T)a.sp.dmin[k] + ((T)(s.base[k] + o) + (T).5) * (T)a.sp.dx[k] - X[k];
+    const int64_t first = first_node<T, d>(a, s), s0 = node_stride(a, d, 0), s1 = node_stride(a, d, 1);
+    constexpr int L = d - 1;       // the last axis
+#pragma unroll
+    for(int ii = 0; ii < 3; ii++)
+#pragma unroll
+        for(int jj = 0; jj < (d == 3 ? 3 : 1); jj++) {
+            T Sw[3] = {0, 0, 0}, Sd[3] = {0, 0, 0}, Tw[3] = {0, 0, 0}, Td[3] = {0, 0, 0};
+            T k01 = 0, k02 = 0, k12 = 0;
+            const int64_t row = (first + ii * s0 + (d == 3 ? jj * s1 : 0)) * d;
+#pragma unroll
+            for(int kk = 0; kk < 3; kk++) {
+                const T w = s.ax[L].w[kk], dw = s.ax[L].dw[kk], wo = w * off[L][kk];
+                T vn[3] = {0, 0, 0}, vf[3] = {0, 0, 0};
+#pragma unroll
+                for(int r = 0; r < d; r++) {
+                    vn[r] = a.gv[row + kk * d + r];
+                    vf[r] = a.gvf[row + kk * d + r];
+                    Sw[r] += vn[r] * w;
+                    Sd[r] += vn[r] * dw;
+                    Tw[r] += vf[r] * w;
+                    Td[r] += vf[r] * wo;
+                }
+                k01 += w * (vf[0] * vn[1] - vf[1] * vn[0]);
+                if(d == 3) {
+                    k02 += w * (vf[0] * vn[2] - vf[2] * vn[0]);
+                    k12 += w * (vf[1] * vn[2] - vf[2] * vn[1]);
+                }
+            }
+            const T wy = d == 3 ? s.ax[1].w[jj] : (T)1, wxy = s.ax[0].w[ii] * wy;
+            const T gx = s.ax[0].dw[ii] * wy, gy = s.ax[0].w[ii] * s.ax[1].dw[jj];
+            K01 += wxy * k01;
+            K02 += wxy * k02;
+            K12 += wxy * k12;
+#pragma unroll
+            for(int r = 0; r < d; r++) {
+                Vpic[r] += wxy * Sw[r];
+                Vpf[r] += wxy * Tw[r];
+                G[r] += gx * Sw[r];
+                Bv[r] += wxy * off[0][ii] * Tw[r];
+                if(d == 3) {
+                    G[r + d] += gy * Sw[r];
+                    Bv[r + d] += wxy * off[1][jj] * Tw[r];
+                }
+                G[r + d * L] += wxy * Sd[r];
+                Bv[r + d * L] += wxy * Td[r];
+            }
         }
-#pragma unroll
-        for(int c = 0; c < d; c++)
-#pragma unroll
-            for(int r = 0; r < d; r++) G[r + d * c] += vn[r] * g[c];
-        T hw = w / 2;
-#pragma unroll
-        for(int c = 0; c < d; c++)
-#pragma unroll
-            for(int r = 0; r < d; r++) Bh[r + d * c] += hw * (vf[r] * Zp[c] + Zm[r] * vf[c]);
-    }
     const T* Fp = a.F + p * d * d;
     T A[9], Fn[9];
 #pragma unroll
@@ -309,11 +342,19 @@ template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
 #pragma unroll
     for(int k = 0; k < d; k++) xn[k] = X[k] + a.dt * Vpic[k];
     T* Bp = a.oB + p * d * d;
+    const T h = (T).5 * a.dt;
+    const T A01 = h * (K01 - (Vpf[0] * Vpic[1] - Vpic[0] * Vpf[1]));
+    Bv[d] += A01;
+    Bv[1] -= A01;
+    if(d == 3) {
+        const T A02 = h * (K02 - (Vpf[0] * Vpic[2] - Vpic[0] * Vpf[2])), A12 = h * (K12 - (Vpf[1] * Vpic[2] - Vpic[1] * Vpf[2]));
+        Bv[6] += A02;
+        Bv[2] -= A02;
+        Bv[7] += A12;
+        Bv[5] -= A12;
+    }
 #pragma unroll
-    for(int c = 0; c < d; c++)
-#pragma unroll
-        for(int r = 0; r < d; r++)
-            Bp[r + d * c] = Bh[r + d * c] - (T).5 * (Vpf[r] * (X[c] + xn[c]) + (X[r] - xn[r]) * Vpf[c]);
+    for(int e = 0; e < d * d; e++) Bp[e] = Bv[e];
 #pragma unroll
     for(int e = 0; e < d * d; e++) { a.oF[p * d * d + e] = Fn[e]; finite = finite && isfinite(Fn[e]); }
     // Reflect_Or_Invalidate_Particle (l.1219-1239): mirrored back across a
