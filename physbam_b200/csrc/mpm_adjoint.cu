@@ -489,6 +489,11 @@ struct DiffTape {
     void* final_state = nullptr;
     uint8_t* final_valid = nullptr;
     void *adj[2] = {nullptr, nullptr};   // X V F B adjoints, double-buffered
+    // a whole tape's forward and backward passes, captured when the same rollout runs
+    // again on the same buffers; graph_dt: of the captured ones
+    cudaGraphExec_t graphs[2] = {nullptr, nullptr};
+    bool replay = false;
+    double graph_dt = 0;
     void *amu = nullptr, *alam = nullptr, *ga[2] = {nullptr, nullptr}, *gma = nullptr;
 };
 
@@ -502,10 +507,43 @@ void diff_invalidate(mpm_handle* h)
     if(t) t->recorded = false;
 }
 
+// The captured passes hold buffer addresses, objects and the step.
+void diff_release_graphs(mpm_handle* h)
+{
+    DiffTape* t = tape(h);
+    if(!t) return;
+    for(cudaGraphExec_t& g: t->graphs) {
+        if(g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
+// Run `enqueue` from its captured graph, captured here on first use.  64 substeps
+// are 576 launches of 4 to 30 us kernels, each carrying up to 4 KB of arguments: on
+// their own the host enqueues them slower than the GPU runs them.
+template<class FN> static int replay(mpm_handle* h, cudaGraphExec_t& ge, FN&& enqueue)
+{
+    if(h->timing || !h->own_stream) return enqueue();
+    if(!ge) {
+        cudaGraph_t g;
+        MPM_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+        const int rc = enqueue();
+        cudaError_t e = cudaStreamEndCapture(h->stream, &g);
+        if(rc) { if(e == cudaSuccess) cudaGraphDestroy(g); return rc; }
+        if(e != cudaSuccess) return check_cuda(h, e, "cudaStreamEndCapture");
+        e = cudaGraphInstantiate(&ge, g, 0);
+        cudaGraphDestroy(g);
+        if(e != cudaSuccess) { ge = nullptr; return check_cuda(h, e, "cudaGraphInstantiate"); }
+    }
+    MPM_CUDA(h, cudaGraphLaunch(ge, h->stream));
+    return MPM_OK;
+}
+
 void diff_free(mpm_handle* h)
 {
     DiffTape* t = tape(h);
     if(!t) return;
+    diff_release_graphs(h);
     void* ps[] = {t->ckpt, t->ckpt_valid, t->seg, t->seg_valid, t->seg_gm, t->seg_gv, t->seg_gu, t->seg_pft, t->final_state,
                   t->final_valid, t->adj[0], t->adj[1], t->amu, t->alam, t->ga[0], t->ga[1], t->gma, t->seg_tiles,
                   t->seg_count};
@@ -632,23 +670,30 @@ int diff_forward(mpm_handle* h, double dt, int nsteps, int every)
         MPM_CUDA(h, cudaMalloc(&t->final_state, st + 1));
         MPM_CUDA(h, cudaMalloc(&t->final_valid, s.n + 1));
     }
-    int rc;
-    for(int k = 0; k < nsteps; k++) {
-        if(t->full) {
-            if(k == 0 && (rc = state_copy(h, t->seg, t->seg_valid, true))) return rc;
-            rc = esz == 8 ? record_substep<double>(h, t, k, true, k + 1 == nsteps)
-                          : record_substep<float>(h, t, k, true, k + 1 == nsteps);
-            if(rc) return rc;
-            continue;
+    t->replay = reuse && t->full;
+    if(t->graph_dt != dt) diff_release_graphs(h);
+    t->graph_dt = dt;
+    int rc = plain_prepare(h);
+    if(rc) return rc;
+    auto steps = [&]() -> int {
+        for(int k = 0; k < nsteps; k++) {
+            if(t->full) {
+                if(k == 0 && (rc = state_copy(h, t->seg, t->seg_valid, true))) return rc;
+                rc = esz == 8 ? record_substep<double>(h, t, k, true, k + 1 == nsteps)
+                              : record_substep<float>(h, t, k, true, k + 1 == nsteps);
+                if(rc) return rc;
+                continue;
+            }
+            if(k % every == 0) {
+                int c = k / every;
+                if((rc = state_copy(h, (char*)t->ckpt + c * st, t->ckpt_valid + c * s.n, true))) return rc;
+            }
+            if((rc = plain_p2g_forces(h, dt))) return rc;
+            if((rc = plain_g2p(h, dt, 0))) return rc;
         }
-        if(k % every == 0) {
-            int c = k / every;
-            if((rc = state_copy(h, (char*)t->ckpt + c * st, t->ckpt_valid + c * s.n, true))) return rc;
-        }
-        if((rc = plain_p2g_forces(h, dt))) return rc;
-        if((rc = plain_g2p(h, dt, 0))) return rc;
-    }
-    if((rc = state_copy(h, t->final_state, t->final_valid, true))) return rc;
+        return state_copy(h, t->final_state, t->final_valid, true);
+    };
+    if((rc = t->replay ? replay(h, t->graphs[0], steps) : steps())) return rc;
     t->recorded = true;
     return MPM_OK;
 }
@@ -680,77 +725,82 @@ template<class T> static int backward_t(mpm_handle* h, const void* gX, const voi
     MPM_CUDA(h, cudaMemcpyAsync(a1 + 3 * n, gV, 3 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(a1 + 6 * n, gF, 9 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(a1 + 15 * n, gB, 9 * n * e, cudaMemcpyDeviceToDevice, h->stream));
-    MPM_CUDA(h, cudaMemsetAsync(t->amu, 0, n * e, h->stream));
-    MPM_CUDA(h, cudaMemsetAsync(t->alam, 0, n * e, h->stream));
-    const int tb = plain::kScatterThreads;
-    // a full tape is one segment, recorded by the forward; otherwise each
-    // checkpoint's segment is recomputed from it, keeping what the adjoint needs
-    const int nck = t->full ? 1 : (t->nsteps + every - 1) / every;
-    const int span = t->full ? t->nsteps : every;
-    int rc;
-    for(int c = nck - 1; c >= 0; c--) {
-        int k0 = c * span, k1 = k0 + span < t->nsteps ? k0 + span : t->nsteps;
-        if(!t->full) {
-            MPM_CUDA(h, cudaMemcpyAsync(t->seg, (char*)t->ckpt + c * st, st, cudaMemcpyDeviceToDevice, h->stream));
-            MPM_CUDA(h, cudaMemcpyAsync(t->seg_valid, t->ckpt_valid + c * n, n, cudaMemcpyDeviceToDevice, h->stream));
-            for(int k = k0; k < k1; k++)
-                if((rc = record_substep<T>(h, t, k - k0, k + 1 < k1, false))) return rc;
+    auto passes = [&]() -> int {
+        MPM_CUDA(h, cudaMemsetAsync(t->amu, 0, n * e, h->stream));
+        MPM_CUDA(h, cudaMemsetAsync(t->alam, 0, n * e, h->stream));
+        const int tb = plain::kScatterThreads;
+        // a full tape is one segment, recorded by the forward; otherwise each
+        // checkpoint's segment is recomputed from it, keeping what the adjoint needs
+        const int nck = t->full ? 1 : (t->nsteps + every - 1) / every;
+        const int span = t->full ? t->nsteps : every;
+        int rc;
+        for(int c = nck - 1; c >= 0; c--) {
+            int k0 = c * span, k1 = k0 + span < t->nsteps ? k0 + span : t->nsteps;
+            if(!t->full) {
+                MPM_CUDA(h, cudaMemcpyAsync(t->seg, (char*)t->ckpt + c * st, st, cudaMemcpyDeviceToDevice, h->stream));
+                MPM_CUDA(h, cudaMemcpyAsync(t->seg_valid, t->ckpt_valid + c * n, n, cudaMemcpyDeviceToDevice, h->stream));
+                for(int k = k0; k < k1; k++)
+                    if((rc = record_substep<T>(h, t, k - k0, k + 1 < k1, false))) return rc;
+            }
+            auto list = [&](int j) { return t->ntiles ? t->seg_tiles + j * t->ntiles : nullptr; };
+            auto count = [&](int j) { return t->ntiles ? t->seg_count + j : nullptr; };
+            int cur = 0;
+            const int slot = timer_begin(h, "adj_clear");
+            k_adj_clear<T><<<blocks_for(h, gn, 256, true), 256, 0, h->stream>>>((T*)t->ga[0], gn, list(k1 - 1 - k0), count(k1 - 1 - k0));
+            timer_end(h, slot);
+            MPM_LAUNCHED(h, "k_adj_clear");
+            for(int k = k1 - 1; k >= k0; k--) {
+                int j = k - k0;
+                const T* base = (const T*)((char*)t->seg + j * st);
+                AdjArgs<T> a;
+                a.sp = h->sp;
+                a.n = n; a.gn = gn;
+                for(int q = 0; q < 3; q++) a.gs[q] = h->sp.counts[q] + 2 * MPM_GHOST;
+                a.X = base; a.V = base + 3 * n; a.F = base + 6 * n; a.B = base + 15 * n;
+                a.valid = t->seg_valid + j * n;
+                a.mass = (const T*)s.mass; a.vol = (const T*)s.vol; a.mu = (const T*)s.mu; a.lam = (const T*)s.lam;
+                a.pft = (const T*)t->seg_pft + j * 9 * n;
+                a.gm = (const T*)t->seg_gm + j * gn;
+                a.gv = (const T*)t->seg_gv + j * gn * 3;
+                a.gu = (const T*)t->seg_gu + j * gn * 3;
+                a.aX1 = a1; a.aV1 = a1 + 3 * n; a.aF1 = a1 + 6 * n; a.aB1 = a1 + 15 * n;
+                a.aX0 = a0; a.aV0 = a0 + 3 * n; a.aF0 = a0 + 6 * n; a.aB0 = a0 + 15 * n;
+                a.amu = (T*)t->amu; a.alam = (T*)t->alam;
+                a.ga = (T*)t->ga[cur]; a.gma = (T*)t->gma;
+                a.ga_next = j ? (T*)t->ga[cur ^ 1] : nullptr;
+                a.tiles = list(j); a.tile_count = count(j);
+                a.next_tiles = j ? list(j - 1) : nullptr; a.next_count = j ? count(j - 1) : nullptr;
+                cur ^= 1;
+                a.dt = (T)t->dt;
+                a.flags = h->d_flags;
+                int slot = timer_begin(h, "adj_g2p");
+                k_adj_g2p<T><<<blocks_for(h, n, tb, false), tb, 0, h->stream>>>(a);
+                timer_end(h, slot);
+                MPM_LAUNCHED(h, "k_adj_g2p");
+                slot = timer_begin(h, "adj_grid");
+                k_adj_grid<T><<<blocks_for(h, gn, 256, true), 256, 0, h->stream>>>(a);
+                timer_end(h, slot);
+                MPM_LAUNCHED(h, "k_adj_grid");
+                slot = timer_begin(h, "adj_p2g");
+                k_adj_p2g<T><<<blocks_for(h, n, tb, false), tb, 0, h->stream>>>(a);
+                timer_end(h, slot);
+                MPM_LAUNCHED(h, "k_adj_p2g");
+                T* tmp = a1; a1 = a0; a0 = tmp;
+            }
         }
-        auto list = [&](int j) { return t->ntiles ? t->seg_tiles + j * t->ntiles : nullptr; };
-        auto count = [&](int j) { return t->ntiles ? t->seg_count + j : nullptr; };
-        int cur = 0;
-        const int slot = timer_begin(h, "adj_clear");
-        k_adj_clear<T><<<blocks_for(h, gn, 256, true), 256, 0, h->stream>>>((T*)t->ga[0], gn, list(k1 - 1 - k0), count(k1 - 1 - k0));
-        timer_end(h, slot);
-        MPM_LAUNCHED(h, "k_adj_clear");
-        for(int k = k1 - 1; k >= k0; k--) {
-            int j = k - k0;
-            const T* base = (const T*)((char*)t->seg + j * st);
-            AdjArgs<T> a;
-            a.sp = h->sp;
-            a.n = n; a.gn = gn;
-            for(int q = 0; q < 3; q++) a.gs[q] = h->sp.counts[q] + 2 * MPM_GHOST;
-            a.X = base; a.V = base + 3 * n; a.F = base + 6 * n; a.B = base + 15 * n;
-            a.valid = t->seg_valid + j * n;
-            a.mass = (const T*)s.mass; a.vol = (const T*)s.vol; a.mu = (const T*)s.mu; a.lam = (const T*)s.lam;
-            a.pft = (const T*)t->seg_pft + j * 9 * n;
-            a.gm = (const T*)t->seg_gm + j * gn;
-            a.gv = (const T*)t->seg_gv + j * gn * 3;
-            a.gu = (const T*)t->seg_gu + j * gn * 3;
-            a.aX1 = a1; a.aV1 = a1 + 3 * n; a.aF1 = a1 + 6 * n; a.aB1 = a1 + 15 * n;
-            a.aX0 = a0; a.aV0 = a0 + 3 * n; a.aF0 = a0 + 6 * n; a.aB0 = a0 + 15 * n;
-            a.amu = (T*)t->amu; a.alam = (T*)t->alam;
-            a.ga = (T*)t->ga[cur]; a.gma = (T*)t->gma;
-            a.ga_next = j ? (T*)t->ga[cur ^ 1] : nullptr;
-            a.tiles = list(j); a.tile_count = count(j);
-            a.next_tiles = j ? list(j - 1) : nullptr; a.next_count = j ? count(j - 1) : nullptr;
-            cur ^= 1;
-            a.dt = (T)t->dt;
-            a.flags = h->d_flags;
-            int slot = timer_begin(h, "adj_g2p");
-            k_adj_g2p<T><<<blocks_for(h, n, tb, false), tb, 0, h->stream>>>(a);
-            timer_end(h, slot);
-            MPM_LAUNCHED(h, "k_adj_g2p");
-            slot = timer_begin(h, "adj_grid");
-            k_adj_grid<T><<<blocks_for(h, gn, 256, true), 256, 0, h->stream>>>(a);
-            timer_end(h, slot);
-            MPM_LAUNCHED(h, "k_adj_grid");
-            slot = timer_begin(h, "adj_p2g");
-            k_adj_p2g<T><<<blocks_for(h, n, tb, false), tb, 0, h->stream>>>(a);
-            timer_end(h, slot);
-            MPM_LAUNCHED(h, "k_adj_p2g");
-            T* tmp = a1; a1 = a0; a0 = tmp;
-        }
-    }
-    // a1 now holds the adjoint of the initial state
+        // leave the handle at the final state again
+        return state_copy(h, t->final_state, t->final_valid, false);
+    };
+    const int rc = t->replay ? replay(h, t->graphs[1], passes) : passes();
+    if(rc) return rc;
+    a1 = (T*)t->adj[t->nsteps & 1];   // the adjoint of the initial state
     MPM_CUDA(h, cudaMemcpyAsync(oX, a1, 3 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(oV, a1 + 3 * n, 3 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(oF, a1 + 6 * n, 9 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(oB, a1 + 15 * n, 9 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(omu, t->amu, n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(olam, t->alam, n * e, cudaMemcpyDeviceToDevice, h->stream));
-    // leave the handle at the final state again
-    return state_copy(h, t->final_state, t->final_valid, false);
+    return MPM_OK;
 }
 
 // grad views: X, V, F, B of n particles in the reference layout, device or host,

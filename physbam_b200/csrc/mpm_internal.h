@@ -36,6 +36,7 @@ struct PlainRecord {
 
 struct PlainState {
     int64_t n = 0, gn = 0;
+    uint64_t generation = 0;   // bumped whenever device buffers are (re)allocated
     void *X = nullptr, *V = nullptr, *F = nullptr, *B = nullptr;
     void *mass = nullptr, *vol = nullptr, *mu = nullptr, *lam = nullptr, *pft = nullptr;
     uint8_t* valid = nullptr;
@@ -294,6 +295,7 @@ int diff_forward(mpm_handle* h, double dt, int nsteps, int every);
 int diff_backward(mpm_handle* h, const mpm_particles_view* gout, mpm_particles_view* gin, void* gmu, void* glam);
 void diff_free(mpm_handle* h);
 void diff_invalidate(mpm_handle* h);
+void diff_release_graphs(mpm_handle* h);
 
 // helpers
 int set_error(mpm_handle* h, int code, const std::string& msg);

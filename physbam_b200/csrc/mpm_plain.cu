@@ -950,6 +950,7 @@ int plain_alloc(mpm_handle* h, int64_t n)
     size_t e = esize(h);
     int64_t gn = 1;
     for(int k = 0; k < d; k++) gn *= h->sp.counts[k] + 2 * MPM_GHOST;
+    if(s.gn != gn || s.n != n) s.generation++;
     if(s.gn != gn) {
         void** g[] = {&s.gm, &s.gmv, &s.gv0, &s.gf, &s.gv, &s.gvf};
         for(void** p: g) { cudaFree(*p); *p = nullptr; }
@@ -1109,6 +1110,7 @@ int plain_plastic_init(mpm_handle* h)
     const size_t e = esize(h);
     const int64_t m = s.n ? s.n : 1;
     if(!s.Fp) {
+        s.generation++;
         MPM_CUDA(h, cudaMalloc(&s.Fp, m * d * d * e));
         void** pa[] = {&s.mu0, &s.lam0, &s.pdef, &s.rhoF, &s.sigY, &s.vc};
         for(void** p: pa) MPM_CUDA(h, cudaMalloc(p, m * e));
