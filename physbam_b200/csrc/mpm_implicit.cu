@@ -41,7 +41,6 @@ constexpr double kCollisionThickness = 1e-15;   // MPM_OBJECTIVE::collision_thic
 
 template<class T> struct ImpArgs {
     PlainArgs<T> a;
-    T *F0, *X0;                 // particle state at the start of the step (Fn = F0)
     // SVD of the current F: U, Fn V, singular values, stress derivative (9 + 3 + 3),
     // component e of the pass's t-th particle at e n + t (coalesced)
     T *U, *FV, *sig, *dP;
@@ -91,87 +90,72 @@ template<class T, int d> __device__ __forceinline__ void node_position(const Imp
 // ---------------------------------------------------------------------------
 // particle passes (weights of the particle positions at the start of the step)
 // ---------------------------------------------------------------------------
-template<class T, int d> __global__ void k_imp_save(ImpArgs<T> ia)
-{
-    const PlainArgs<T>& a = ia.a;
-    for(int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n; p += (int64_t)gridDim.x * blockDim.x) {
-        for(int e = 0; e < d * d; e++) ia.F0[p * d * d + e] = a.F[p * d * d + e];
-        for(int e = 0; e < d; e++) ia.X0[p * d + e] = a.X[p * d + e];
-    }
-}
+// What an evaluation leaves behind besides the force factors.
+enum { EVAL_ENERGY = 1, EVAL_DERIVATIVE = 2 };
 
-// MPM_OBJECTIVE::Restore_F
-template<class T, int d> __global__ void k_imp_restore(ImpArgs<T> ia)
-{
-    const PlainArgs<T>& a = ia.a;
-    for(int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n; p += (int64_t)gridDim.x * blockDim.x) {
-        for(int e = 0; e < d * d; e++) a.F[p * d * d + e] = ia.F0[p * d * d + e];
-        for(int e = 0; e < d; e++) a.X[p * d + e] = ia.X0[p * d + e];
-    }
-}
-
-// MPM_OBJECTIVE::Update_F (l.96-131): F = (I + dt grad v) F0, X = X0 + dt V_p.
-template<class T, int d> __global__ void k_imp_update_F(ImpArgs<T> ia, const T* v)
+// MPM_OBJECTIVE::Update_F (l.96-131), F = (I + dt grad v) Fn and X = Xn + dt V_p, in
+// registers: the particles keep the state of the step's start, so nothing is saved or
+// restored.  Then
+// MPM_FINITE_ELEMENTS::Precompute (l.47-67) on F, and as asked the stress derivative
+// (only the evaluation before a CG needs it: 36 of the 46 values stored) and the
+// potential energy of the particle (Energy_Density times volume, l.71-80, plus
+// MPM_GRAVITY::Potential_Energy, MPM_GRAVITY.cpp:48-57).
+template<class T, int d> __global__ void k_imp_evaluate(ImpArgs<T> ia, const T* v, int what)
 {
     const PlainArgs<T>& a = ia.a;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if(t >= a.n) return;
     const int64_t p = particle_at(ia, t);
-    if(!a.valid[p]) return;
+    T F[9], X[3];
+#pragma unroll
+    for(int e = 0; e < d * d; e++) F[e] = a.F[p * d * d + e];
+#pragma unroll
+    for(int k = 0; k < d; k++) X[k] = a.X[p * d + k];
+    const T* F0 = a.F + p * d * d;
     Stencil<T, d> s;
-    if(!make_stencil<T, d>(a, ia.X0 + p * d, s)) return;
-    T Vp[3] = {0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const int nq = d == 3 ? 27 : 9;
-    for(int q = 0; q < nq; q++) {
-        int64_t i;
-        T w, g[3], Z[3];
-        node<T, d>(a, s, q, i, w, g, Z);
+    if(a.valid[p] && make_stencil<T, d>(a, X, s)) {
+        T Vp[3] = {0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        const int nq = d == 3 ? 27 : 9;
+        for(int q = 0; q < nq; q++) {
+            int64_t i;
+            T w, g[3], Z[3];
+            node<T, d>(a, s, q, i, w, g, Z);
 #pragma unroll
-        for(int r = 0; r < d; r++) {
-            const T vr = v[i * d + r];
-            Vp[r] += w * vr;
+            for(int r = 0; r < d; r++) {
+                const T vr = v[i * d + r];
+                Vp[r] += w * vr;
 #pragma unroll
-            for(int c = 0; c < d; c++) G[r + d * c] += vr * g[c];
+                for(int c = 0; c < d; c++) G[r + d * c] += vr * g[c];
+            }
         }
+        T F1[9];
+#pragma unroll
+        for(int c = 0; c < d; c++)
+#pragma unroll
+            for(int r = 0; r < d; r++) {
+                T sum = F[r + d * c];
+#pragma unroll
+                for(int k = 0; k < d; k++) sum += a.dt * G[r + d * k] * F[k + d * c];
+                F1[r + d * c] = sum;
+            }
+#pragma unroll
+        for(int e = 0; e < d * d; e++) F[e] = F1[e];
+#pragma unroll
+        for(int k = 0; k < d; k++) X[k] += a.dt * Vp[k];
     }
-    const T* F0 = ia.F0 + p * d * d;
-#pragma unroll
-    for(int c = 0; c < d; c++)
-#pragma unroll
-        for(int r = 0; r < d; r++) {
-            T sum = F0[r + d * c];
-#pragma unroll
-            for(int k = 0; k < d; k++) sum += a.dt * G[r + d * k] * F0[k + d * c];
-            a.F[p * d * d + r + d * c] = sum;
-        }
-#pragma unroll
-    for(int r = 0; r < d; r++) a.X[p * d + r] = ia.X0[p * d + r] + a.dt * Vp[r];
-}
-
-// MPM_FINITE_ELEMENTS::Precompute (l.47-67) on the current F with Fn = F0, the
-// stress derivative, and the potential energy of the particle (Energy_Density
-// times volume, l.71-80, plus MPM_GRAVITY::Potential_Energy, MPM_GRAVITY.cpp:48-57).
-template<class T, int d> __global__ void k_imp_precompute(ImpArgs<T> ia)
-{
-    const PlainArgs<T>& a = ia.a;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if(t >= a.n) return;
-    const int64_t p = particle_at(ia, t);
     // IMPLICIT_OBJECT_COLLISION_PENALTY_FORCES::Update_Position_Based_State
     // runs over every particle, simulated or not (its energy counts them all).
     double epen = 0;
     if(a.sp.npen) {
         T fp[3] = {0, 0, 0}, Hp[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         epen = (double)penalty_particle<T, d>(a.sp.pen, a.sp.npen, (T)a.sp.pen_stiffness, (T)a.sp.pen_separation,
-                                              a.X + p * d, fp, Hp);
+                                              X, fp, Hp);
         T* q = ia.pen + p * (d + d * d);
         for(int e = 0; e < d; e++) q[e] = fp[e];
         for(int e = 0; e < d * d; e++) q[d + e] = Hp[e];
     }
     if(!a.valid[p]) { ia.pe[p] = epen; return; }
-    T F[9], U[9], V[9], S[3], P[3];
-#pragma unroll
-    for(int e = 0; e < d * d; e++) F[e] = a.F[p * d * d + e];
+    T U[9], V[9], S[3], P[3];
     bool ok = true;
     if(d == 3) ok = svd3<T>(F, U, S, V);
     else svd2<T>(F, U, S, V);
@@ -179,7 +163,6 @@ template<class T, int d> __global__ void k_imp_precompute(ImpArgs<T> ia)
     const T mu = a.mu[p], la = a.lam[p];
     const int model = model_of(a, p);
     phat<T, d>(model, S, mu, la, P);
-    const T* F0 = ia.F0 + p * d * d;
     T FV[9];
 #pragma unroll
     for(int c = 0; c < d; c++)
@@ -200,18 +183,21 @@ template<class T, int d> __global__ void k_imp_precompute(ImpArgs<T> ia)
             for(int k = 0; k < d; k++) sum += U[r + d * k] * P[k] * FV[c + d * k];
             a.pft[p * d * d + r + d * c] = sum;
         }
-    T H[9], Bv[3], Cv[3];
-    stress_derivative<T, d>(model, S, mu, la, H, Bv, Cv);
+    if(what & EVAL_DERIVATIVE) {
+        T H[9], Bv[3], Cv[3];
+        stress_derivative<T, d>(model, S, mu, la, H, Bv, Cv);
 #pragma unroll
-    for(int e = 0; e < d * d; e++) { ia.U[e * a.n + t] = U[e]; ia.FV[e * a.n + t] = FV[e]; }
+        for(int e = 0; e < d * d; e++) { ia.U[e * a.n + t] = U[e]; ia.FV[e * a.n + t] = FV[e]; }
 #pragma unroll
-    for(int e = 0; e < d; e++) ia.sig[e * a.n + t] = S[e];
+        for(int e = 0; e < d; e++) ia.sig[e * a.n + t] = S[e];
 #pragma unroll
-    for(int e = 0; e < 9; e++) ia.dP[e * a.n + t] = H[e];
+        for(int e = 0; e < 9; e++) ia.dP[e * a.n + t] = H[e];
 #pragma unroll
-    for(int e = 0; e < 3; e++) { ia.dP[(9 + e) * a.n + t] = Bv[e]; ia.dP[(12 + e) * a.n + t] = Cv[e]; }
+        for(int e = 0; e < 3; e++) { ia.dP[(9 + e) * a.n + t] = Bv[e]; ia.dP[(12 + e) * a.n + t] = Cv[e]; }
+    }
+    if(!(what & EVAL_ENERGY)) return;
     double e = (double)a.vol[p] * (double)energy_density<T, d>(model, S, mu, la);
-    for(int k = 0; k < d; k++) e -= (double)a.mass[p] * (double)a.X[p * d + k] * a.sp.gravity[k];
+    for(int k = 0; k < d; k++) e -= (double)a.mass[p] * (double)X[k] * a.sp.gravity[k];
     ia.pe[p] = e + epen;
 }
 
@@ -228,7 +214,7 @@ template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_im
     if(t < a.n) {
         const int64_t p = particle_at(ia, t);
         Stencil<T, d> s;
-        if(a.valid[p] && make_stencil<T, d>(a, ia.X0 + p * d, s)) {
+        if(a.valid[p] && make_stencil<T, d>(a, a.X + p * d, s)) {
             first = first_node<T, d>(a, s);
             T A[d * d], c[d];
             const T vol = a.vol[p], mp = a.mass[p];
@@ -236,7 +222,7 @@ template<class T, int d> __global__ void __launch_bounds__(kScatterThreads) k_im
             for(int e = 0; e < d * d; e++) A[e] = -a.pft[p * d * d + e] * vol;
 #pragma unroll
             for(int e = 0; e < d; e++) c[e] = mp * (T)a.sp.gravity[e] + (a.sp.npen ? ia.pen[p * (d + d * d) + e] : (T)0);
-            scatter_row<T, d>(S.row[lane], s.ax, ia.X0 + p * d, a.sp.dmin, a.sp.dx, c, nullptr, A, (T)0);
+            scatter_row<T, d>(S.row[lane], s.ax, a.X + p * d, a.sp.dmin, a.sp.dx, c, nullptr, A, (T)0);
         }
     }
     S.base[lane] = first;
@@ -259,7 +245,7 @@ template<class T, int d> __device__ __forceinline__ int64_t hessian_row(const Im
     const int64_t p = particle_at(ia, t);
     if(!a.valid[p]) return -1;
     Stencil<T, d> s;
-    if(!make_stencil<T, d>(a, ia.X0 + p * d, s)) return -1;
+    if(!make_stencil<T, d>(a, a.X + p * d, s)) return -1;
     T W[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, zp[3] = {0, 0, 0};
     const bool pen = a.sp.npen != 0;
     const int nq = d == 3 ? 27 : 9;
@@ -329,7 +315,7 @@ template<class T, int d> __device__ __forceinline__ int64_t hessian_row(const Im
             for(int k = 0; k < d; k++) sum += UD[r + d * k] * FV[c + d * k];
             M[r + d * c] = sum * vol;
         }
-    scatter_row<T, d>(row, s.ax, ia.X0 + p * d, a.sp.dmin, a.sp.dx, Hz, nullptr, M, (T)0);
+    scatter_row<T, d>(row, s.ax, a.X + p * d, a.sp.dmin, a.sp.dx, Hz, nullptr, M, (T)0);
     return first_node<T, d>(a, s);
 }
 
@@ -373,15 +359,6 @@ template<class T, int d> __global__ void k_imp_copy(ImpArgs<T> ia, T* out, T c, 
 {
     mass_nodes(ia, [&](int64_t i) {
         for(int k = 0; k < d; k++) out[i * d + k] = c * x[i * d + k] + (y ? y[i * d + k] : (T)0);
-    });
-}
-
-// gradient of MPM_OBJECTIVE::Compute_Unconstrained (l.71-91): g = dv - dt/m f
-template<class T, int d> __global__ void k_imp_grad(ImpArgs<T> ia, T* g, const T* dv, const T* f)
-{
-    mass_nodes(ia, [&](int64_t i) {
-        const T s = ia.a.dt / ia.a.gm[i];
-        for(int k = 0; k < d; k++) g[i * d + k] = dv[i * d + k] - s * f[i * d + k];
     });
 }
 
@@ -480,79 +457,129 @@ __global__ void k_imp_max_final(const double* partial, int count, double* out)
 // the node onto the object (or to the object's velocity for a sticky one) and
 // records the collision; an earlier object's projection feeds the next one's
 // test.  A moving object is tested at its frames of the substep's start and end.
+template<class T, int d> __device__ __forceinline__ void adjust_node(const ImpArgs<T>& ia, int64_t i, T* dv)
+{
+    const PlainArgs<T>& a = ia.a;
+    uint8_t mask = 0, stuck = 0;
+    T X0[3];
+    node_position<T, d>(ia, i, X0);
+    for(int j = 0; j < ia.nobj; j++) {
+        const DevObject& o = a.sp.objs[j];
+        T V[3], X[3];
+#pragma unroll
+        for(int k = 0; k < d; k++) { V[k] = a.gv0[i * d + k] + dv[k]; X[k] = X0[k] + a.dt * V[k]; }
+        const T phi0 = phi_at<T, d>(o, a.motion, a.moving, j, false, X0);
+        const T phi = phi_at<T, d>(o, a.motion, a.moving, j, true, X) - fmin(phi0, (T)0);
+        if(o.type == MPM_STICK && phi0 > 0) continue;
+        if(o.type == MPM_SLIP && phi0 > 0) continue;
+        if(o.type == MPM_SEPARATE && phi > (T)kCollisionThickness) continue;
+        if(o.type != MPM_STICK && phi > (T)FLT_MAX) continue;
+        T n[3];
+        normal_at<T, d>(o, a.motion, a.moving, j, X, n);
+        T* cd = ia.cdat + (i * ia.nobj + j) * (2 + 3 * d);
+        cd[0] = phi;
+        cd[1] = 0;
+        for(int k = 0; k < d; k++) { cd[2 + k] = n[k]; cd[2 + d + k] = X[k]; cd[2 + 2 * d + k] = 0; }
+        mask |= (uint8_t)(1u << j);
+        for(int k = 0; k < d; k++) { X[k] -= phi * n[k]; V[k] = (X[k] - X0[k]) / a.dt; }
+        if(o.type == MPM_STICK) {
+            velocity_at<T, d>(a.motion, a.moving, j, X, V);
+            for(int k = 0; k < d; k++) ia.svel[i * d + k] = V[k];
+            stuck = 1;
+        }
+        for(int k = 0; k < d; k++) dv[k] = V[k] - a.gv0[i * d + k];
+    }
+    ia.cmask[i] = mask;
+    ia.stuck[i] = stuck;
+}
+
 template<class T, int d> __global__ void k_imp_adjust(ImpArgs<T> ia, T* dv)
 {
-    mass_nodes(ia, [&](int64_t i) {
-        const PlainArgs<T>& a = ia.a;
-        uint8_t mask = 0, stuck = 0;
-        T X0[3];
-        node_position<T, d>(ia, i, X0);
-        for(int j = 0; j < ia.nobj; j++) {
-            const DevObject& o = a.sp.objs[j];
-            T V[3], X[3];
+    mass_nodes(ia, [&](int64_t i) { adjust_node<T, d>(ia, i, dv + i * d); });
+}
+
+// The node work of an evaluation before the particles': the point x + t dx (dx null:
+// x), its feasible copy (Adjust_For_Collision), the velocity v0 + dv there, the force
+// cleared, and the sum m |dv|^2 of the energy.
+template<class T, int d> __global__ void __launch_bounds__(kRedThreads) k_imp_point(ImpArgs<T> ia, const T* x, const T* dx, T t,
+    T* feasible, T* v, T* f, Reduction red)
+{
+    double acc = 0;
+    for_nodes(ia.a, [&](int64_t i) {
 #pragma unroll
-            for(int k = 0; k < d; k++) { V[k] = a.gv0[i * d + k] + dv[i * d + k]; X[k] = X0[k] + a.dt * V[k]; }
-            const T phi0 = phi_at<T, d>(o, a.motion, a.moving, j, false, X0);
-            const T phi = phi_at<T, d>(o, a.motion, a.moving, j, true, X) - fmin(phi0, (T)0);
-            if(o.type == MPM_STICK && phi0 > 0) continue;
-            if(o.type == MPM_SLIP && phi0 > 0) continue;
-            if(o.type == MPM_SEPARATE && phi > (T)kCollisionThickness) continue;
-            if(o.type != MPM_STICK && phi > (T)FLT_MAX) continue;
-            T n[3];
-            normal_at<T, d>(o, a.motion, a.moving, j, X, n);
-            T* cd = ia.cdat + (i * ia.nobj + j) * (2 + 3 * d);
-            cd[0] = phi;
-            cd[1] = 0;
-            for(int k = 0; k < d; k++) { cd[2 + k] = n[k]; cd[2 + d + k] = X[k]; cd[2 + 2 * d + k] = 0; }
-            mask |= (uint8_t)(1u << j);
-            for(int k = 0; k < d; k++) { X[k] -= phi * n[k]; V[k] = (X[k] - X0[k]) / a.dt; }
-            if(o.type == MPM_STICK) {
-                velocity_at<T, d>(a.motion, a.moving, j, X, V);
-                for(int k = 0; k < d; k++) ia.svel[i * d + k] = V[k];
-                stuck = 1;
-            }
-            for(int k = 0; k < d; k++) dv[i * d + k] = V[k] - a.gv0[i * d + k];
+        for(int k = 0; k < d; k++) f[i * d + k] = 0;
+        if(ia.a.gm[i] == 0) return;
+        T dv[3];
+#pragma unroll
+        for(int k = 0; k < d; k++) dv[k] = dx ? t * dx[i * d + k] + x[i * d + k] : x[i * d + k];
+        if(ia.nobj) adjust_node<T, d>(ia, i, dv);
+#pragma unroll
+        for(int k = 0; k < d; k++) {
+            feasible[i * d + k] = dv[k];
+            v[i * d + k] = dv[k] + ia.a.gv0[i * d + k];
         }
-        ia.cmask[i] = mask;
-        ia.stuck[i] = stuck;
+        acc += node_dot<T, d>(ia, i, dv, dv);
     });
+    grid_sum(acc, red);
 }
 
 // MPM_OBJECTIVE::Project_Gradient_And_Prune_Constraints (l.226-248): the
 // collisions in reverse order; one whose node may leave the object (separate
 // with allow_sep, or not penetrating) and whose gradient points out of it is
 // dropped, else the normal part of the gradient is removed.
+template<class T, int d> __device__ __forceinline__ void project_node(const ImpArgs<T>& ia, int64_t i, T* g, int allow_sep)
+{
+    uint8_t mask = ia.cmask[i];
+    if(!mask && !ia.stuck[i]) return;
+    if(ia.stuck[i])
+        for(int k = 0; k < d; k++) g[k] = 0;
+    for(int j = ia.nobj - 1; j >= 0; j--) {
+        if(!(mask & (1u << j))) continue;
+        T* cd = ia.cdat + (i * ia.nobj + j) * (2 + 3 * d);
+        T ndE = 0;
+        for(int k = 0; k < d; k++) ndE += g[k] * cd[2 + k];
+        cd[1] = ndE;
+        const bool sep = ia.a.sp.objs[j].type == MPM_SEPARATE;
+        if(((allow_sep && sep) || cd[0] <= (T)kCollisionThickness) && ndE < 0) {
+            mask &= (uint8_t)~(1u << j);
+            continue;
+        }
+        // H_dE = H g; g -= n_dE n + phi H_dE
+        T H[9], gv[3];
+        hessian_at<T, d>(ia.a.sp.objs[j], ia.a.motion, ia.a.moving, j, cd + 2 + d, H);
+        for(int k = 0; k < d; k++) gv[k] = g[k];
+        for(int r = 0; r < d; r++) {
+            T hd = 0;
+            for(int c = 0; c < d; c++) hd += H[r + d * c] * gv[c];
+            cd[2 + 2 * d + r] = hd;
+        }
+        for(int k = 0; k < d; k++) g[k] -= ndE * cd[2 + k] + cd[0] * cd[2 + 2 * d + k];
+    }
+    ia.cmask[i] = mask;
+}
+
 template<class T, int d> __global__ void k_imp_project(ImpArgs<T> ia, T* g, int allow_sep)
 {
+    mass_nodes(ia, [&](int64_t i) { project_node<T, d>(ia, i, g + i * d, allow_sep); });
+}
+
+// ... and after them: the gradient of Compute_Unconstrained (l.71-91), g = dv - dt/m f,
+// projected as asked (project < 0: not), and its product with y (null: with itself).
+template<class T, int d> __global__ void __launch_bounds__(kRedThreads) k_imp_gradient(ImpArgs<T> ia, T* g, const T* dv, const T* f,
+    int project, const T* y, Reduction red)
+{
+    double acc = 0;
     mass_nodes(ia, [&](int64_t i) {
-        uint8_t mask = ia.cmask[i];
-        if(!mask && !ia.stuck[i]) return;
-        if(ia.stuck[i])
-            for(int k = 0; k < d; k++) g[i * d + k] = 0;
-        for(int j = ia.nobj - 1; j >= 0; j--) {
-            if(!(mask & (1u << j))) continue;
-            T* cd = ia.cdat + (i * ia.nobj + j) * (2 + 3 * d);
-            T ndE = 0;
-            for(int k = 0; k < d; k++) ndE += g[i * d + k] * cd[2 + k];
-            cd[1] = ndE;
-            const bool sep = ia.a.sp.objs[j].type == MPM_SEPARATE;
-            if(((allow_sep && sep) || cd[0] <= (T)kCollisionThickness) && ndE < 0) {
-                mask &= (uint8_t)~(1u << j);
-                continue;
-            }
-            // H_dE = H g; g -= n_dE n + phi H_dE
-            T H[9], gv[3];
-            hessian_at<T, d>(ia.a.sp.objs[j], ia.a.motion, ia.a.moving, j, cd + 2 + d, H);
-            for(int k = 0; k < d; k++) gv[k] = g[i * d + k];
-            for(int r = 0; r < d; r++) {
-                T hd = 0;
-                for(int c = 0; c < d; c++) hd += H[r + d * c] * gv[c];
-                cd[2 + 2 * d + r] = hd;
-            }
-            for(int k = 0; k < d; k++) g[i * d + k] -= ndE * cd[2 + k] + cd[0] * cd[2 + 2 * d + k];
-        }
-        ia.cmask[i] = mask;
+        const T s = ia.a.dt / ia.a.gm[i];
+        T gi[3];
+#pragma unroll
+        for(int k = 0; k < d; k++) gi[k] = dv[i * d + k] - s * f[i * d + k];
+        if(project >= 0) project_node<T, d>(ia, i, gi, project);
+#pragma unroll
+        for(int k = 0; k < d; k++) g[i * d + k] = gi[k];
+        acc += node_dot<T, d>(ia, i, gi, y ? y + i * d : gi);
     });
+    grid_sum(acc, red);
 }
 
 // The node passes of a CG iteration (CONJUGATE_GRADIENT.cpp:20-85), three
@@ -709,14 +736,14 @@ struct ImplicitState {
     int nobj = 0, d = 0;
     size_t esz = 0;
     void* vec = nullptr;           // V_COUNT node vectors of gn * d scalars
-    void* part = nullptr;          // F0, X0, U, FV, sig, dP, pen
+    void* part = nullptr;          // U, FV, sig, dP, pen
     double* pe = nullptr;
     uint8_t* cmask = nullptr;
     uint8_t* stuck = nullptr;
     void* cdat = nullptr;
-    double* partial = nullptr;     // 2 * kRedBlocks
-    unsigned* done = nullptr;      // finished CTAs of the 2 reductions
-    double* dout = nullptr;        // 2 results
+    double* partial = nullptr;     // 3 * kRedBlocks
+    unsigned* done = nullptr;      // finished CTAs of the 3 reductions
+    double* dout = nullptr;        // 3 results
     double* hout = nullptr;        // the same in pinned host memory
     uint32_t *keys = nullptr, *sorted = nullptr, *perm = nullptr, *alt_k = nullptr, *alt_v = nullptr, *scratch = nullptr;
     int key_bits = 1;
@@ -740,7 +767,7 @@ template<class T, int d> struct Solver {
         ia.a = args<T>(h, dt);
         const int64_t n = s.n ? s.n : 1;
         T* P = (T*)s.part;
-        ia.F0 = P; ia.X0 = P + n * d * d; ia.U = ia.X0 + n * d; ia.FV = ia.U + n * d * d;
+        ia.U = P; ia.FV = ia.U + n * d * d;
         ia.sig = ia.FV + n * d * d; ia.dP = ia.sig + n * d; ia.pen = ia.dP + n * 15;
         ia.pe = s.pe; ia.cmask = s.cmask; ia.stuck = s.stuck; ia.cdat = (T*)s.cdat; ia.nobj = h->sp.nobj;
         ia.order = nullptr;
@@ -777,17 +804,6 @@ template<class T, int d> struct Solver {
         check("implicit dot");
         return s.hout[0];
     }
-    // m-weighted |x|^2 / 2 + potential energy, in one read-back
-    double energy(const T* x)
-    {
-        ImplicitState& s = *h->imp;
-        k_imp_dot<T, d><<<rb, kRedThreads, 0, st>>>(ia, x, x, reduction(0));
-        k_imp_sum_particles<<<rb, kRedThreads, 0, st>>>(s.pe, s.n, reduction(1));
-        cudaStreamSynchronize(st);
-        check("implicit energy");
-        return s.hout[0] / 2 + s.hout[1];
-    }
-
     // vector ops on nodes with mass ---------------------------------------
     void copy(T* out, T c, const T* x, const T* y = nullptr) { k_imp_copy<T, d><<<gb, 256, 0, st>>>(ia, out, c, x, y); }
     void zero(T* x, int count = 1) { k_imp_zero<T, d><<<gb, 256, 0, st>>>(ia, x, ia.a.gn * d, count); }
@@ -803,27 +819,30 @@ template<class T, int d> struct Solver {
         if(!ia.nobj) return;
         k_imp_project<T, d><<<gb, 256, 0, st>>>(ia, g, allow_sep ? 1 : 0);
     }
-    // Compute_Unconstrained: F, X at v0 + dv; forces, gradient and energy as asked
-    void compute_unconstrained(const T* dv, T* g, double* e)
+    // The particles' part of Compute_Unconstrained (l.71-91): stress at the velocity
+    // v[V_V1] and the forces, into v[V_TMP2] (cleared).  A step limited by the sound speed
+    // reads the last evaluation's stress derivative.
+    void particles(bool energy, bool derivative)
     {
-        copy(v[V_V1], 1, dv, ia.a.gv0);
-        k_imp_update_F<T, d><<<pb, 128, 0, st>>>(ia, v[V_V1]);
-        k_imp_precompute<T, d><<<pb, 128, 0, st>>>(ia);
-        if(e) *e = energy(dv);
-        if(g) {
-            zero(v[V_TMP2]);
-            k_imp_forces<T, d><<<pb, kScatterThreads, 0, st>>>(ia, v[V_TMP2]);
-            k_imp_grad<T, d><<<gb, 256, 0, st>>>(ia, g, dv, v[V_TMP2]);
-        }
-        check("compute_unconstrained");
+        ImplicitState& s = *h->imp;
+        const int what = (energy ? EVAL_ENERGY : 0) | (derivative || h->dt_control.sound_cfl ? EVAL_DERIVATIVE : 0);
+        k_imp_evaluate<T, d><<<pb, 128, 0, st>>>(ia, v[V_V1], what);
+        if(energy) k_imp_sum_particles<<<rb, kRedThreads, 0, st>>>(s.pe, s.n, reduction(1));
+        k_imp_forces<T, d><<<pb, kScatterThreads, 0, st>>>(ia, v[V_TMP2]);
     }
-    // Compute (l.48-65): at the feasible copy of dv; the gradient projected
-    void compute(const T* dv, bool hess, T* g, double* e)
+    // Compute (l.48-65) at the feasible copy of x + t dx (dx null: x): the gradient g,
+    // projected, its product with y (null: with itself), and the energy as asked; one
+    // read-back.
+    double compute(const T* x, const T* dx, double t, bool hess, T* g, const T* y, double* e)
     {
-        copy(v[V_TMP1], 1, dv);
-        adjust(v[V_TMP1]);
-        compute_unconstrained(v[V_TMP1], g, e);
-        if(g) project(g, hess);
+        ImplicitState& s = *h->imp;
+        k_imp_point<T, d><<<rb, kRedThreads, 0, st>>>(ia, x, dx, (T)t, v[V_TMP1], v[V_V1], v[V_TMP2], reduction(0));
+        particles(e != nullptr, hess);
+        k_imp_gradient<T, d><<<rb, kRedThreads, 0, st>>>(ia, g, v[V_TMP1], v[V_TMP2], ia.nobj ? (hess ? 1 : 0) : -1, y, reduction(2));
+        cudaStreamSynchronize(st);
+        check("implicit compute");
+        if(e) *e = s.hout[0] / 2 + s.hout[1];
+        return s.hout[2];
     }
     void make_feasible(T* x) { adjust(x); }
 
@@ -865,9 +884,7 @@ template<class T, int d> struct Solver {
     // PARAMETRIC_LINE::Compute for the line search: objective along x + t dx
     void line_eval(const T* x, const T* dx, double t, double& f, double& df)
     {
-        copy(v[V_GRAD], (T)t, dx, x);              // the reference reuses grad as the point
-        compute(v[V_GRAD], false, v[V_TM], &f);
-        df = dot(v[V_TM], dx);
+        df = compute(x, dx, t, false, v[V_TM], dx, &f);
     }
 
     struct Wolfe { double a, fa, dfa; };
@@ -925,11 +942,9 @@ template<class T, int d> struct Solver {
     {
         double e0 = 0, e1 = 0;
         zero(dv);
-        compute(dv, false, v[V_TMP0], &e0);
+        const double g0 = sqrt(compute(dv, nullptr, 0, false, v[V_TMP0], nullptr, &e0));
         copy(dv, -1, v[V_TMP0]);
-        const double g0 = sqrt(dot(v[V_TMP0], v[V_TMP0]));
-        compute(dv, false, v[V_TMP0], &e1);
-        const double g1 = sqrt(dot(v[V_TMP0], v[V_TMP0]));
+        const double g1 = sqrt(compute(dv, nullptr, 0, false, v[V_TMP0], nullptr, &e1));
         if(e1 < std::max(e0, e0 * 1.1)) return true;
         if(g1 < g0 * 1.1 || g1 < tolerance) return true;
         zero(dv);
@@ -949,8 +964,8 @@ template<class T, int d> struct Solver {
         make_feasible(x);
         int it;
         for(it = 0; it < local_max && !failed(); it++) {
-            compute(x, true, grad, nullptr);   // the energy only feeds the reference's log
-            const double norm_grad = sqrt(dot(grad, grad)), conv = norm_grad;
+            // the energy only feeds the reference's log
+            const double norm_grad = sqrt(compute(x, nullptr, 0, true, grad, nullptr, nullptr)), conv = norm_grad;
             h->imp_stats.residual = conv;
             if(conv < tolerance && (it || !require_one || !conv)) { result = true; break; }
             if(conv < countdown_tolerance) { result = true; local_max = std::min(local_max, it + countdown_iterations); }
@@ -985,7 +1000,6 @@ template<class T, int d> struct Solver {
             check("implicit keys");
             if((rc = sort_keys_device(h, s.keys, s.n, s.key_bits, s.sorted, s.perm, s.alt_k, s.alt_v, s.scratch))) return rc;
             ia.order = s.perm;
-            k_imp_save<T, d><<<pb, 128, 0, st>>>(ia);
         }
         zero(v[0], V_COUNT);
         if(ia.nobj) {
@@ -1000,14 +1014,16 @@ template<class T, int d> struct Solver {
         if(failed()) return rc;
         // Apply_Friction: velocity_friction_save = dv; Coulomb friction on the collisions
         if(ia.nobj) {
-            compute_unconstrained(dv, v[V_TMP0], nullptr);
+            copy(v[V_V1], 1, dv, ia.a.gv0);
+            zero(v[V_TMP2]);
+            particles(false, false);
+            k_imp_gradient<T, d><<<rb, kRedThreads, 0, st>>>(ia, v[V_TMP0], dv, v[V_TMP2], -1, nullptr, reduction(2));
             copy(v[V_TMP1], 1, v[V_TMP0]);
             project(v[V_TMP1], true);
             k_imp_friction<T, d><<<gb, 256, 0, st>>>(ia, dv, v[V_TMP0], v[V_TMP1], v[V_VFS]);
         } else {
             copy(v[V_VFS], 1, dv);
         }
-        if(s.n) k_imp_restore<T, d><<<pb, 128, 0, st>>>(ia);
         k_imp_finish<T, d><<<gb, 256, 0, st>>>(ia, dv, v[V_VFS]);
         // Reflect_Boundary_Velocity on velocity and velocity_friction_save (MPM_DRIVER.cpp:1055-1057)
         if(h->reflect.enabled && !h->reflect.full_reflection) plain_reflect_velocity(h);
@@ -1033,18 +1049,18 @@ template<class T> int ensure_state(mpm_handle* h)
     t.gn = ps.gn; t.n = ps.n; t.nobj = h->sp.nobj; t.d = d; t.esz = e;
     const int64_t n = t.n ? t.n : 1;
     MPM_CUDA(h, cudaMalloc(&t.vec, (size_t)V_COUNT * t.gn * d * e));
-    MPM_CUDA(h, cudaMalloc(&t.part, (size_t)n * (d * d * 4 + d * 3 + 15) * e));
+    MPM_CUDA(h, cudaMalloc(&t.part, (size_t)n * (d * d * 3 + d * 2 + 15) * e));
     MPM_CUDA(h, cudaMalloc(&t.pe, (size_t)n * sizeof(double)));
     MPM_CUDA(h, cudaMalloc(&t.cmask, (size_t)t.gn));
     MPM_CUDA(h, cudaMalloc(&t.stuck, (size_t)t.gn));
     MPM_CUDA(h, cudaMemset(t.cmask, 0, (size_t)t.gn));
     MPM_CUDA(h, cudaMemset(t.stuck, 0, (size_t)t.gn));
     if(t.nobj) MPM_CUDA(h, cudaMalloc(&t.cdat, (size_t)t.gn * t.nobj * (2 + 3 * d) * e));
-    MPM_CUDA(h, cudaMalloc(&t.partial, 2 * kRedBlocks * sizeof(double)));
-    MPM_CUDA(h, cudaMalloc(&t.done, 2 * sizeof(unsigned)));
-    MPM_CUDA(h, cudaMemset(t.done, 0, 2 * sizeof(unsigned)));
-    MPM_CUDA(h, cudaMalloc(&t.dout, 2 * sizeof(double)));
-    MPM_CUDA(h, cudaMallocHost(&t.hout, 2 * sizeof(double)));
+    MPM_CUDA(h, cudaMalloc(&t.partial, 3 * kRedBlocks * sizeof(double)));
+    MPM_CUDA(h, cudaMalloc(&t.done, 3 * sizeof(unsigned)));
+    MPM_CUDA(h, cudaMemset(t.done, 0, 3 * sizeof(unsigned)));
+    MPM_CUDA(h, cudaMalloc(&t.dout, 3 * sizeof(double)));
+    MPM_CUDA(h, cudaMallocHost(&t.hout, 3 * sizeof(double)));
     uint32_t** sb[] = {&t.keys, &t.sorted, &t.perm, &t.alt_k, &t.alt_v};
     for(uint32_t** p: sb) MPM_CUDA(h, cudaMalloc(p, (size_t)n * sizeof(uint32_t)));
     MPM_CUDA(h, cudaMalloc(&t.scratch, (size_t)sort_scratch_words(n) * sizeof(uint32_t)));
