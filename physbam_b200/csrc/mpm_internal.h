@@ -118,7 +118,9 @@ struct FastState {
     bool sorted_now = false;                  // this substep's order is built (P2G may repeat)
     uint32_t* nb_flag = nullptr;              // node-block touched this substep
     uint32_t* nb_list = nullptr;              // touched node blocks
+    uint8_t* nb_differs = nullptr;            // two bytes per node block: its halves hold a node with v_fric != v_new
     uint32_t* counters = nullptr;             // 2 x 16 words, one set per parity: see FastCounter
+    bool grid_marked = false;                 // the last grid update wrote nb_differs (G2P may stream its items)
     int grid_set = 0;                         // counter set of the last grid update (its node blocks)
     float4* acc = nullptr;                    // P2G accumulator: momentum+dt*force (xyz), mass (w)
     float4* vel = nullptr;                    // per node 2 x float4: vnew.xyz, vfric.x | vfric.yz, mass, 0

@@ -89,11 +89,49 @@ def test_fast_item_counts(cuda_device, variant, threads, n):
     check(run_gpu(scene, 10, D().FP32, D().PATH_FAST, shape=(variant, threads, 1)), run_oracle(scene, 10), TOL32)
 
 
+def test_fast_block_of_many_items(cuda_device):
+    """4,500 particles in one block: more work items (64 particles each) than a warp has lanes."""
+    scene = pick(S.small_3d(ppc=24), 4500)
+    scene.X[:] = 0.25 + (0.1 + 3.8 * np.random.default_rng(1).random((scene.n, 3))) / 16
+    assert scene.n == 4500
+    check(run_gpu(scene, 5, D().FP32, D().PATH_FAST, shape=(2, 64, 1)), run_oracle(scene, 5), TOL32)
+
+
 def test_fast_particle_without_mass(cuda_device):
     """A particle of zero mass takes part with its force alone, as on the plain path."""
     scene = pick(S.small_3d(), 700)
     scene.mass[::50] = 0.0
     check(run_gpu(scene, 5, D().FP32, D().PATH_FAST), run_oracle(scene, 5), TOL32)
+
+
+@pytest.mark.parametrize("shape", [(3, 128, 1), (2, 64, 1), (1, 256, 1), (3, 64, 1), (0, 128, 2)])
+def test_fast_many_items_in_two_scenes(cuda_device, shape):
+    """Enough work items that G2P streams them (two and more per CTA), blocks of every fill, a
+    scene change on the way, walls with friction, particles that leave the domain: against the
+    plain path in FP64, scene by scene."""
+    scenes = [S.small_3d(G=88, friction=0.3), S.small_3d(seed=9, G=82, model=S.NEO_HOOKEAN, with_walls=False)]
+    keep = np.random.default_rng(2).random(scenes[1].n) < 0.6
+    scenes[1] = scenes[1].subset(np.flatnonzero(keep))
+    scenes[1].X[:50] = 1.0 - 1e-6
+    scenes[1].V[:50] = 10.0
+    assert sum(s.n for s in scenes) > 2 * 2 * 592 * 128
+    drv = D().MPM_BATCH(scenes)
+    drv.set_launch_shape(*shape)
+    drv.set_scene_particles()
+    drv.advance(4, 1e-5)
+    drv.synchronize()
+    got = drv.split(drv.get_particles())
+    drv.close()
+    for s, g in zip(scenes, got):
+        ref = D().MPM_DRIVER(s, precision=D().FP64, path=D().PATH_PLAIN)
+        ref.set_scene_particles(s)
+        ref.advance(4, 1e-5)
+        r = ref.get_particles()
+        ref.close()
+        np.testing.assert_array_equal(g["valid"], r["valid"])
+        keep, vmax = r["valid"].astype(bool), np.abs(r["V"]).max()
+        for k, scale in (("X", 1.0), ("V", vmax), ("F", 1.0), ("B", vmax / s.dx)):
+            assert np.abs(g[k] - r[k])[keep].max() <= TOL32[k] * scale, k
 
 
 def big(scene_fn, **kw):
