@@ -103,7 +103,7 @@ struct FastState {
     uint32_t* bstart[2] = {nullptr, nullptr}; // per particle block
     uint32_t* bend[2] = {nullptr, nullptr};
     uint4* active[2] = {nullptr, nullptr};    // active particle blocks: (block, start, count, scene)
-    uint4* chunks[2] = {nullptr, nullptr};    // work items, two uint4 each: (block, part, parts, scene), (block start, block count, 0, 0)
+    uint4* chunks[2] = {nullptr, nullptr};    // work items, two uint4 each: (block, first, end, scene), (block x | y << 16, z, 0, 0)
     int64_t chunk_cap = 0;
     // routing from one substep's order to the next (mpm_fast.cu, k_bins / k_route):
     // per block a row of arrival counts by direction (G2P) and the row of their

@@ -1,6 +1,6 @@
-// Plain path: a direct GPU port of the reference's explicit substep, one thread
-// per particle (or grid node), global atomics for every scatter, particles in
-// the reference's MPM_PARTICLES layout and arrival order.  Templated on the
+// Plain path: the reference's explicit substep with particles in its
+// MPM_PARTICLES layout and arrival order, one thread per particle or grid node; the
+// scatters sum runs of particles (mpm_scatter.cuh) and send global atomics.  Templated on the
 // scalar type; in FP64 it is the baseline the FP32 fast path is measured
 // against, and the path whose grids are checked node-for-node against the
 // reference (it keeps velocity_save and separate force arrays like the
