@@ -565,6 +565,7 @@ static int state_copy(mpm_handle* h, void* dst, uint8_t* dvalid, bool to_tape)
         else MPM_CUDA(h, cudaMemcpyAsync(parts[k], d, cnt[k] * e, cudaMemcpyDeviceToDevice, h->stream));
         d += cnt[k] * e;
     }
+    if(!to_tape) s.scattered = false;
     if(to_tape) MPM_CUDA(h, cudaMemcpyAsync(dvalid, s.valid, n, cudaMemcpyDeviceToDevice, h->stream));
     else MPM_CUDA(h, cudaMemcpyAsync(s.valid, dvalid, n, cudaMemcpyDeviceToDevice, h->stream));
     return MPM_OK;
@@ -694,6 +695,7 @@ int diff_forward(mpm_handle* h, double dt, int nsteps, int every)
         return state_copy(h, t->final_state, t->final_valid, true);
     };
     if((rc = t->replay ? replay(h, t->graphs[0], steps) : steps())) return rc;
+    s.scattered = false;
     t->recorded = true;
     return MPM_OK;
 }
@@ -793,6 +795,7 @@ template<class T> static int backward_t(mpm_handle* h, const void* gX, const voi
     };
     const int rc = t->replay ? replay(h, t->graphs[1], passes) : passes();
     if(rc) return rc;
+    s.scattered = false;
     a1 = (T*)t->adj[t->nsteps & 1];   // the adjoint of the initial state
     MPM_CUDA(h, cudaMemcpyAsync(oX, a1, 3 * n * e, cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(oV, a1 + 3 * n, 3 * n * e, cudaMemcpyDeviceToDevice, h->stream));

@@ -258,6 +258,7 @@ static int run_substep(mpm_handle* h, double dt, double time)
     MPM_CUDA(h, cudaGraphLaunch(ge, h->stream));
     h->last_dt = dt;
     if(fast(h)) h->fast.cur = 1 - par;
+    else h->plain.scattered = false;
     return MPM_OK;
 }
 

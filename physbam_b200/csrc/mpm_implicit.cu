@@ -1139,6 +1139,7 @@ void implicit_free(mpm_handle* h)
 
 int plain_implicit_forces(mpm_handle* h, double dt, double)
 {
+    plain_before_forces(h);
     return h->model.precision == MPM_FP64 ? implicit_t<double>(h, dt) : implicit_t<float>(h, dt);
 }
 

@@ -23,7 +23,6 @@ struct SceneParams {
     mpm::DevObject pen[MPM_MAX_OBJECTS];
 };
 
-// Reference-layout device arrays for the plain path (one thread per particle).
 // One substep of a recorded rollout (mpm_adjoint.cu, 3D): the particles are read from
 // `in` (X 3n, V 3n, F 9n, B 9n scalars) and G2P writes them to `out` (null: to the
 // handle's own arrays); P F^T, node mass, velocity and velocity before the
@@ -34,6 +33,7 @@ struct PlainRecord {
     uint32_t *tiles, *tile_count;
 };
 
+// Reference-layout device arrays for the plain path (one thread per particle).
 struct PlainState {
     int64_t n = 0, gn = 0;
     uint64_t generation = 0;   // bumped whenever device buffers are (re)allocated
@@ -47,6 +47,7 @@ struct PlainState {
     uint8_t* tile_flag = nullptr;
     uint32_t *tiles = nullptr, *tile_count = nullptr;
     bool grid_listed = false;
+    bool scattered = false;   // the grid holds a P2G of the particles where they are now
     const PlainRecord* record = nullptr;   // set while a rollout's substep is recorded
     void *Fp = nullptr, *mu0 = nullptr, *lam0 = nullptr;   // plastic state (plasticity on): clamp
     void *pdef = nullptr, *rhoF = nullptr, *sigY = nullptr, *vc = nullptr;   // Drucker-Prager
@@ -236,6 +237,7 @@ int plain_set_particles(mpm_handle* h, const mpm_particles_view* v);
 int plain_get_particles(mpm_handle* h, mpm_particles_view* v);
 int plain_prepare(mpm_handle* h);
 bool plain_listed(const mpm_handle* h);
+void plain_before_forces(mpm_handle* h);
 int plain_p2g(mpm_handle* h, double dt, double time);
 int plain_p2g_forces(mpm_handle* h, double dt);
 int plain_forces(mpm_handle* h, double dt, double time);

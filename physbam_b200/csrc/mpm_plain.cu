@@ -628,6 +628,7 @@ template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_tile_list");
     }
+    h->plain.scattered = true;
     if(a.reflect && !h->reflect.full_reflection && (rc = reflect_pass<T>(h, a, REFLECT_MM))) return rc;
     if(with_forces) return MPM_OK;
     slot = timer_begin(h, "plain_normalize");
@@ -908,6 +909,7 @@ template<class T> int g2p_t(mpm_handle* h, double dt)
 {
     PlainArgs<T> a = args<T>(h, dt);
     if(!a.n) return MPM_OK;
+    h->plain.scattered = false;
     const int t = 128;
     int slot = timer_begin(h, "plain_g2p");
     if(h->sp.dim == 3) launch_chained(k_g2p<T, 3>, pblocks(a.n, t), t, 0, h->stream, a);
@@ -967,6 +969,10 @@ int plain_alloc(mpm_handle* h, int64_t n)
             MPM_CUDA(h, cudaMalloc(&s.tile_flag, span));
             MPM_CUDA(h, cudaMalloc(&s.tiles, nt * sizeof(uint32_t)));
             MPM_CUDA(h, cudaMalloc(&s.tile_count, sizeof(uint32_t)));
+            // an empty list: node passes may come before the first P2G (the phase entry points)
+            MPM_CUDA(h, cudaMemsetAsync(s.tile_flag, 0, span, h->stream));
+            MPM_CUDA(h, cudaMemsetAsync(s.tile_count, 0, sizeof(uint32_t), h->stream));
+            s.grid_listed = true;
         }
     }
     if(s.n != n) {
@@ -993,8 +999,8 @@ int plain_alloc(mpm_handle* h, int64_t n)
 }
 
 // Before a substep, never inside a captured one: the whole grid to zero where the
-// tile list does not describe it (new arrays, or reflection boundaries, whose
-// passes write every node, were on).
+// tile list does not describe it (after reflection boundaries, whose passes write
+// every node, and after plain_before_forces).
 int plain_prepare(mpm_handle* h)
 {
     PlainState& s = h->plain;
@@ -1016,6 +1022,14 @@ int plain_prepare(mpm_handle* h)
 }
 
 bool plain_listed(const mpm_handle* h) { return list_tiles(h); }
+
+// Before a force phase of its own (mpm_apply_forces): particles that no P2G put on the
+// grid where they are now scatter their forces outside the listed tiles, so the passes
+// run over every node, and the next P2G clears the whole grid.
+void plain_before_forces(mpm_handle* h)
+{
+    if(!h->plain.scattered) h->plain.grid_listed = false;
+}
 
 void plain_free(mpm_handle* h)
 {
@@ -1087,6 +1101,7 @@ int plain_set_particles(mpm_handle* h, const mpm_particles_view* v)
     const int d = h->sp.dim;
     bool dev = v->on_device != 0;
     int64_t n = v->n;
+    s.scattered = false;
     if(!n) return MPM_OK;
     if((rc = copy_in(h, s.X, v->X, n * d, v->dtype, dev))) return rc;
     if((rc = copy_in(h, s.V, v->V, n * d, v->dtype, dev))) return rc;
@@ -1219,6 +1234,7 @@ int plain_p2g_forces(mpm_handle* h, double dt)
 }
 int plain_forces(mpm_handle* h, double dt, double)
 {
+    plain_before_forces(h);
     return h->model.precision == MPM_FP64 ? forces_t<double>(h, dt, false) : forces_t<float>(h, dt, false);
 }
 int plain_reflect_velocity(mpm_handle* h)

@@ -165,7 +165,8 @@ template<class T> inline PlainArgs<T> args(mpm_handle* h, double dt)
     a.pmask = s.pmask;
     a.motion = h->motion_dev;
     a.moving = h->motion_dev ? h->moving : 0u;
-    const bool listed = list_tiles(h);
+    // the grid may be of a P2G before list_tiles changed (a setter between the phases)
+    const bool listed = list_tiles(h) && s.grid_listed;
     a.tile_flag = listed ? s.tile_flag : nullptr;
     a.tiles = listed ? s.tiles : nullptr;
     a.tile_count = s.tile_count;

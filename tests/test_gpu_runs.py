@@ -145,6 +145,36 @@ def test_plain_listed_tiles(cuda_device, n):
     check(run_gpu(scene, 10, D().FP64, D().PATH_PLAIN), run_oracle(scene, 10), TOL64)
 
 
+def test_plain_node_passes_before_p2g(cuda_device):
+    """The phase entry points in any order: node passes before the first P2G find an empty tile
+    list; forces of particles that have moved since the last P2G leave nothing on the grid for
+    the next; a grid update after the reflection was switched off runs over the whole grid."""
+    scene = pick(big(S.small_3d, ppc=4), 500)
+    drv = D().MPM_DRIVER(scene, precision=D().FP64, path=D().PATH_PLAIN)
+    drv.set_scene_particles(scene)
+    drv.add_grid_forces(np.ones(tuple(c + 2 * S.GHOST for c in scene.counts) + (3,)))
+    drv.Apply_Forces()
+    drv.advance(3)
+    drv.Apply_Forces()
+    drv.advance(2)
+    drv.synchronize()
+    check(drv.get_particles(), run_oracle(scene, 5), TOL64)
+    grids = []
+    for reflect in (False, True):                  # far from the faces reflection changes nothing
+        drv.set_scene_particles(scene)
+        if reflect:
+            drv.set_reflection(S.Reflection(side_type=(S.BC_SLIP,) * 6))
+        drv.Particle_To_Grid()
+        if reflect:
+            drv.set_reflection(None)
+        drv.Apply_Forces()
+        grids.append(drv.get_grid())
+    drv.close()
+    assert np.abs(grids[0]["grid_v"]).max() > 0
+    for k in grids[0]:
+        np.testing.assert_allclose(grids[1][k], grids[0][k], rtol=0, atol=1e-12 * np.abs(grids[0][k]).max())
+
+
 def test_implicit_listed_tiles(cuda_device):
     """On a grid with listed tiles, over a sticking floor: the solve agrees with itself to the
     Newton tolerance and, at a small step, with the explicit substep.  Backward and symplectic
