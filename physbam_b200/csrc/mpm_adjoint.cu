@@ -597,23 +597,34 @@ template<class T> static int record_substep(mpm_handle* h, DiffTape* t, int j, b
     return rc;
 }
 
+// A group of a tape's buffers, all of them or none (the first one non-null: they are there).
+struct TapeBuffer { void** ptr; size_t bytes; };
+static int alloc_group(mpm_handle* h, const std::vector<TapeBuffer>& group)
+{
+    int rc = MPM_OK;
+    for(const TapeBuffer& b: group)
+        if(!rc) rc = device_alloc(h, b.ptr, b.bytes);
+    if(rc)
+        for(const TapeBuffer& b: group) { cudaFree(*b.ptr); *b.ptr = nullptr; }
+    return rc;
+}
+
 // Tape slots for `slots` substeps (the segment buffers the backward reads).
 static int alloc_segments(mpm_handle* h, DiffTape* t, int slots)
 {
     const int64_t n = t->n, gn = t->gn;
     const size_t e = t->esz, st = 24 * n * e;
-    MPM_CUDA(h, cudaMalloc(&t->seg, slots * st + 1));
-    MPM_CUDA(h, cudaMalloc(&t->seg_valid, slots * n + 1));
-    MPM_CUDA(h, cudaMalloc(&t->seg_gm, slots * gn * e));
-    MPM_CUDA(h, cudaMalloc(&t->seg_gv, slots * gn * 3 * e));
-    MPM_CUDA(h, cudaMalloc(&t->seg_gu, slots * gn * 3 * e));
-    MPM_CUDA(h, cudaMalloc(&t->seg_pft, slots * 9 * n * e + 1));
-    t->ntiles = plain_listed(h) ? (gn + plain::kTileNodes - 1) / plain::kTileNodes : 0;
-    if(t->ntiles) {
-        MPM_CUDA(h, cudaMalloc(&t->seg_tiles, slots * t->ntiles * sizeof(uint32_t)));
-        MPM_CUDA(h, cudaMalloc(&t->seg_count, slots * sizeof(uint32_t)));
+    const int64_t nt = plain_listed(h) ? (gn + plain::kTileNodes - 1) / plain::kTileNodes : 0;
+    std::vector<TapeBuffer> group = {{&t->seg, slots * st + 1}, {(void**)&t->seg_valid, (size_t)(slots * n + 1)},
+        {&t->seg_gm, slots * gn * e}, {&t->seg_gv, slots * gn * 3 * e}, {&t->seg_gu, slots * gn * 3 * e},
+        {&t->seg_pft, slots * 9 * n * e + 1}};
+    if(nt) {
+        group.push_back({(void**)&t->seg_tiles, slots * nt * sizeof(uint32_t)});
+        group.push_back({(void**)&t->seg_count, slots * sizeof(uint32_t)});
     }
-    return MPM_OK;
+    const int rc = alloc_group(h, group);
+    t->ntiles = rc ? 0 : nt;
+    return rc;
 }
 
 // Bytes of the tape slots of one substep.
@@ -656,20 +667,20 @@ int diff_forward(mpm_handle* h, double dt, int nsteps, int every)
         t->n = s.n; t->gn = s.gn; t->nsteps = nsteps; t->every = every;
         t->esz = esz;
         t->full = want_full;
-        if(t->full) {
-            int arc = alloc_segments(h, t, nsteps);
-            if(arc) return arc;
-        }
     }
     t->recorded = false;
     t->dt = dt;
     size_t st = 24 * s.n * t->esz;
     int nck = (nsteps + every - 1) / every;
     if(!reuse) {
-        MPM_CUDA(h, cudaMalloc(&t->ckpt, nck * st + 1));
-        MPM_CUDA(h, cudaMalloc(&t->ckpt_valid, nck * s.n + 1));
-        MPM_CUDA(h, cudaMalloc(&t->final_state, st + 1));
-        MPM_CUDA(h, cudaMalloc(&t->final_valid, s.n + 1));
+        int arc = t->full ? alloc_segments(h, t, nsteps) : MPM_OK;
+        if(!arc)
+            arc = alloc_group(h, {{&t->ckpt, nck * st + 1}, {(void**)&t->ckpt_valid, (size_t)(nck * s.n + 1)},
+                                  {&t->final_state, st + 1}, {(void**)&t->final_valid, (size_t)(s.n + 1)}});
+        if(arc) {      // no tape of this shape: the next call starts from nothing
+            diff_free(h);
+            return arc;
+        }
     }
     t->replay = reuse && t->full;
     if(t->graph_dt != dt) diff_release_graphs(h);
@@ -714,11 +725,9 @@ template<class T> static int backward_t(mpm_handle* h, const void* gX, const voi
         if(arc) return arc;
     }
     if(!t->adj[0]) {
-        for(int k = 0; k < 2; k++) MPM_CUDA(h, cudaMalloc(&t->adj[k], st + 1));
-        MPM_CUDA(h, cudaMalloc(&t->amu, n * e + 1));
-        MPM_CUDA(h, cudaMalloc(&t->alam, n * e + 1));
-        for(int k = 0; k < 2; k++) MPM_CUDA(h, cudaMalloc(&t->ga[k], gn * 3 * e));
-        MPM_CUDA(h, cudaMalloc(&t->gma, gn * e));
+        const int arc = alloc_group(h, {{&t->adj[0], st + 1}, {&t->adj[1], st + 1}, {&t->amu, n * e + 1}, {&t->alam, n * e + 1},
+                                        {&t->ga[0], gn * 3 * e}, {&t->ga[1], gn * 3 * e}, {&t->gma, gn * e}});
+        if(arc) return arc;
     }
     // seed: adjoint of the final state (device arrays of T)
     T* a1 = (T*)t->adj[0];
@@ -843,7 +852,10 @@ int diff_backward(mpm_handle* h, const mpm_particles_view* gout, mpm_particles_v
     }
     int rc = prec == MPM_FP64 ? backward_t<double>(h, dsrc[0], dsrc[1], dsrc[2], dsrc[3], dout[0], dout[1], dout[2], dout[3], dout[4], dout[5])
                               : backward_t<float>(h, dsrc[0], dsrc[1], dsrc[2], dsrc[3], dout[0], dout[1], dout[2], dout[3], dout[4], dout[5]);
-    if(rc) return rc;
+    if(rc) {
+        for(void* p: owned) cudaFreeAsync(p, h->stream);
+        return rc;
+    }
     if(!gin->on_device)
         for(int k = 0; k < 6; k++) MPM_CUDA(h, cudaMemcpyAsync(dst[k], dout[k], cnt[k] * e, cudaMemcpyDeviceToHost, h->stream));
     for(void* p: owned) MPM_CUDA(h, cudaFreeAsync(p, h->stream));

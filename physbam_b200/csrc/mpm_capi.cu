@@ -17,6 +17,16 @@ int set_error(mpm_handle* h, int code, const std::string& msg)
     return code;
 }
 
+int device_alloc(mpm_handle* h, void** ptr, size_t bytes)
+{
+    const bool refused = h->fail_alloc > 0 && --h->fail_alloc == 0;
+    const cudaError_t e = refused ? cudaErrorMemoryAllocation : cudaMalloc(ptr, bytes);
+    if(e == cudaSuccess) return MPM_OK;
+    *ptr = nullptr;
+    cudaGetLastError();   // reported here, not by the next launch
+    return check_cuda(h, e, "cudaMalloc");
+}
+
 int check_cuda(mpm_handle* h, cudaError_t e, const char* what)
 {
     std::string msg = std::string(what) + ": " + cudaGetErrorString(e);
@@ -164,13 +174,13 @@ static int fill_motion_table(mpm_handle* h, double dt, double time, int nsteps)
         MPM_CUDA(h, cudaStreamSynchronize(h->stream));
         cudaFree(h->motion_table); cudaFree(h->motion_table_f);
         h->motion_table = nullptr; h->motion_table_f = nullptr; h->motion_cap = 0;
-        MPM_CUDA(h, cudaMalloc(&h->motion_table, one * nsteps));
-        MPM_CUDA(h, cudaMalloc(&h->motion_table_f, onef * nsteps));
+        MPM_ALLOC(h, &h->motion_table, one * nsteps);
+        MPM_ALLOC(h, &h->motion_table_f, onef * nsteps);
         h->motion_cap = nsteps;
     }
-    if(!h->motion_slot) MPM_CUDA(h, cudaMalloc(&h->motion_slot, sizeof(unsigned)));
-    if(!h->motion_dev) MPM_CUDA(h, cudaMalloc(&h->motion_dev, one));
-    if(!h->motion_dev_f) MPM_CUDA(h, cudaMalloc(&h->motion_dev_f, onef));
+    if(!h->motion_slot) MPM_ALLOC(h, &h->motion_slot, sizeof(unsigned));
+    if(!h->motion_dev) MPM_ALLOC(h, &h->motion_dev, one);
+    if(!h->motion_dev_f) MPM_ALLOC(h, &h->motion_dev_f, onef);
     std::vector<mpm::ObjMotion> m((size_t)nsteps * MPM_MAX_OBJECTS);
     std::vector<mpm::ObjMotionF> mf((size_t)nsteps * MPM_MAX_OBJECTS);
     for(int s = 0; s < nsteps; s++) {
@@ -202,8 +212,8 @@ int update_motion(mpm_handle* h, double time, double dt)
     mpm::ObjMotionF mf[MPM_MAX_OBJECTS] = {};
     int rc = eval_motion(h, time, dt, m, mf);
     if(rc) return rc;
-    if(!h->motion_dev) MPM_CUDA(h, cudaMalloc(&h->motion_dev, sizeof(m)));
-    if(!h->motion_dev_f) MPM_CUDA(h, cudaMalloc(&h->motion_dev_f, sizeof(mf)));
+    if(!h->motion_dev) MPM_ALLOC(h, &h->motion_dev, sizeof(m));
+    if(!h->motion_dev_f) MPM_ALLOC(h, &h->motion_dev_f, sizeof(mf));
     MPM_CUDA(h, cudaMemcpyAsync(h->motion_dev, m, sizeof(m), cudaMemcpyHostToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(h->motion_dev_f, mf, sizeof(mf), cudaMemcpyHostToDevice, h->stream));
     return MPM_OK;
@@ -400,9 +410,10 @@ int mpm_set_collision_objects(mpm_handle* h, const mpm_collision_object* objs, i
         for(int i = 0; i < count; i++) f.objs_h[i] = h->sp.objs[i];
         f.scenes_h[0].obj_begin = 0;
         f.scenes_h[0].nobj = count;
+        mpm::DevObject* objs_d = nullptr;
+        MPM_ALLOC(h, &objs_d, f.objs_h.size() * sizeof(mpm::DevObject));
         cudaFree(f.objs);
-        f.objs = nullptr;
-        MPM_CUDA(h, cudaMalloc(&f.objs, f.objs_h.size() * sizeof(mpm::DevObject)));
+        f.objs = objs_d;
         MPM_CUDA(h, cudaMemcpy(f.objs, f.objs_h.data(), f.objs_h.size() * sizeof(mpm::DevObject), cudaMemcpyHostToDevice));
         MPM_CUDA(h, cudaMemcpy(f.scenes, f.scenes_h.data(), sizeof(SceneDev), cudaMemcpyHostToDevice));
     }
@@ -419,6 +430,8 @@ int mpm_set_particles(mpm_handle* h, const mpm_particles_view* v)
     // captured substeps hold buffer addresses: keep them only if none moved.  Capturing
     // the plain path's anew was 150 us of the 2D block's 2.1 ms call.
     if(h->fast.generation + h->plain.generation != gen || rc) release_graph(h);
+    // short of memory, the buffers of the old particles are gone as well
+    if(rc && rc != MPM_ERR_ARG) h->have_particles = false;
     if(rc) return rc;
     MPM_CUDA(h, cudaStreamSynchronize(h->stream));
     h->n = v->n;
@@ -636,6 +649,13 @@ int mpm_debug_set_sort_epoch(mpm_handle* h, uint32_t epoch)
     return debug_set_sort_epoch(h, epoch);
 }
 
+int mpm_debug_fail_allocation(mpm_handle* h, int which)
+{
+    if(!h || which < 0) return MPM_ERR_ARG;
+    h->fail_alloc = which;
+    return MPM_OK;
+}
+
 int mpm_debug_set_svd_iterations(int max_it)
 {
     if(max_it < 0 || max_it > 1000000) return MPM_ERR_ARG;
@@ -723,7 +743,7 @@ int mpm_set_penalty_objects(mpm_handle* h, const mpm_collision_object* objs, int
             tab[i].friction = (float)o.friction;
             for(int k = 0; k < 3; k++) { tab[i].a[k] = (float)o.a[k]; tab[i].b[k] = (float)o.b[k]; }
         }
-        if(!h->pen_f) MPM_CUDA(h, cudaMalloc(&h->pen_f, sizeof(tab)));
+        if(!h->pen_f) MPM_ALLOC(h, &h->pen_f, sizeof(tab));
         MPM_CUDA(h, cudaMemcpy(h->pen_f, tab, sizeof(tab), cudaMemcpyHostToDevice));
         return fast_penalty_buffers(h);
     }
@@ -754,7 +774,7 @@ static int set_particle_bytes(mpm_handle* h, uint8_t*& dst, const uint8_t* src, 
         dst = nullptr;
         return MPM_OK;
     }
-    if(!dst) MPM_CUDA(h, cudaMalloc(&dst, (size_t)(n ? n : 1)));
+    if(!dst) MPM_ALLOC(h, &dst, (size_t)(n ? n : 1));
     MPM_CUDA(h, cudaMemcpy(dst, src, (size_t)n, cudaMemcpyHostToDevice));
     return MPM_OK;
 }
@@ -864,11 +884,14 @@ int mpm_set_plasticity(mpm_handle* h, const mpm_plasticity_desc* p)
         if(!(phi0 > 0 && phi0 < 90)) return set_error(h, MPM_ERR_ARG, "friction angle a0 - a4 outside (0, 90) degrees");
     }
     release_graph(h);
-    const int was = h->plastic.kind;
+    const mpm_plasticity_desc was = h->plastic;
     h->plastic = *p;
-    if(p->kind && p->kind != was && h->have_particles) {
+    if(p->kind && p->kind != was.kind && h->have_particles) {
         int rc = fast(h) ? fast_plastic_init(h) : plain_plastic_init(h);
-        if(rc) return rc;
+        if(rc) {
+            h->plastic = was;
+            return rc;
+        }
         MPM_CUDA(h, cudaStreamSynchronize(h->stream));
     }
     return MPM_OK;
@@ -925,7 +948,7 @@ int mpm_compute_dt(mpm_handle* h, double cfl, double max_dt, double* dt)
     if(h->have_particles) {
         if(!h->speed_host) MPM_CUDA(h, cudaMallocHost(&h->speed_host, sizeof(double)));
         if(!h->speed_state) {
-            MPM_CUDA(h, cudaMalloc(&h->speed_state, 2 * sizeof(unsigned long long)));
+            MPM_ALLOC(h, &h->speed_state, 2 * sizeof(unsigned long long));
             MPM_CUDA(h, cudaMemsetAsync(h->speed_state, 0, 2 * sizeof(unsigned long long), h->stream));
         }
         *h->speed_host = 0;

@@ -2123,13 +2123,13 @@ int fast_setup_scenes(mpm_handle* h, const mpm_scene_desc* descs, int count, con
         for(int64_t b = sc[s].block_base; b < b1; b++) bs[b] = (uint16_t)s;
         for(int64_t b = sc[s].nb_base; b < n1; b++) ns[b] = (uint16_t)s;
     }
-    MPM_CUDA(h, cudaMalloc(&f.scenes, count * sizeof(SceneDev)));
+    MPM_ALLOC(h, &f.scenes, count * sizeof(SceneDev));
     MPM_CUDA(h, cudaMemcpy(f.scenes, sc.data(), count * sizeof(SceneDev), cudaMemcpyHostToDevice));
-    MPM_CUDA(h, cudaMalloc(&f.pbase, (count + 1) * sizeof(int64_t)));
+    MPM_ALLOC(h, &f.pbase, (count + 1) * sizeof(int64_t));
     MPM_CUDA(h, cudaMemcpy(f.pbase, pb.data(), (count + 1) * sizeof(int64_t), cudaMemcpyHostToDevice));
-    MPM_CUDA(h, cudaMalloc(&f.block_scene, blocks * sizeof(uint16_t)));
+    MPM_ALLOC(h, &f.block_scene, blocks * sizeof(uint16_t));
     MPM_CUDA(h, cudaMemcpy(f.block_scene, bs.data(), blocks * sizeof(uint16_t), cudaMemcpyHostToDevice));
-    MPM_CUDA(h, cudaMalloc(&f.nb_scene, nblocks * sizeof(uint16_t)));
+    MPM_ALLOC(h, &f.nb_scene, nblocks * sizeof(uint16_t));
     MPM_CUDA(h, cudaMemcpy(f.nb_scene, ns.data(), nblocks * sizeof(uint16_t), cudaMemcpyHostToDevice));
     f.objs_h.assign(nobjs > 0 ? nobjs : 1, DevObject{});
     for(int i = 0; i < nobjs; i++) {
@@ -2139,36 +2139,36 @@ int fast_setup_scenes(mpm_handle* h, const mpm_scene_desc* descs, int count, con
         o.friction = objs[i].friction;
         for(int k = 0; k < 3; k++) { o.a[k] = objs[i].a[k]; o.b[k] = objs[i].b[k]; }
     }
-    MPM_CUDA(h, cudaMalloc(&f.objs, f.objs_h.size() * sizeof(DevObject)));
+    MPM_ALLOC(h, &f.objs, f.objs_h.size() * sizeof(DevObject));
     MPM_CUDA(h, cudaMemcpy(f.objs, f.objs_h.data(), f.objs_h.size() * sizeof(DevObject), cudaMemcpyHostToDevice));
     f.grid_nodes = nodes;
     f.grid_node_blocks = nblocks;
     f.grid_dirty = false;
-    MPM_CUDA(h, cudaMalloc(&f.acc, nodes * sizeof(float4)));
-    MPM_CUDA(h, cudaMalloc(&f.vel, nodes * 2 * sizeof(float4)));
+    MPM_ALLOC(h, &f.acc, nodes * sizeof(float4));
+    MPM_ALLOC(h, &f.vel, nodes * 2 * sizeof(float4));
     MPM_CUDA(h, cudaMemset(f.acc, 0, nodes * sizeof(float4)));
     MPM_CUDA(h, cudaMemset(f.vel, 0, nodes * 2 * sizeof(float4)));
     for(int k = 0; k < 2; k++) {
-        MPM_CUDA(h, cudaMalloc(&f.bstart[k], blocks * sizeof(uint32_t)));
-        MPM_CUDA(h, cudaMalloc(&f.bend[k], blocks * sizeof(uint32_t)));
-        MPM_CUDA(h, cudaMalloc(&f.active[k], blocks * sizeof(uint4)));
+        MPM_ALLOC(h, &f.bstart[k], blocks * sizeof(uint32_t));
+        MPM_ALLOC(h, &f.bend[k], blocks * sizeof(uint32_t));
+        MPM_ALLOC(h, &f.active[k], blocks * sizeof(uint4));
     }
-    MPM_CUDA(h, cudaMalloc(&f.nb_flag, nblocks * sizeof(uint32_t)));
-    MPM_CUDA(h, cudaMalloc(&f.nb_list, nblocks * sizeof(uint32_t)));
+    MPM_ALLOC(h, &f.nb_flag, nblocks * sizeof(uint32_t));
+    MPM_ALLOC(h, &f.nb_list, nblocks * sizeof(uint32_t));
     MPM_CUDA(h, cudaMemset(f.nb_flag, 0, nblocks * sizeof(uint32_t)));
-    MPM_CUDA(h, cudaMalloc(&f.nb_differs, 2 * nblocks));
+    MPM_ALLOC(h, &f.nb_differs, 2 * nblocks);
     MPM_CUDA(h, cudaMemset(f.nb_differs, 0, 2 * nblocks));
-    MPM_CUDA(h, cudaMalloc(&f.counters, 2 * CNT_COUNT * sizeof(uint32_t)));
+    MPM_ALLOC(h, &f.counters, 2 * CNT_COUNT * sizeof(uint32_t));
     MPM_CUDA(h, cudaMemset(f.counters, 0, 2 * CNT_COUNT * sizeof(uint32_t)));
     // routing between substeps: direction counts and offsets, far arrivals,
     // the block scan's epoch word and look-back status words (two chains)
-    MPM_CUDA(h, cudaMalloc(&f.dcount, (size_t)ROW * blocks * sizeof(uint32_t)));
-    MPM_CUDA(h, cudaMalloc(&f.doff, (size_t)ROW * blocks * sizeof(uint32_t)));
-    MPM_CUDA(h, cudaMalloc(&f.bcount, blocks * sizeof(unsigned long long)));
+    MPM_ALLOC(h, &f.dcount, (size_t)ROW * blocks * sizeof(uint32_t));
+    MPM_ALLOC(h, &f.doff, (size_t)ROW * blocks * sizeof(uint32_t));
+    MPM_ALLOC(h, &f.bcount, blocks * sizeof(unsigned long long));
     MPM_CUDA(h, cudaMemset(f.bcount, 0, blocks * sizeof(unsigned long long)));
     MPM_CUDA(h, cudaMemset(f.dcount, 0, (size_t)ROW * blocks * sizeof(uint32_t)));
     const int64_t tiles = (blocks + SCAN_TILE - 1) / SCAN_TILE;
-    MPM_CUDA(h, cudaMalloc(&f.scan, (8 + 4 * STATUS_STRIDE * tiles) * sizeof(uint32_t)));
+    MPM_ALLOC(h, &f.scan, (8 + 4 * STATUS_STRIDE * tiles) * sizeof(uint32_t));
     MPM_CUDA(h, cudaMemset(f.scan, 0, (8 + 4 * STATUS_STRIDE * tiles) * sizeof(uint32_t)));
     f.order_ready = false;
     f.sorted_now = false;
@@ -2205,7 +2205,7 @@ static int encode_tile_maps(mpm_handle* h)
     }
     cudaFree(f.tmaps);
     f.tmaps = nullptr;
-    MPM_CUDA(h, cudaMalloc(&f.tmaps, maps.size() * sizeof(CUtensorMap)));
+    MPM_ALLOC(h, &f.tmaps, maps.size() * sizeof(CUtensorMap));
     MPM_CUDA(h, cudaMemcpy(f.tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     return MPM_OK;
 }
@@ -2234,7 +2234,24 @@ int fast_single_scene(mpm_handle* h)
     return rc;
 }
 
-int fast_alloc(mpm_handle* h, int64_t n)
+static void free_particle_buffers(FastState& f)
+{
+    for(int b = 0; b < 2; b++) {
+        cudaFree(f.soa[b]); cudaFree(f.attr[b]); cudaFree(f.pid[b]); cudaFree(f.plas[b]);
+        f.soa[b] = nullptr; f.attr[b] = nullptr; f.pid[b] = nullptr; f.plas[b] = nullptr;
+        cudaFree(f.chunks[b]); f.chunks[b] = nullptr;
+        cudaFree(f.dirs[b]); f.dirs[b] = nullptr;
+    }
+    uint32_t** ps[] = {&f.keys[0], &f.keys[1], &f.sorted_keys, &f.perm, &f.sort_keys_alt, &f.sort_vals_alt,
+                       &f.sort_scratch};
+    for(uint32_t** p: ps) { cudaFree(*p); *p = nullptr; }
+    cudaFree(f.vkick);
+    f.vkick = nullptr;
+    cudaFree(f.pmodel); cudaFree(f.pmask);   // per caller index: a new count drops them
+    f.pmodel = nullptr; f.pmask = nullptr;
+}
+
+static int fast_alloc_buffers(mpm_handle* h, int64_t n)
 {
     FastState& f = h->fast;
     if(h->sp.dim != 3) return set_error(h, MPM_ERR_ARG, "the fast path is 3D; use MPM_PATH_PLAIN for 2D");
@@ -2250,40 +2267,26 @@ int fast_alloc(mpm_handle* h, int64_t n)
     }
     if(f.n != n || !f.soa[0]) {
         f.generation++;
-        for(int b = 0; b < 2; b++) {
-            cudaFree(f.soa[b]); cudaFree(f.attr[b]); cudaFree(f.pid[b]); cudaFree(f.plas[b]);
-            f.soa[b] = nullptr; f.attr[b] = nullptr; f.pid[b] = nullptr; f.plas[b] = nullptr;
-        }
-        uint32_t** ps[] = {&f.keys[0], &f.keys[1], &f.sorted_keys, &f.perm, &f.sort_keys_alt, &f.sort_vals_alt,
-                           &f.sort_scratch};
-        for(uint32_t** p: ps) { cudaFree(*p); *p = nullptr; }
-        for(int k = 0; k < 2; k++) {
-            cudaFree(f.chunks[k]); f.chunks[k] = nullptr;
-            cudaFree(f.dirs[k]); f.dirs[k] = nullptr;
-        }
-        cudaFree(f.vkick);
-        f.vkick = nullptr;
-        cudaFree(f.pmodel); cudaFree(f.pmask);   // per caller index: a new count drops them
-        f.pmodel = nullptr; f.pmask = nullptr;
+        free_particle_buffers(f);
         int64_t np = ((n ? n : 1) + 31) / 32 * 32;
         f.npad = np;
         for(int b = 0; b < 2; b++) {
-            MPM_CUDA(h, cudaMalloc(&f.soa[b], NCOMP * np * sizeof(float)));
-            MPM_CUDA(h, cudaMalloc(&f.attr[b], np * sizeof(float4)));
-            MPM_CUDA(h, cudaMalloc(&f.pid[b], np * sizeof(int)));
+            MPM_ALLOC(h, &f.soa[b], NCOMP * np * sizeof(float));
+            MPM_ALLOC(h, &f.attr[b], np * sizeof(float4));
+            MPM_ALLOC(h, &f.pid[b], np * sizeof(int));
         }
         for(int k = 0; k < 2; k++) {
-            MPM_CUDA(h, cudaMalloc(&f.keys[k], np * sizeof(uint32_t)));
-            MPM_CUDA(h, cudaMalloc(&f.dirs[k], np * sizeof(uint8_t)));
+            MPM_ALLOC(h, &f.keys[k], np * sizeof(uint32_t));
+            MPM_ALLOC(h, &f.dirs[k], np * sizeof(uint8_t));
         }
         // work items: a block's particles in parts of at least 64
         f.chunk_cap = np / 64 + std::min<int64_t>(np, f.total_blocks) + 1;
-        for(int k = 0; k < 2; k++) MPM_CUDA(h, cudaMalloc(&f.chunks[k], 2 * f.chunk_cap * sizeof(uint4)));
-        MPM_CUDA(h, cudaMalloc(&f.sorted_keys, np * sizeof(uint32_t)));
-        MPM_CUDA(h, cudaMalloc(&f.perm, np * sizeof(uint32_t)));
-        MPM_CUDA(h, cudaMalloc(&f.sort_keys_alt, np * sizeof(uint32_t)));
-        MPM_CUDA(h, cudaMalloc(&f.sort_vals_alt, np * sizeof(uint32_t)));
-        MPM_CUDA(h, cudaMalloc(&f.sort_scratch, mpm_sort::scratch_words(np) * sizeof(uint32_t)));
+        for(int k = 0; k < 2; k++) MPM_ALLOC(h, &f.chunks[k], 2 * f.chunk_cap * sizeof(uint4));
+        MPM_ALLOC(h, &f.sorted_keys, np * sizeof(uint32_t));
+        MPM_ALLOC(h, &f.perm, np * sizeof(uint32_t));
+        MPM_ALLOC(h, &f.sort_keys_alt, np * sizeof(uint32_t));
+        MPM_ALLOC(h, &f.sort_vals_alt, np * sizeof(uint32_t));
+        MPM_ALLOC(h, &f.sort_scratch, mpm_sort::scratch_words(np) * sizeof(uint32_t));
         MPM_CUDA(h, cudaMemsetAsync(f.sort_scratch, 0, mpm_sort::scratch_words(np) * sizeof(uint32_t), h->stream));
         MPM_CUDA(h, mpm_sort::prepare());
         f.n = n;
@@ -2293,13 +2296,28 @@ int fast_alloc(mpm_handle* h, int64_t n)
     return fast_penalty_buffers(h);
 }
 
+// All buffers of n particles, or none of them: a batch keeps its scenes, a single-scene
+// handle builds its own anew.
+int fast_alloc(mpm_handle* h, int64_t n)
+{
+    FastState& f = h->fast;
+    const int rc = fast_alloc_buffers(h, n);
+    if(!rc || rc == MPM_ERR_ARG) return rc;
+    if(f.batch) {
+        free_particle_buffers(f);
+        f.n = f.npad = 0;
+        f.keys_ready = f.order_ready = f.sorted_now = false;
+    } else fast_free(h);
+    return rc;
+}
+
 // The side buffer of the penalty impulse, once there are penalty objects and particles.
 int fast_penalty_buffers(mpm_handle* h)
 {
     FastState& f = h->fast;
     if(h->sp.npen && f.npad && !f.vkick) {
         f.generation++;   // make_args changes: graphs captured without the buffer are stale
-        MPM_CUDA(h, cudaMalloc(&f.vkick, 3 * f.npad * sizeof(float)));
+        MPM_ALLOC(h, &f.vkick, 3 * f.npad * sizeof(float));
     }
     return MPM_OK;
 }
@@ -2307,19 +2325,12 @@ int fast_penalty_buffers(mpm_handle* h)
 void fast_free(mpm_handle* h)
 {
     FastState& f = h->fast;
-    for(int b = 0; b < 2; b++) {
-        cudaFree(f.soa[b]); cudaFree(f.attr[b]); cudaFree(f.pid[b]); cudaFree(f.plas[b]);
-        f.soa[b] = nullptr; f.attr[b] = nullptr; f.pid[b] = nullptr; f.plas[b] = nullptr;
-    }
-    void** ps[] = {(void**)&f.keys[0], (void**)&f.keys[1], (void**)&f.dirs[0], (void**)&f.dirs[1],
-                   (void**)&f.sorted_keys, (void**)&f.perm,
-                   (void**)&f.sort_keys_alt, (void**)&f.sort_vals_alt, (void**)&f.sort_scratch, (void**)&f.bstart[0],
-                   (void**)&f.bend[0], (void**)&f.active[0], (void**)&f.chunks[0], (void**)&f.bstart[1],
-                   (void**)&f.bend[1], (void**)&f.active[1], (void**)&f.chunks[1], (void**)&f.nb_flag,
-                   (void**)&f.nb_list, (void**)&f.counters, (void**)&f.acc, (void**)&f.vel, (void**)&f.scenes,
-                   (void**)&f.block_scene, (void**)&f.nb_scene, (void**)&f.pbase, (void**)&f.objs, (void**)&f.vkick,
-                   (void**)&f.pmodel, (void**)&f.pmask, (void**)&f.dcount, (void**)&f.doff,
-                   (void**)&f.scan, (void**)&f.tmaps, (void**)&f.bcount, (void**)&f.nb_differs};
+    free_particle_buffers(f);
+    void** ps[] = {(void**)&f.bstart[0], (void**)&f.bend[0], (void**)&f.active[0], (void**)&f.bstart[1], (void**)&f.bend[1],
+                   (void**)&f.active[1], (void**)&f.nb_flag, (void**)&f.nb_list, (void**)&f.counters, (void**)&f.acc,
+                   (void**)&f.vel, (void**)&f.scenes, (void**)&f.block_scene, (void**)&f.nb_scene, (void**)&f.pbase,
+                   (void**)&f.objs, (void**)&f.dcount, (void**)&f.doff, (void**)&f.scan, (void**)&f.tmaps,
+                   (void**)&f.bcount, (void**)&f.nb_differs};
     for(void** p: ps) { cudaFree(*p); *p = nullptr; }
     f.order_ready = false;
     f.sorted_now = false;
@@ -2341,7 +2352,7 @@ static int fast_staging(mpm_handle* h, size_t bytes, uint8_t** out)
         cudaFree(f.staging);
         f.staging = nullptr;
         f.staging_bytes = 0;
-        MPM_CUDA(h, cudaMalloc(&f.staging, bytes));
+        MPM_ALLOC(h, &f.staging, bytes);
         f.staging_bytes = bytes;
     }
     *out = (uint8_t*)f.staging;
@@ -2412,8 +2423,15 @@ int fast_plastic_init(mpm_handle* h)
 {
     FastState& f = h->fast;
     if(!f.soa[0]) return MPM_OK;
-    if(!f.plas[0])
-        for(int b = 0; b < 2; b++) MPM_CUDA(h, cudaMalloc(&f.plas[b], NPLAS * f.npad * sizeof(float)));
+    if(!f.plas[0]) {
+        MPM_ALLOC(h, &f.plas[0], NPLAS * f.npad * sizeof(float));
+        const int rc = device_alloc(h, (void**)&f.plas[1], NPLAS * f.npad * sizeof(float));
+        if(rc) {
+            cudaFree(f.plas[0]);
+            f.plas[0] = nullptr;
+            return rc;
+        }
+    }
     if(!f.n) return MPM_OK;
     const mpm_plasticity_desc& pl = h->plastic;
     if(pl.kind == MPM_PLASTICITY_DRUCKER_PRAGER) {
@@ -2845,7 +2863,7 @@ int fast_autotune(mpm_handle* h, double dt, int substeps, int flags, char* repor
         int l2 = 0;
         cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device);
         scrub_bytes = 2 * (size_t)(l2 > 0 ? l2 : (64 << 20));
-        MPM_CUDA(h, cudaMalloc(&scrub, scrub_bytes));
+        MPM_ALLOC(h, &scrub, scrub_bytes);
     }
     // keep the current state: both buffers + keys
     const int64_t np = f.npad;
@@ -2853,10 +2871,10 @@ int fast_autotune(mpm_handle* h, double dt, int substeps, int flags, char* repor
     float4* save_attr = nullptr;
     int* save_pid = nullptr;
     uint32_t* save_keys = nullptr;
-    MPM_CUDA(h, cudaMalloc(&save_soa, NCOMP * np * sizeof(float)));
-    MPM_CUDA(h, cudaMalloc(&save_attr, np * sizeof(float4)));
-    MPM_CUDA(h, cudaMalloc(&save_pid, np * sizeof(int)));
-    MPM_CUDA(h, cudaMalloc(&save_keys, np * sizeof(uint32_t)));
+    MPM_ALLOC(h, &save_soa, NCOMP * np * sizeof(float));
+    MPM_ALLOC(h, &save_attr, np * sizeof(float4));
+    MPM_ALLOC(h, &save_pid, np * sizeof(int));
+    MPM_ALLOC(h, &save_keys, np * sizeof(uint32_t));
     const int cur0 = f.cur;
     MPM_CUDA(h, cudaMemcpyAsync(save_soa, f.soa[cur0], NCOMP * np * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
     MPM_CUDA(h, cudaMemcpyAsync(save_attr, f.attr[cur0], np * sizeof(float4), cudaMemcpyDeviceToDevice, h->stream));
@@ -2865,7 +2883,7 @@ int fast_autotune(mpm_handle* h, double dt, int substeps, int flags, char* repor
     float* save_plas = nullptr;
     const bool plastic = h->plastic.kind && f.plas[0];
     if(plastic) {
-        MPM_CUDA(h, cudaMalloc(&save_plas, NPLAS * np * sizeof(float)));
+        MPM_ALLOC(h, &save_plas, NPLAS * np * sizeof(float));
         MPM_CUDA(h, cudaMemcpyAsync(save_plas, f.plas[cur0], NPLAS * np * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
     }
     cudaEvent_t e0[64], e1[64];

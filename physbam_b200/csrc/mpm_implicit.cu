@@ -1035,7 +1035,7 @@ template<class T, int d> struct Solver {
     }
 };
 
-template<class T> int ensure_state(mpm_handle* h)
+template<class T> int alloc_state(mpm_handle* h)
 {
     PlainState& ps = h->plain;
     const int d = h->sp.dim;
@@ -1048,26 +1048,34 @@ template<class T> int ensure_state(mpm_handle* h)
     ImplicitState& t = *h->imp;
     t.gn = ps.gn; t.n = ps.n; t.nobj = h->sp.nobj; t.d = d; t.esz = e;
     const int64_t n = t.n ? t.n : 1;
-    MPM_CUDA(h, cudaMalloc(&t.vec, (size_t)V_COUNT * t.gn * d * e));
-    MPM_CUDA(h, cudaMalloc(&t.part, (size_t)n * (d * d * 3 + d * 2 + 15) * e));
-    MPM_CUDA(h, cudaMalloc(&t.pe, (size_t)n * sizeof(double)));
-    MPM_CUDA(h, cudaMalloc(&t.cmask, (size_t)t.gn));
-    MPM_CUDA(h, cudaMalloc(&t.stuck, (size_t)t.gn));
+    MPM_ALLOC(h, &t.vec, (size_t)V_COUNT * t.gn * d * e);
+    MPM_ALLOC(h, &t.part, (size_t)n * (d * d * 3 + d * 2 + 15) * e);
+    MPM_ALLOC(h, &t.pe, (size_t)n * sizeof(double));
+    MPM_ALLOC(h, &t.cmask, (size_t)t.gn);
+    MPM_ALLOC(h, &t.stuck, (size_t)t.gn);
     MPM_CUDA(h, cudaMemset(t.cmask, 0, (size_t)t.gn));
     MPM_CUDA(h, cudaMemset(t.stuck, 0, (size_t)t.gn));
-    if(t.nobj) MPM_CUDA(h, cudaMalloc(&t.cdat, (size_t)t.gn * t.nobj * (2 + 3 * d) * e));
-    MPM_CUDA(h, cudaMalloc(&t.partial, 3 * kRedBlocks * sizeof(double)));
-    MPM_CUDA(h, cudaMalloc(&t.done, 3 * sizeof(unsigned)));
+    if(t.nobj) MPM_ALLOC(h, &t.cdat, (size_t)t.gn * t.nobj * (2 + 3 * d) * e);
+    MPM_ALLOC(h, &t.partial, 3 * kRedBlocks * sizeof(double));
+    MPM_ALLOC(h, &t.done, 3 * sizeof(unsigned));
     MPM_CUDA(h, cudaMemset(t.done, 0, 3 * sizeof(unsigned)));
-    MPM_CUDA(h, cudaMalloc(&t.dout, 3 * sizeof(double)));
+    MPM_ALLOC(h, &t.dout, 3 * sizeof(double));
     MPM_CUDA(h, cudaMallocHost(&t.hout, 3 * sizeof(double)));
     uint32_t** sb[] = {&t.keys, &t.sorted, &t.perm, &t.alt_k, &t.alt_v};
-    for(uint32_t** p: sb) MPM_CUDA(h, cudaMalloc(p, (size_t)n * sizeof(uint32_t)));
-    MPM_CUDA(h, cudaMalloc(&t.scratch, (size_t)sort_scratch_words(n) * sizeof(uint32_t)));
+    for(uint32_t** p: sb) MPM_ALLOC(h, p, (size_t)n * sizeof(uint32_t));
+    MPM_ALLOC(h, &t.scratch, (size_t)sort_scratch_words(n) * sizeof(uint32_t));
     MPM_CUDA(h, cudaMemset(t.scratch, 0, (size_t)sort_scratch_words(n) * sizeof(uint32_t)));
     t.key_bits = 1;
     while((int64_t)((1ull << t.key_bits) - 1) < t.gn) t.key_bits++;
     return MPM_OK;
+}
+
+// The whole state, or none of it.
+template<class T> int ensure_state(mpm_handle* h)
+{
+    const int rc = alloc_state<T>(h);
+    if(rc) implicit_free(h);
+    return rc;
 }
 
 template<class T> int implicit_t(mpm_handle* h, double dt)

@@ -183,6 +183,7 @@ struct mpm_handle {
     mpm::DevObjectF* pen_f = nullptr;   // penalty objects rounded to float (fast path), MPM_MAX_OBJECTS
     int64_t n = 0;
     bool have_particles = false;
+    int fail_alloc = 0;                 // > 0: the allocation that fails, counted from here (mpm_debug_fail_allocation)
     unsigned* d_flags = nullptr;
     // Compute_Dt's speed bound: reduction state (2 words), and the result in pinned memory
     unsigned long long* speed_state = nullptr;
@@ -303,11 +304,19 @@ void diff_release_graphs(mpm_handle* h);
 
 // helpers
 int set_error(mpm_handle* h, int code, const std::string& msg);
+// cudaMalloc for the handle.  A caller that fills several pointers frees all of them when
+// one fails (what it keeps, the next call takes for complete).
+int device_alloc(mpm_handle* h, void** ptr, size_t bytes);
 int check_cuda(mpm_handle* h, cudaError_t e, const char* what);
 #define MPM_CUDA(h, call)                                   \
     do {                                                    \
         cudaError_t e__ = (call);                           \
         if(e__ != cudaSuccess) return check_cuda(h, e__, #call); \
+    } while(0)
+#define MPM_ALLOC(h, ptr, bytes)                            \
+    do {                                                    \
+        int r__ = device_alloc(h, (void**)(ptr), bytes);    \
+        if(r__) return r__;                                 \
     } while(0)
 #define MPM_LAUNCHED(h, what)                               \
     do {                                                    \

@@ -945,7 +945,7 @@ template<class Tin, class Tout> __global__ void k_convert(const Tin* in, Tout* o
 
 }  // namespace
 
-int plain_alloc(mpm_handle* h, int64_t n)
+static int plain_alloc_buffers(mpm_handle* h, int64_t n)
 {
     PlainState& s = h->plain;
     const int d = h->sp.dim;
@@ -956,8 +956,8 @@ int plain_alloc(mpm_handle* h, int64_t n)
     if(s.gn != gn) {
         void** g[] = {&s.gm, &s.gmv, &s.gv0, &s.gf, &s.gv, &s.gvf};
         for(void** p: g) { cudaFree(*p); *p = nullptr; }
-        MPM_CUDA(h, cudaMalloc(&s.gm, gn * e));
-        for(int i = 1; i < 6; i++) MPM_CUDA(h, cudaMalloc(g[i], gn * d * e));
+        MPM_ALLOC(h, &s.gm, gn * e);
+        for(int i = 1; i < 6; i++) MPM_ALLOC(h, g[i], gn * d * e);
         s.gn = gn;
         for(void** p: g) MPM_CUDA(h, cudaMemsetAsync(*p, 0, (p == &s.gm ? gn : gn * d) * e, h->stream));
         cudaFree(s.tile_flag); s.tile_flag = nullptr;
@@ -966,9 +966,9 @@ int plain_alloc(mpm_handle* h, int64_t n)
         s.grid_listed = false;
         if(gn >= kListedGrid) {
             const int64_t nt = (gn + kTileNodes - 1) / kTileNodes, span = (nt + kTileSpan - 1) / kTileSpan * kTileSpan;
-            MPM_CUDA(h, cudaMalloc(&s.tile_flag, span));
-            MPM_CUDA(h, cudaMalloc(&s.tiles, nt * sizeof(uint32_t)));
-            MPM_CUDA(h, cudaMalloc(&s.tile_count, sizeof(uint32_t)));
+            MPM_ALLOC(h, &s.tile_flag, span);
+            MPM_ALLOC(h, &s.tiles, nt * sizeof(uint32_t));
+            MPM_ALLOC(h, &s.tile_count, sizeof(uint32_t));
             // an empty list: node passes may come before the first P2G (the phase entry points)
             MPM_CUDA(h, cudaMemsetAsync(s.tile_flag, 0, span, h->stream));
             MPM_CUDA(h, cudaMemsetAsync(s.tile_count, 0, sizeof(uint32_t), h->stream));
@@ -983,19 +983,31 @@ int plain_alloc(mpm_handle* h, int64_t n)
         cudaFree(s.pmodel); s.pmodel = nullptr;
         cudaFree(s.pmask); s.pmask = nullptr;
         int64_t m = n ? n : 1;
-        MPM_CUDA(h, cudaMalloc(&s.X, m * d * e));
-        MPM_CUDA(h, cudaMalloc(&s.V, m * d * e));
-        MPM_CUDA(h, cudaMalloc(&s.F, m * d * d * e));
-        MPM_CUDA(h, cudaMalloc(&s.B, m * d * d * e));
-        MPM_CUDA(h, cudaMalloc(&s.pft, m * d * d * e));
-        MPM_CUDA(h, cudaMalloc(&s.mass, m * e));
-        MPM_CUDA(h, cudaMalloc(&s.vol, m * e));
-        MPM_CUDA(h, cudaMalloc(&s.mu, m * e));
-        MPM_CUDA(h, cudaMalloc(&s.lam, m * e));
-        MPM_CUDA(h, cudaMalloc(&s.valid, m));
+        MPM_ALLOC(h, &s.X, m * d * e);
+        MPM_ALLOC(h, &s.V, m * d * e);
+        MPM_ALLOC(h, &s.F, m * d * d * e);
+        MPM_ALLOC(h, &s.B, m * d * d * e);
+        MPM_ALLOC(h, &s.pft, m * d * d * e);
+        MPM_ALLOC(h, &s.mass, m * e);
+        MPM_ALLOC(h, &s.vol, m * e);
+        MPM_ALLOC(h, &s.mu, m * e);
+        MPM_ALLOC(h, &s.lam, m * e);
+        MPM_ALLOC(h, &s.valid, m);
         s.n = n;
     }
     return MPM_OK;
+}
+
+// All buffers, or none.
+int plain_alloc(mpm_handle* h, int64_t n)
+{
+    const int rc = plain_alloc_buffers(h, n);
+    if(rc) {
+        const uint64_t generation = h->plain.generation;
+        plain_free(h);
+        h->plain.generation = generation;
+    }
+    return rc;
 }
 
 // Before a substep, never inside a captured one: the whole grid to zero where the
@@ -1126,9 +1138,14 @@ int plain_plastic_init(mpm_handle* h)
     const int64_t m = s.n ? s.n : 1;
     if(!s.Fp) {
         s.generation++;
-        MPM_CUDA(h, cudaMalloc(&s.Fp, m * d * d * e));
-        void** pa[] = {&s.mu0, &s.lam0, &s.pdef, &s.rhoF, &s.sigY, &s.vc};
-        for(void** p: pa) MPM_CUDA(h, cudaMalloc(p, m * e));
+        void** pa[] = {&s.Fp, &s.mu0, &s.lam0, &s.pdef, &s.rhoF, &s.sigY, &s.vc};
+        int rc = MPM_OK;
+        for(void** p: pa)
+            if(!rc) rc = device_alloc(h, p, (p == &s.Fp ? m * d * d : m) * e);
+        if(rc) {
+            for(void** p: pa) { cudaFree(*p); *p = nullptr; }
+            return rc;
+        }
     }
     if(!s.n) return MPM_OK;
     const int b = gblocks(h, s.n, 256);

@@ -10,6 +10,9 @@ the same process keeps sorting and simulating correctly.
 * The FP64 SVD (the reference's unbounded implicit-shift QR,
   Core/Matrices/MATRIX_3X3.cpp:202-236) gets a one-sweep bound: the substep
   reports MPM_ERR_NOT_CONVERGED.
+* Each of the library's device allocations reports, once, that memory is short
+  (a failure made on the host): the call returns MPM_ERR_NOMEM and leaves nothing
+  half-built behind, so the same call works when it is made again.
 The reference's counterparts are assertion failures that throw
 (Core/Log/DEBUG_UTILITIES.cpp:95-103); here they are status codes.
 """
@@ -20,7 +23,7 @@ from physbam_b200 import scenes as S
 
 pytestmark = pytest.mark.gpu
 
-TIMEOUT, NOT_CONVERGED = 5, 8
+TIMEOUT, NOMEM, STATE, NOT_CONVERGED = 5, 6, 7, 8
 
 
 def D():
@@ -86,3 +89,100 @@ def test_svd_non_convergence_is_reported(cuda_device, path):
     drv.synchronize()
     assert drv.count_valid() == scene.n
     drv.close()
+
+
+def refuse_each(make, call, after=lambda drv: None):
+    """`call(drv)` on a new handle per allocation it makes, that allocation refused: it returns
+    MPM_ERR_NOMEM, and the same call made again works.  Its results, the undisturbed call's last."""
+    out = []
+    for k in range(1, 100):
+        drv = make()
+        drv._check(drv.L.mpm_debug_fail_allocation(drv.h, k), "mpm_debug_fail_allocation")
+        try:
+            try:
+                out.append(call(drv))
+                return out
+            except D().MPMError as e:
+                assert e.code == NOMEM, e
+            after(drv)
+            out.append(call(drv))
+        finally:
+            drv.close()
+    raise AssertionError("never succeeded")
+
+
+@pytest.mark.parametrize("G", [16, 40])                # dense node passes, listed tiles
+@pytest.mark.parametrize("budget", [-1, 0])            # the whole tape, segments
+@pytest.mark.parametrize("phase", ["forward", "backward"])
+def test_rollout_short_of_memory(cuda_device, G, budget, phase):
+    import torch
+    scene = S.small_3d(G=G, ppc=1, with_walls=False)
+    one = [torch.ones((scene.n, k), dtype=torch.float64, device="cuda") for k in (3, 3, 9, 9)]
+
+    def make():
+        drv = D().MPM_DRIVER(scene, precision=D().FP64, path=D().PATH_PLAIN)
+        drv.set_diff_tape_budget(budget)
+        drv.set_scene_particles(scene)
+        if phase == "backward":
+            drv.diff_forward(7, 3)
+        return drv
+
+    def call(drv):
+        if phase == "forward":
+            drv.diff_forward(7, 3)
+            return [drv.get_particles()["X"]]
+        return [g.cpu().numpy() for g in drv.diff_backward(*one)]
+
+    out = refuse_each(make, call)
+    slots = 6 if G == 16 else 8
+    assert len(out) - 1 == (4 if phase == "forward" else 7) + (slots if (phase == "forward") == (budget < 0) else 0)
+    for got in out[:-1]:
+        for a, b in zip(got, out[-1]):
+            assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max()
+
+
+def test_implicit_short_of_memory(cuda_device):
+    scene = S.small_3d_implicit(nsteps=2)
+
+    def make():
+        drv = D().MPM_DRIVER(scene, precision=D().FP64, path=D().PATH_PLAIN)
+        drv.set_scene_particles(scene)
+        return drv
+
+    def call(drv):
+        drv.Advance_One_Time_Step()
+        return drv.get_particles()["X"]
+
+    out = refuse_each(make, call)
+    assert len(out) >= 14
+    for X in out[:-1]:
+        assert np.abs(X - out[-1]).max() < 2e-9        # Newton to its own tolerance
+
+
+@pytest.mark.parametrize("path,scene", [("plain", S.small_3d(G=40, ppc=1)), ("plain", S.small_snow_3d()),
+                                        ("fast", S.small_3d()), ("fast", S.small_snow_3d())])
+def test_upload_short_of_memory(cuda_device, path, scene):
+    """More particles than the handle held: refused, it holds none and says so."""
+    precision, path = (D().FP64, D().PATH_PLAIN) if path == "plain" else (D().FP32, D().PATH_FAST)
+
+    def make():
+        drv = D().MPM_DRIVER(scene, precision=precision, path=path)
+        drv.set_scene_particles(scene.subset(np.arange(100)))
+        drv.advance(2)
+        return drv
+
+    def call(drv):
+        drv.set_scene_particles(scene)
+        drv.advance(3)
+        drv.synchronize()
+        return drv.get_particles()["X"]
+
+    def refused(drv):
+        with pytest.raises(D().MPMError) as e:
+            drv.advance(1)
+        assert e.value.code == STATE
+
+    out = refuse_each(make, call, refused)
+    assert len(out) >= 10
+    for X in out[:-1]:
+        assert np.abs(X - out[-1]).max() < (1e-12 if precision == D().FP64 else 2e-6)
