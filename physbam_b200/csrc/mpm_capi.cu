@@ -267,8 +267,10 @@ static int run_substep(mpm_handle* h, double dt, double time)
     }
     MPM_CUDA(h, cudaGraphLaunch(ge, h->stream));
     h->last_dt = dt;
-    if(fast(h)) h->fast.cur = 1 - par;
-    else h->plain.scattered = false;
+    if(fast(h)) {
+        h->fast.grid_set = par;        // as fast_forces sets it where it is enqueued
+        h->fast.cur = 1 - par;
+    } else h->plain.scattered = false;
     return MPM_OK;
 }
 
