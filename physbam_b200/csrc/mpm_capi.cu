@@ -250,6 +250,8 @@ static int run_substep(mpm_handle* h, double dt, double time)
     // the fast path's full sort after new particles runs eagerly, never in a graph
     int prc = fast(h) ? fast_prepare(h) : plain_prepare(h);
     if(prc) return prc;
+    // a P2G phase has routed this substep's order already: a captured one would do so again
+    if(fast(h) && h->fast.sorted_now) return enqueue_substep(h, dt, time);
     const int par = fast(h) ? h->fast.cur : 0;
     cudaGraphExec_t& ge = h->graphs[par];
     if(!ge) {

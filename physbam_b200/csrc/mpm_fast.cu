@@ -2650,7 +2650,12 @@ int fast_p2g(mpm_handle* h, double dt, double)
         timer_end(h, ps);
         MPM_LAUNCHED(h, "k_penalty_kick");
     }
-    if(repeat) {   // P2G again before a G2P (the phase entry points): its work tickets restart
+    if(repeat) {   // P2G again before a G2P (the phase entry points): work tickets, node blocks and sums restart
+        if(f.grid_dirty) {   // no grid update read the first P2G's sums
+            MPM_CUDA(h, cudaMemsetAsync(f.acc, 0, f.grid_nodes * sizeof(float4), h->stream));
+            MPM_CUDA(h, cudaMemsetAsync(f.nb_flag, 0, f.grid_node_blocks * sizeof(uint32_t), h->stream));
+        }
+        MPM_CUDA(h, cudaMemsetAsync(a.ctr + CNT_NODE_BLOCKS, 0, sizeof(uint32_t), h->stream));
         MPM_CUDA(h, cudaMemsetAsync(a.ctr + CNT_P2G_WORK, 0, sizeof(uint32_t), h->stream));
         MPM_CUDA(h, cudaMemsetAsync(a.ctr + CNT_FALLBACK, 0, 2 * sizeof(uint32_t), h->stream));
     }

@@ -155,3 +155,36 @@ def test_grid_of_the_last_replayed_substep(cuda_device, batch):
         assert ta["mass"] == pytest.approx(tb["mass"], rel=1e-6)
     replayed.close()
     eager.close()
+
+
+def test_fast_phases_repeated(cuda_device):
+    """P2G again before the grid update or after it gives the grid of one P2G, and whole substeps may
+    follow a P2G phase, captured ones among them."""
+    scene = S.small_3d()
+    drv, once = D().MPM_DRIVER(scene), D().MPM_DRIVER(scene)
+    for d in (drv, once):
+        d.set_scene_particles(scene)
+        d.advance(4)                       # both parities captured
+    once.Particle_To_Grid()
+    once.Apply_Forces()
+    want = once.get_grid()
+    once.close()
+    drv.Particle_To_Grid()
+    drv.Particle_To_Grid()
+    drv.Apply_Forces()
+    for again in range(3):
+        got = drv.get_grid()
+        for k in want:
+            assert np.abs(got[k] - want[k]).max() <= 1e-4 * np.abs(want[k]).max(), (again, k)
+        drv.Particle_To_Grid()
+        drv.Apply_Forces()
+    drv.Grid_To_Particle()
+    drv.Particle_To_Grid()
+    drv.advance(4)
+    drv.synchronize()
+    got = drv.get_particles()
+    drv.close()
+    st = oracle.State(scene)
+    oracle.run(st, 9)
+    assert np.abs(got["X"] - st.X).max() <= 2e-6
+    assert np.abs(got["V"] - st.V).max() <= 2e-3 * np.abs(st.V).max()
