@@ -1094,8 +1094,9 @@ __global__ void __launch_bounds__(256) k_grid(FastArgs a)
                 differs = vf[0] != vn[0] || vf[1] != vn[1] || vf[2] != vn[2];
                 o0 = make_float4(vn[0], vn[1], vn[2], vf[0]);
                 o1 = make_float4(vf[1], vf[2], c.w, 0.f);
-                a.acc[q] = make_float4(0, 0, 0, 0);
             }
+            // the force of a massless particle goes to massless nodes too; it is not kept
+            if(c.x != 0.f || c.y != 0.f || c.z != 0.f || c.w != 0.f) a.acc[q] = make_float4(0, 0, 0, 0);
             a.vel[2 * q] = o0;
             a.vel[2 * q + 1] = o1;
             if(a.nb_differs) {                                     // half a node block per warp

@@ -104,6 +104,38 @@ def test_fast_particle_without_mass(cuda_device):
     check(run_gpu(scene, 5, D().FP32, D().PATH_FAST), run_oracle(scene, 5), TOL32)
 
 
+@pytest.mark.parametrize("upload", [False, True])
+def test_fast_force_on_massless_nodes(cuda_device, upload):
+    """The force of a stressed particle of zero mass away from the others is gone with its substep: a
+    body that reaches its nodes later, in the same run or after a re-upload, moves as on the plain path."""
+    scene = pick(S.small_3d(with_walls=False, friction=0.0), 400)
+    scene.X[:] = 0.3 + 0.2 * np.random.default_rng(4).random((scene.n, 3))
+    scene.V[:] = [20.0, 0.0, 0.0]
+    scene.X[-8:] = [0.72, 0.4, 0.4]                # three cells ahead of the body
+    scene.V[-8:] = 0.0
+    scene.mass[-8:] = 0.0
+    scene.F[-8:] = np.diag([0.5, 1.2, 0.9])
+    later = scene.copy()
+    later.X[:-8, 0] += 0.2
+    out = []
+    for precision, path in ((D().FP32, D().PATH_FAST), (D().FP64, D().PATH_PLAIN)):
+        drv = D().MPM_DRIVER(scene, precision=precision, path=path)
+        drv.set_scene_particles(scene)
+        drv.advance(40 if upload else 100)         # short of the massless ones' nodes, or over them
+        if upload:
+            drv.set_scene_particles(later)
+            drv.advance(20)
+        drv.synchronize()
+        out.append(drv.get_particles())
+        drv.close()
+    got, ref = out
+    assert ref["X"][:-8, 0].max() > 0.62           # within a cell and a half of the massless ones
+    # positions: the velocities' tolerance over 100 substeps of 1e-4 (left-over forces: 3e-2)
+    vmax = np.abs(ref["V"]).max()
+    assert np.abs(got["V"] - ref["V"])[:-8].max() <= 2e-3 * vmax
+    assert np.abs(got["X"] - ref["X"])[:-8].max() <= 100 * 1e-4 * 2e-3 * vmax
+
+
 @pytest.mark.parametrize("shape", [(3, 128, 1), (2, 64, 1), (1, 256, 1), (3, 64, 1), (0, 128, 2)])
 def test_fast_many_items_in_two_scenes(cuda_device, shape):
     """Enough work items that G2P streams them (two and more per CTA), blocks of every fill, a
