@@ -791,6 +791,17 @@ __device__ __forceinline__ void factors_from(const FastArgs& a, const SceneDev& 
     for(int o = 0; o < 3; o++) { P.w[o] = wx.w[o]; P.w[3 + o] = wy.w[o]; P.w[6 + o] = wz.w[o]; }
 }
 
+// Whether the mass and the momentum factors are finite (their sum too).
+__device__ __forceinline__ bool finite_factors(float m, const P2GFactors& P)
+{
+    float s = m;
+#pragma unroll
+    for(int r = 0; r < 3; r++)
+#pragma unroll
+        for(int o = 0; o < 3; o++) s += (P.q[r].Hx[o] + P.q[r].Hy[o]) + P.q[r].Hz[o];
+    return isfinite(s);
+}
+
 // i = perm[j], the slot of sorted position j.  Returns the mass.
 __device__ __forceinline__ float particle_factors(const FastArgs& a, const SceneDev& sc, uint32_t j, uint32_t i, P2GFactors& P)
 {
@@ -823,6 +834,13 @@ __device__ __forceinline__ void p2g_fallback_force(const FastArgs& a, uint32_t k
     const float4 at = a.src_attr[i];
     if(!stress_fp64(slot_model(a, sc, i), F, at.z, at.w, S)) atomicOr(a.flags, MPM_FLAG_NOT_CONVERGED);
     const float sv = a.dt * at.y;
+    float total = 0.f;
+#pragma unroll
+    for(int e = 0; e < 9; e++) total += sv * S[e];
+    if(!isfinite(total)) {   // as finite_factors
+        atomicOr(a.flags, MPM_FLAG_NAN);
+        return;
+    }
     const Axis<float> wx = spline_axis<float>(X[0], sc.dmin[0], sc.dx[0], sc.inv[0]);
     const Axis<float> wy = spline_axis<float>(X[1], sc.dmin[1], sc.dx[1], sc.inv[1]);
     const Axis<float> wz = spline_axis<float>(X[2], sc.dmin[2], sc.dx[2], sc.inv[2]);
@@ -983,6 +1001,11 @@ template<int T, int PER, int CTAS> __global__ void __launch_bounds__(T, CTAS) k_
                     row[6 + o] = make_float4(P.q[0].Hz[o], P.q[1].Hz[o], P.q[2].Hz[o], P.w[6 + o]);
                 }
                 *reinterpret_cast<float2*>(row + 9) = make_float2(m, __int_as_float((int)cell[u]));
+                if(!finite_factors(m, P)) {   // reported, and nothing of it goes to the nodes around
+                    atomicOr(a.flags, MPM_FLAG_NAN);
+                    for(int o = 0; o < 9; o++) row[o] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float2*>(row + 9) = make_float2(0.f, __int_as_float((int)cell[u]));
+                }
             }
         }
         if(threadIdx.x == 0) {

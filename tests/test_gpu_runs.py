@@ -136,6 +136,30 @@ def test_fast_force_on_massless_nodes(cuda_device, upload):
     assert np.abs(got["X"] - ref["X"])[:-8].max() <= 100 * 1e-4 * 2e-3 * vmax
 
 
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("field,bad", [("V", np.nan), ("V", np.inf), ("B", -np.inf), ("F", np.nan), ("mass", np.inf),
+                                       ("mass", np.nan), ("V", 1e37)])
+def test_fast_p2g_reports_non_finite(cuda_device, variant, field, bad):
+    """A particle that is not finite, or whose momentum is not, is reported by the P2G phase already
+    and leaves the grid finite."""
+    scene = pick(S.small_3d(), 600)
+    getattr(scene, field)[300] = bad
+    if bad == 1e37:
+        scene.mass[300] = 1e6
+    drv = D().MPM_DRIVER(scene)
+    drv.set_launch_shape(variant, 128, 1)
+    drv.set_scene_particles(scene)
+    drv.Particle_To_Grid()
+    with pytest.raises(D().MPMError) as e:
+        drv.synchronize()
+    assert e.value.code == 3
+    drv.Apply_Forces()
+    grid = drv.get_grid()
+    drv.close()
+    assert (grid["grid_m"] > 0).sum() > 100
+    assert all(np.isfinite(grid[k]).all() for k in grid)
+
+
 @pytest.mark.parametrize("shape", [(3, 128, 1), (2, 64, 1), (1, 256, 1), (3, 64, 1), (0, 128, 2)])
 def test_fast_many_items_in_two_scenes(cuda_device, shape):
     """Enough work items that G2P streams them (two and more per CTA), blocks of every fill, a
