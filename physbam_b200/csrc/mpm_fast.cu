@@ -16,8 +16,8 @@
 //            grid with one float4 reduction per node and run (Particle_To_Grid
 //            l.245-306 with MPM_FINITE_ELEMENTS::Add_Forces folded in).  It marks
 //            the node blocks its block's stencils cover.
-//   grid     one thread per node of the marked node blocks: v = (mv + dt f)/m
-//            + dt g, collision projection and friction (Apply_Forces
+//   grid     one thread per node of the marked node blocks: its sums added and
+//            v = (mv + dt f)/m + dt g in FP64, collision projection and friction (Apply_Forces
 //            l.959-1060); clears the accumulator for the next substep.
 //   g2p      persistent CTAs over the work items: the tile of (v, v_fric) by TMA
 //            (the next item's copy in flight), gather, update F,
@@ -101,7 +101,8 @@ struct FastArgs {
     uint8_t* nb_differs;        // per node block two bytes (its halves): v_fric differs from v_new somewhere (k_grid; null: not asked)
     uint32_t* fallback;   // sorted positions whose stress takes the FP64 route (P2G)
     const CUtensorMap* tmaps;   // per scene: its grid of 8-float nodes as a 4D tensor (G2P tiles)
-    float4* acc;
+    float4* acc;                // P2G's sums: `sums` per node (node_sum)
+    int sums;
     float4* vel;
     const SceneDev* scenes;
     const uint16_t* block_scene;
@@ -815,6 +816,24 @@ __device__ __forceinline__ float particle_factors(const FastArgs& a, const Scene
     return at.x;
 }
 
+// P2G's sums of a node: a.sums float4 (momentum + dt force, mass), by the column of the
+// stencil a contribution comes from (its x offset central or not, its y offset central or
+// not), added up in FP64 by k_grid.  A node receives some 65 run sums in FP32 from all
+// around it; in one float4 their rounding was the largest part of what the run sums lost
+// against a tile of 46-bit integers per item, which left 7 per node.  The central column
+// holds over half of a node's mass in a ninth of its run sums, so apart from the rest both
+// round less.  Error of B against 64 bits, tile / one sum / four sums and the division in
+// FP64: 32^3 box 2.09e-6 / 2.25e-6 / 1.96e-6, spheres 64^3 3.07e-6 / 3.43e-6 / 2.97e-6, 128^3
+// 1.064e-5 / 1.097e-5 / 1.056e-5; V no larger either.  Per call 4.77 -> 4.78 ms
+// (spheres), 8.74 -> 8.82 (128^3 dam break), 10.87 -> 11.11 (256 scenes).  Grids of more than
+// kSplitNodes nodes keep one sum: four of them would take 17 GB and up.
+constexpr int kSums = 4;
+constexpr int64_t kSplitNodes = 1LL << 28;
+__device__ __forceinline__ int64_t node_sum(const FastArgs& a, int64_t node, int i, int j)
+{
+    return a.sums * node + (a.sums > 1 ? 2 * (i != 1) + (j != 1) : 0);
+}
+
 // The elastic force of the particles the P2G kernels listed for the FP64
 // stress route: -dt vol PF^T grad w added to the momentum of their 27 nodes.
 // Their nodes lie in their block's tile, whose node blocks P2G already
@@ -853,7 +872,7 @@ __device__ __forceinline__ void p2g_fallback_force(const FastArgs& a, uint32_t k
 #pragma unroll
                 for(int r = 0; r < 3; r++) f[r] = -sv * (S[r] * g0 + S[r + 3] * g1 + S[r + 6] * g2);
                 const int qx = wx.base + MPM_GHOST + ii, qy = wy.base + MPM_GHOST + jj, qz = wz.base + MPM_GHOST + kk;
-                atomicAdd(&a.acc[node_index(sc, qx, qy, qz)], make_float4(f[0], f[1], f[2], 0.f));
+                atomicAdd(&a.acc[node_sum(a, node_index(sc, qx, qy, qz), ii, jj)], make_float4(f[0], f[1], f[2], 0.f));
             }
 }
 
@@ -907,7 +926,7 @@ __global__ void k_penalty_kick(FastArgs a)
 // per particle, of which the preparation is two thirds, at 24 warps per SM; the
 // factor reads take a quarter of the shared-memory pipe.  It replaced a 6^3
 // fixed-point tile of shared integer atomics (216 per particle, 74 issue slots
-// and seven barriers per item; the float sums here are no further from FP64):
+// and seven barriers per item; for the precision of its sums see node_sum):
 // 540 -> 323 us there, 52 -> 32 us on the 242,752 particles of the spheres.
 // 128 threads and particles per item: 256 and 256 took 348 and 33 us (fewer
 // CTAs to fill each other's barriers), 64 and 64 331 and 33 us.
@@ -1015,8 +1034,8 @@ template<int T, int PER, int CTAS> __global__ void __launch_bounds__(T, CTAS) k_
         __syncthreads();
         if(threadIdx.x == 0) work_prefetch(a, wnext, nwork, S.work[cur]);
         if(lane < 27) {
-            const int sy = S.sc.GA[2], sx = S.sc.GA[1] * S.sc.GA[2];
-            float4* const base = a.acc + node_index(S.sc, 4 * bx + gi, 4 * by + gj, 4 * bz);
+            const int sz = a.sums, sy = sz * S.sc.GA[2], sx = S.sc.GA[1] * sy;
+            float4* const base = a.acc + node_sum(a, node_index(S.sc, 4 * bx + gi, 4 * by + gj, 4 * bz), gi, gj);
             const uint32_t r0 = cnt * (uint32_t)grp / GROUPS, r1 = cnt * (uint32_t)(grp + 1) / GROUPS;
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             float4 A0 = zero, A1 = zero, A2 = zero;
@@ -1031,11 +1050,11 @@ template<int T, int PER, int CTAS> __global__ void __launch_bounds__(T, CTAS) k_
                     if(pc == run + 1 && (pc & 3)) {        // the next cell along z
                         red_add(at, A0);
                         A0 = A1; A1 = A2; A2 = zero;
-                        at++;
+                        at += sz;
                     } else {
-                        if(run >= 0) { red_add(at, A0); red_add(at + 1, A1); red_add(at + 2, A2); }
+                        if(run >= 0) { red_add(at, A0); red_add(at + sz, A1); red_add(at + 2 * sz, A2); }
                         A0 = A1 = A2 = zero;
-                        at = base + (pc >> 4) * sx + ((pc >> 2) & 3) * sy + (pc & 3);
+                        at = base + (pc >> 4) * sx + ((pc >> 2) & 3) * sy + (pc & 3) * sz;
                     }
                     run = pc;
                 }
@@ -1052,7 +1071,7 @@ template<int T, int PER, int CTAS> __global__ void __launch_bounds__(T, CTAS) k_
                 add(A1, z1);
                 add(A2, z2);
             }
-            if(run >= 0) { red_add(at, A0); red_add(at + 1, A1); red_add(at + 2, A2); }
+            if(run >= 0) { red_add(at, A0); red_add(at + sz, A1); red_add(at + 2 * sz, A2); }
         }
         if(nb_prev == 0u) a.nb_list[atomicAdd(&a.ctr[CNT_NODE_BLOCKS], 1u)] = nb;
     }
@@ -1097,12 +1116,24 @@ __global__ void __launch_bounds__(256) k_grid(FastArgs a)
             int nz = lnb % sc.NN[2], r = lnb / sc.NN[2], ny = r % sc.NN[1], nx = r / sc.NN[1];
             int qx = 4 * nx + (t >> 4), qy = 4 * ny + ((t >> 2) & 3), qz = 4 * nz + (t & 3);
             int64_t q = node_index(sc, qx, qy, qz);
-            float4 c = a.acc[q];
+            float4* const sums = a.acc + a.sums * q;
+            double m = 0, P[3] = {0, 0, 0};
+            bool held = false;
+            auto take = [&](const float4& c) {
+                m += c.w; P[0] += c.x; P[1] += c.y; P[2] += c.z;
+                held |= c.x != 0.f || c.y != 0.f || c.z != 0.f || c.w != 0.f;
+            };
+            if(a.sums == kSums) {
+#pragma unroll
+                for(int s = 0; s < kSums; s++) take(sums[s]);
+            } else take(sums[0]);
             float4 o0 = make_float4(0, 0, 0, 0), o1 = make_float4(0, 0, 0, 0);
             bool differs = false;
-            if(c.w != 0.f) {
-                float im = 1.f / c.w;
-                float V[3] = {c.x * im + a.dt * sc.gravity[0], c.y * im + a.dt * sc.gravity[1], c.z * im + a.dt * sc.gravity[2]};
+            if(m != 0) {
+                const double im = 1 / m;
+                float V[3];
+#pragma unroll
+                for(int k = 0; k < 3; k++) V[k] = (float)(P[k] * im + (double)a.dt * sc.gravity[k]);
                 float vn[3], vf[3];
                 if(sc.nobj) {
                     float X0[3] = {sc.dmin[0] + ((float)(qx - MPM_GHOST) + 0.5f) * sc.dx[0],
@@ -1116,10 +1147,11 @@ __global__ void __launch_bounds__(256) k_grid(FastArgs a)
                 }
                 differs = vf[0] != vn[0] || vf[1] != vn[1] || vf[2] != vn[2];
                 o0 = make_float4(vn[0], vn[1], vn[2], vf[0]);
-                o1 = make_float4(vf[1], vf[2], c.w, 0.f);
+                o1 = make_float4(vf[1], vf[2], (float)m, 0.f);
             }
             // the force of a massless particle goes to massless nodes too; it is not kept
-            if(c.x != 0.f || c.y != 0.f || c.z != 0.f || c.w != 0.f) a.acc[q] = make_float4(0, 0, 0, 0);
+            if(held)
+                for(int s = 0; s < a.sums; s++) sums[s] = make_float4(0, 0, 0, 0);
             a.vel[2 * q] = o0;
             a.vel[2 * q + 1] = o1;
             if(a.nb_differs) {                                     // half a node block per warp
@@ -2022,7 +2054,7 @@ FastArgs make_args(mpm_handle* h, double dt)
     a.part = kPartSize[f.route_variant];
     a.chunk_cap = (uint32_t)f.chunk_cap;
     a.nb_flag = f.nb_flag; a.nb_list = f.nb_list; a.nb_differs = f.nb_differs;
-    a.acc = f.acc; a.vel = f.vel;
+    a.acc = f.acc; a.sums = f.sums; a.vel = f.vel;
     a.fallback = f.sort_keys_alt;   // the full sort's ping-pong buffer is free during substeps
     a.tmaps = (const CUtensorMap*)f.tmaps;
     a.scenes = f.scenes; a.block_scene = f.block_scene; a.nb_scene = f.nb_scene; a.pbase = f.pbase;
@@ -2168,9 +2200,10 @@ int fast_setup_scenes(mpm_handle* h, const mpm_scene_desc* descs, int count, con
     f.grid_nodes = nodes;
     f.grid_node_blocks = nblocks;
     f.grid_dirty = false;
-    MPM_ALLOC(h, &f.acc, nodes * sizeof(float4));
+    f.sums = nodes > kSplitNodes ? 1 : kSums;
+    MPM_ALLOC(h, &f.acc, f.sums * nodes * sizeof(float4));
     MPM_ALLOC(h, &f.vel, nodes * 2 * sizeof(float4));
-    MPM_CUDA(h, cudaMemset(f.acc, 0, nodes * sizeof(float4)));
+    MPM_CUDA(h, cudaMemset(f.acc, 0, f.sums * nodes * sizeof(float4)));
     MPM_CUDA(h, cudaMemset(f.vel, 0, nodes * 2 * sizeof(float4)));
     for(int k = 0; k < 2; k++) {
         MPM_ALLOC(h, &f.bstart[k], blocks * sizeof(uint32_t));
@@ -2390,7 +2423,7 @@ int fast_set_particles(mpm_handle* h, const mpm_particles_view* v)
     FastState& f = h->fast;
     int64_t n = v->n;
     if(f.grid_dirty) {   // a P2G without its grid update left mass in the kept accumulator
-        MPM_CUDA(h, cudaMemsetAsync(f.acc, 0, f.grid_nodes * sizeof(float4), h->stream));
+        MPM_CUDA(h, cudaMemsetAsync(f.acc, 0, f.sums * f.grid_nodes * sizeof(float4), h->stream));
         MPM_CUDA(h, cudaMemsetAsync(f.nb_flag, 0, f.grid_node_blocks * sizeof(uint32_t), h->stream));
         f.grid_dirty = false;
     }
@@ -2676,7 +2709,7 @@ int fast_p2g(mpm_handle* h, double dt, double)
     }
     if(repeat) {   // P2G again before a G2P (the phase entry points): work tickets, node blocks and sums restart
         if(f.grid_dirty) {   // no grid update read the first P2G's sums
-            MPM_CUDA(h, cudaMemsetAsync(f.acc, 0, f.grid_nodes * sizeof(float4), h->stream));
+            MPM_CUDA(h, cudaMemsetAsync(f.acc, 0, f.sums * f.grid_nodes * sizeof(float4), h->stream));
             MPM_CUDA(h, cudaMemsetAsync(f.nb_flag, 0, f.grid_node_blocks * sizeof(uint32_t), h->stream));
         }
         MPM_CUDA(h, cudaMemsetAsync(a.ctr + CNT_NODE_BLOCKS, 0, sizeof(uint32_t), h->stream));
@@ -2781,13 +2814,15 @@ template<class S> __global__ void k_add_forces(FastArgs a, const S* f, float dt,
         const int qx = 4 * nx + (t >> 4), qy = 4 * ny + ((t >> 2) & 3), qz = 4 * nz + (t & 3);
         if(qx >= G0 || qy >= G1 || qz >= G2) continue;
         const int64_t q = node_index(sc, qx, qy, qz);
-        float4 c = a.acc[q];
-        if(c.w == 0.f) continue;
+        double m = 0;
+        for(int s = 0; s < a.sums; s++) m += a.acc[a.sums * q + s].w;
+        if(m == 0) continue;
+        float4 c = a.acc[a.sums * q];
         const int64_t o = 3 * (((int64_t)qx * G1 + qy) * G2 + qz);
         c.x += dt * (float)f[o];
         c.y += dt * (float)f[o + 1];
         c.z += dt * (float)f[o + 2];
-        a.acc[q] = c;
+        a.acc[a.sums * q] = c;
     }
 }
 }  // namespace

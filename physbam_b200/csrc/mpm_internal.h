@@ -123,7 +123,8 @@ struct FastState {
     uint32_t* counters = nullptr;             // 2 x 16 words, one set per parity: see FastCounter
     bool grid_marked = false;                 // the last grid update wrote nb_differs (G2P may stream its items)
     int grid_set = 0;                         // counter set of the last grid update (its node blocks)
-    float4* acc = nullptr;                    // P2G accumulator: momentum+dt*force (xyz), mass (w)
+    float4* acc = nullptr;                    // P2G accumulator: momentum+dt*force (xyz), mass (w), `sums` per node
+    int sums = 1;
     float4* vel = nullptr;                    // per node 2 x float4: vnew.xyz, vfric.x | vfric.yz, mass, 0
     float* vkick = nullptr;                   // penalty objects on: 3 * npad floats, V + dt f / m per slot
     uint8_t* pmodel = nullptr;                // constitutive model per caller particle index (null: the scene's)

@@ -190,6 +190,21 @@ def test_fast_many_items_in_two_scenes(cuda_device, shape):
             assert np.abs(g[k] - r[k])[keep].max() <= TOL32[k] * scale, k
 
 
+@pytest.mark.parametrize("ppc", [1, 8])
+def test_fast_grid_of_one_sum_per_node(cuda_device, ppc):
+    """More than 2^28 nodes (P2G keeps one sum per node, not four): a body in the corner of a 660^3
+    grid moves as on a 40^3 grid of the same cells."""
+    scene = S.small_3d(G=40, ppc=ppc, with_walls=False)
+    far = scene.copy()
+    far.counts = [660] * 3
+    far.domain_max = [660 / 40.0] * 3
+    got, ref = (run_gpu(s, 10, D().FP32, D().PATH_FAST) for s in (far, scene))
+    np.testing.assert_array_equal(got["valid"], ref["valid"])
+    vmax = np.abs(ref["V"]).max()
+    for k, scale in (("X", 1.0), ("V", vmax), ("F", 1.0), ("B", vmax / scene.dx)):
+        assert np.abs(got[k] - ref[k]).max() <= TOL32[k] * scale, k
+
+
 def big(scene_fn, **kw):
     """A small body on a 40^3 grid: 46^3 nodes, past the size from which tiles are listed."""
     return scene_fn(G=40, **kw)
