@@ -45,7 +45,7 @@ struct PlainState {
     // flagged tiles and its length.  The grid arrays are zero outside the listed tiles
     // (`grid_listed`); small grids and reflection boundaries run over every node instead.
     uint8_t* tile_flag = nullptr;
-    uint32_t *tiles = nullptr, *tile_count = nullptr;
+    uint32_t *tiles = nullptr, *tile_count = nullptr;   // [0]: the list's length; then k_tile_count's counts
     bool grid_listed = false;
     bool scattered = false;   // the grid holds a P2G of the particles where they are now
     const PlainRecord* record = nullptr;   // set while a rollout's substep is recorded

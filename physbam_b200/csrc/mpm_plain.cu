@@ -43,54 +43,91 @@ template<class T> __global__ void k_clear(PlainArgs<T> a)
     });
 }
 
-// The flagged tiles in tile order, and their number.  A CTA lists kTileSpan
-// tiles; the flags before its own it counts itself (one byte each, 0 or 1, read
-// as 16-byte words), so the list takes one launch and no CTA waits for another.
-constexpr int kTileSpan = 1024, kTileThreads = 256;
-__global__ void __launch_bounds__(kTileThreads) k_tile_list(const uint8_t* flag, int64_t ntiles, uint32_t* tiles, uint32_t* count,
-    uint32_t* rec_tiles, uint32_t* rec_count)   // and the same into a rollout's record, or null
+// The flagged tiles in tile order, and their number.  A CTA lists the spans of
+// kTileSpan tiles that fall to it (`spans`, of `per` each); it finds the number of
+// flagged tiles before them itself, so no CTA waits for another: up to kDirectSpans
+// spans from the flags (one byte each, 0 or 1, read as 16-byte words), in one
+// launch, and past that, where reading them all in every CTA would take longer
+// than anything else of a substep (bytes by the square of the grid), from the
+// counts that k_tile_count left.
+constexpr int kTileSpan = 1024, kTileThreads = 256, kDirectSpans = 128, kTileCtas = 1024;
+
+__device__ __forceinline__ uint32_t count_flags(const uint8_t* flag, int64_t from, int64_t to)   // multiples of 16
+{
+    uint32_t c = 0;
+    const uint4* f16 = reinterpret_cast<const uint4*>(flag);
+    for(int64_t k = from / 16 + threadIdx.x; k < to / 16; k += kTileThreads) {
+        const uint4 v = f16[k];
+        c += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+    }
+    return c;
+}
+
+__device__ __forceinline__ uint32_t tile_block_sum(uint32_t v)
+{
+    __shared__ uint32_t sh[kTileThreads / 32];
+#pragma unroll
+    for(int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t t = 0;
+#pragma unroll
+    for(int w = 0; w < kTileThreads / 32; w++) t += sh[w];
+    return t;
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_tile_count(const uint8_t* flag, int64_t spans, int64_t per, uint32_t* counts)
 {
     chain_begin();
-    __shared__ uint32_t s_warp[kTileThreads / 32], s_before[kTileThreads / 32];
+    const int64_t s0 = blockIdx.x * per, s1 = s0 + per < spans ? s0 + per : spans;
+    const uint32_t c = tile_block_sum(count_flags(flag, s0 * kTileSpan, s1 * kTileSpan));
+    if(threadIdx.x == 0) counts[blockIdx.x] = c;
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_tile_list(const uint8_t* flag, int64_t spans, int64_t per, const uint32_t* counts,
+    uint32_t* tiles, uint32_t* count, uint32_t* rec_tiles, uint32_t* rec_count)   // rec: the same into a rollout's record, or null
+{
+    chain_begin();
+    __shared__ uint32_t s_warp[2][kTileThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t first = (int64_t)blockIdx.x * kTileSpan;
+    const int64_t s0 = blockIdx.x * per, s1 = s0 + per < spans ? s0 + per : spans;
     uint32_t before = 0;
-    const uint4* f16 = reinterpret_cast<const uint4*>(flag);
-    for(int64_t k = threadIdx.x; k < first / 16; k += kTileThreads) {
-        const uint4 v = f16[k];
-        before += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
-    }
-    // this CTA's tiles, four per thread (the flags are padded to whole spans)
-    const uint32_t mine = reinterpret_cast<const uint32_t*>(flag + first)[threadIdx.x];
-    const uint32_t c = __popc(mine);
-    uint32_t x = c;
+    if(counts)
+        for(int k = threadIdx.x; k < (int)blockIdx.x; k += kTileThreads) before += counts[k];
+    else before = count_flags(flag, 0, s0 * kTileSpan);
+    uint32_t base = tile_block_sum(before);
+    for(int64_t s = s0; s < s1; s++) {
+        // this span's tiles, four per thread (the flags are padded to whole spans)
+        const int64_t first = s * kTileSpan;
+        const uint32_t mine = reinterpret_cast<const uint32_t*>(flag + first)[threadIdx.x];
+        const uint32_t c = __popc(mine);
+        uint32_t x = c;
 #pragma unroll
-    for(int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if(lane >= o) x += y;
-    }
-#pragma unroll
-    for(int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-    if(lane == 31) s_warp[warp] = x;
-    if(lane == 0) s_before[warp] = before;
-    __syncthreads();
-    uint32_t at = x - c, total = 0;
-#pragma unroll
-    for(int w = 0; w < kTileThreads / 32; w++) {
-        at += s_before[w] + (w < warp ? s_warp[w] : 0u);
-        total += s_before[w] + s_warp[w];
-    }
-#pragma unroll
-    for(int k = 0; k < 4; k++)
-        if((mine >> (8 * k)) & 1u) {
-            const uint32_t t = (uint32_t)(first + 4 * threadIdx.x + k);
-            tiles[at] = t;
-            if(rec_tiles) rec_tiles[at] = t;
-            at++;
+        for(int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if(lane >= o) x += y;
         }
+        uint32_t* sums = s_warp[s & 1];
+        if(lane == 31) sums[warp] = x;
+        __syncthreads();
+        uint32_t at = base + x - c;
+#pragma unroll
+        for(int w = 0; w < kTileThreads / 32; w++) {
+            if(w < warp) at += sums[w];
+            base += sums[w];
+        }
+#pragma unroll
+        for(int k = 0; k < 4; k++)
+            if((mine >> (8 * k)) & 1u) {
+                const uint32_t t = (uint32_t)(first + 4 * threadIdx.x + k);
+                tiles[at] = t;
+                if(rec_tiles) rec_tiles[at] = t;
+                at++;
+            }
+    }
     if(blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-        *count = total;
-        if(rec_count) *rec_count = total;
+        *count = base;
+        if(rec_count) *rec_count = base;
     }
 }
 
@@ -620,11 +657,16 @@ template<class T> int p2g_t(mpm_handle* h, double dt, bool with_forces)
         MPM_LAUNCHED(h, "k_p2g");
     }
     if(a.tile_flag) {
-        const int64_t nt = (a.gn + kTileNodes - 1) / kTileNodes;
+        const int64_t nt = (a.gn + kTileNodes - 1) / kTileNodes, spans = (nt + kTileSpan - 1) / kTileSpan;
+        const bool direct = spans <= kDirectSpans;
+        const int64_t per = direct ? 1 : (spans + kTileCtas - 1) / kTileCtas;
+        const unsigned ctas = (unsigned)((spans + per - 1) / per);
+        uint32_t* counts = direct ? nullptr : h->plain.tile_count + 1;
         slot = timer_begin(h, "plain_tiles");
         const PlainRecord* r = h->plain.record;
-        launch_chained(k_tile_list, (unsigned)((nt + kTileSpan - 1) / kTileSpan), kTileThreads, 0, h->stream,
-            a.tile_flag, nt, h->plain.tiles, h->plain.tile_count, r ? r->tiles : nullptr, r ? r->tile_count : nullptr);
+        if(!direct) launch_chained(k_tile_count, ctas, kTileThreads, 0, h->stream, a.tile_flag, spans, per, counts);
+        launch_chained(k_tile_list, ctas, kTileThreads, 0, h->stream, a.tile_flag, spans, per, counts, h->plain.tiles,
+            h->plain.tile_count, r ? r->tiles : nullptr, r ? r->tile_count : nullptr);
         timer_end(h, slot);
         MPM_LAUNCHED(h, "k_tile_list");
     }
@@ -968,7 +1010,7 @@ static int plain_alloc_buffers(mpm_handle* h, int64_t n)
             const int64_t nt = (gn + kTileNodes - 1) / kTileNodes, span = (nt + kTileSpan - 1) / kTileSpan * kTileSpan;
             MPM_ALLOC(h, &s.tile_flag, span);
             MPM_ALLOC(h, &s.tiles, nt * sizeof(uint32_t));
-            MPM_ALLOC(h, &s.tile_count, sizeof(uint32_t));
+            MPM_ALLOC(h, &s.tile_count, (1 + kTileCtas) * sizeof(uint32_t));
             // an empty list: node passes may come before the first P2G (the phase entry points)
             MPM_CUDA(h, cudaMemsetAsync(s.tile_flag, 0, span, h->stream));
             MPM_CUDA(h, cudaMemsetAsync(s.tile_count, 0, sizeof(uint32_t), h->stream));

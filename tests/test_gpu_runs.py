@@ -216,6 +216,27 @@ def test_plain_listed_tiles(cuda_device, n):
     check(run_gpu(scene, 10, D().FP64, D().PATH_PLAIN), run_oracle(scene, 10), TOL64)
 
 
+@pytest.mark.parametrize("G", [156, 164, 330])
+def test_plain_tile_list_of_large_grids(cuda_device, G):
+    """The list of touched tiles around the sizes where it takes a count first (128 spans of 32,768 nodes)
+    and where a CTA takes several spans (1,024): bodies in the low and the high corner of the grid
+    move as on a small grid of the same cells."""
+    scene = S.small_3d(G=24, ppc=2, with_walls=False)
+    ref = run_gpu(scene, 5, D().FP64, D().PATH_PLAIN)
+    grid = scene.copy()
+    grid.counts, grid.domain_max = [G] * 3, [G / 24.0] * 3
+    grid = grid.subset(np.tile(np.arange(scene.n), 2))
+    shift = (G - 24) // 8 * 8 / 24.0                 # whole cells, exact in binary
+    grid.X[scene.n:] += shift
+    got = run_gpu(grid, 5, D().FP64, D().PATH_PLAIN)
+    # a position is rounded at the size of the shift, and B divides that by dx twice
+    eps, vmax = 2.0 ** -52 * (1 + shift), np.abs(ref["V"]).max()
+    for body in (0, 1):
+        part = slice(body * scene.n, (body + 1) * scene.n)
+        assert np.abs(got["X"][part] - body * shift - ref["X"]).max() <= 100 * eps
+        assert np.abs(got["V"][part] - ref["V"]).max() <= 1e-9 * vmax
+
+
 def test_plain_node_passes_before_p2g(cuda_device):
     """The phase entry points in any order: node passes before the first P2G find an empty tile
     list; forces of particles that have moved since the last P2G leave nothing on the grid for
