@@ -41,8 +41,8 @@ struct PlainState {
     void *mass = nullptr, *vol = nullptr, *mu = nullptr, *lam = nullptr, *pft = nullptr;
     uint8_t* valid = nullptr;
     void *gm = nullptr, *gmv = nullptr, *gv0 = nullptr, *gf = nullptr, *gv = nullptr, *gvf = nullptr;
-    // the nodes of the last P2G, in tiles of 32 consecutive ones: a flag per tile, the list of
-    // flagged tiles and its length.  The grid arrays are zero outside the listed tiles
+    // the nodes of the last P2G (and the one before), in tiles of 32 consecutive ones: a flag per
+    // tile, the list of flagged tiles and its length.  The grid arrays are zero outside the listed tiles
     // (`grid_listed`); small grids and reflection boundaries run over every node instead.
     uint8_t* tile_flag = nullptr;
     uint32_t *tiles = nullptr, *tile_count = nullptr;   // [0]: the list's length; then k_tile_count's counts

@@ -267,6 +267,18 @@ def test_plain_node_passes_before_p2g(cuda_device):
         np.testing.assert_allclose(grids[1][k], grids[0][k], rtol=0, atol=1e-12 * np.abs(grids[0][k]).max())
 
 
+def test_plain_tiles_of_moving_bodies(cuda_device):
+    """Two bodies, their particles in no order, that part and on their way cross several tiles and
+    leave others (up to five cells per axis)."""
+    scene = pick(big(S.small_3d, ppc=2, with_walls=False), 1500)
+    half = scene.n // 2
+    scene.X[:, 0] = 0.24 + 0.4 * (scene.X[:, 0] - 0.2)
+    scene.X[:half, 0] += 0.36                          # 0.24 to 0.4, and 0.6 to 0.76
+    scene.V[:half] = [30.0, 10.0, 20.0]
+    scene.V[half:] = [-30.0, 10.0, -20.0]
+    check(run_gpu(scene, 40, D().FP64, D().PATH_PLAIN), run_oracle(scene, 40), TOL64)
+
+
 def test_implicit_listed_tiles(cuda_device):
     """On a grid with listed tiles, over a sticking floor: the solve agrees with itself to the
     Newton tolerance and, at a small step, with the explicit substep.  Backward and symplectic
