@@ -198,3 +198,51 @@ def test_adjoint_differentiable_config_with_walls_fd(cuda_device):
     s.objects = S.walls(3, s.counts, s.domain_min, s.domain_max, 63, S.SLIP, 0.0, 0.05) + [
         S.CollisionObject(S.PLANE, S.SLIP, 0.0, [-1.0, 0.0, 0.0], [0.653, 0.5, 0.5])]
     check_case(s, 64, 8, check_E=False)
+
+
+def test_repeated_rollouts_follow_their_inputs(cuda_device):
+    """A rollout of a shape seen before is replayed from captured passes: what changes between two of
+    them (the step, the objects, the particles and their number, the tape, substeps in between) is in
+    the next one's state and gradient, as on a handle of its own."""
+    import torch
+    from physbam_b200 import driver as D
+    scene = S.small_3d(G=16, ppc=2, with_walls=False)
+    walls = S.walls(3, scene.counts, scene.domain_min, scene.domain_max, 63, S.SLIP, 0.0, 0.2)
+    few = np.arange(scene.n - 40)
+
+    def rollout(drv, s, dt):
+        drv.set_scene_particles(s)
+        drv.diff_forward(6, 2, dt=dt)
+        X = drv.get_particles()["X"]
+        rng = np.random.default_rng(5)
+        g = [torch.tensor(rng.standard_normal((s.n, k)), device="cuda") for k in (3, 3, 9, 9)]
+        return [X] + [t.cpu().numpy() for t in drv.diff_backward(*g)]
+
+    moved = scene.copy()
+    moved.X += 0.01
+    moved.mu *= 1.5
+    drv = D.MPM_DRIVER(scene, precision=D.FP64, path=D.PATH_PLAIN)
+    objects = []
+    steps = [(scene, 1e-4), (scene, 1e-4), (scene, 1e-4), (moved, 1e-4), (scene, 2e-4), (scene, 2e-4), "walls",
+             (scene, 2e-4), (scene, 2e-4), (scene.subset(few), 2e-4), (scene, 2e-4), "advance", (scene, 2e-4), "segments",
+             (scene, 2e-4), (moved, 2e-4), "timing", (scene, 2e-4)]
+    for step in steps:
+        if step == "walls":
+            objects = walls
+            drv.set_collision_objects(objects)
+        elif step == "advance":
+            drv.advance(3, 1e-4)
+        elif step == "segments":
+            drv.set_diff_tape_budget(0)
+        elif step == "timing":
+            drv.set_timing(True)
+        else:
+            s, dt = step
+            alone = D.MPM_DRIVER(s, precision=D.FP64, path=D.PATH_PLAIN)
+            alone.set_collision_objects(objects)
+            want = rollout(alone, s, dt)
+            alone.close()
+            got = rollout(drv, s, dt)
+            for a, b in zip(got, want):
+                assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max()
+    drv.close()

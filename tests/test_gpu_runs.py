@@ -205,6 +205,31 @@ def test_fast_grid_of_one_sum_per_node(cuda_device, ppc):
         assert np.abs(got[k] - ref[k]).max() <= TOL32[k] * scale, k
 
 
+@pytest.mark.parametrize("G", [16, 40])
+def test_plain_captured_substeps_after_upload(cuda_device, G):
+    """Captured substeps kept over an upload of as many particles run on the new ones; an upload of
+    another number, new objects and another step are captured anew."""
+    scene = S.small_3d(G=G, ppc=2)
+    other = scene.copy()
+    other.X += 0.01
+    other.V *= -0.5
+    other.mu *= 2.0
+    few = other.subset(np.arange(other.n - 50))
+    bare = scene.copy()
+    bare.objects = []
+    drv = D().MPM_DRIVER(scene, precision=D().FP64, path=D().PATH_PLAIN)
+    for s, steps, dt in ((scene, 4, 1e-4), (other, 4, 1e-4), (few, 4, 1e-4), (scene, 3, 5e-5), (bare, 3, 5e-5)):
+        if s is bare:
+            drv.set_collision_objects([])
+        drv.set_scene_particles(s)
+        drv.advance(steps, dt)
+        drv.synchronize()
+        ref = s.copy()
+        ref.dt = dt
+        check(drv.get_particles(), run_oracle(ref, steps), TOL64)
+    drv.close()
+
+
 def big(scene_fn, **kw):
     """A small body on a 40^3 grid: 46^3 nodes, past the size from which tiles are listed."""
     return scene_fn(G=40, **kw)
