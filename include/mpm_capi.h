@@ -554,11 +554,14 @@ int mpm_debug_sort_state(mpm_handle* h, uint32_t* slot_keys, uint32_t* sorted_ke
  * current device (default 64); a particle whose SVD does not converge within
  * the bound sets MPM_ERR_NOT_CONVERGED.
  * mpm_debug_fail_allocation makes the handle's which-th device allocation from
- * now report MPM_ERR_NOMEM (0: none). */
+ * now report MPM_ERR_NOMEM (0: none).  mpm_debug_g2p_streamed tells whether the
+ * last substep enqueued or captured on a fast-path handle streams its work items
+ * through G2P. */
 int mpm_debug_sort_stall(const uint32_t* keys, int64_t n, int bits, uint32_t spin_limit);
 int mpm_debug_set_sort_epoch(mpm_handle* h, uint32_t epoch);
 int mpm_debug_set_svd_iterations(int max_it);
 int mpm_debug_fail_allocation(mpm_handle* h, int which);
+int mpm_debug_g2p_streamed(mpm_handle* h, int* streamed);
 
 /* Human-readable text of the last error on this handle / of a status code. */
 int mpm_last_error(mpm_handle* h, char* buf, int len);

@@ -660,6 +660,14 @@ int mpm_debug_fail_allocation(mpm_handle* h, int which)
     return MPM_OK;
 }
 
+int mpm_debug_g2p_streamed(mpm_handle* h, int* streamed)
+{
+    if(!h || !streamed) return MPM_ERR_ARG;
+    if(!fast(h)) return set_error(h, MPM_ERR_ARG, "work items exist on the fast path only");
+    *streamed = h->fast.grid_marked ? 1 : 0;
+    return MPM_OK;
+}
+
 int mpm_debug_set_svd_iterations(int max_it)
 {
     if(max_it < 0 || max_it > 1000000) return MPM_ERR_ARG;

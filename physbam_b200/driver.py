@@ -127,7 +127,8 @@ EXPORTS = ["mpm_create", "mpm_destroy", "mpm_set_stream", "mpm_set_collision_obj
            "mpm_get_implicit_stats", "mpm_set_dt_control", "mpm_simulate_frame", "mpm_last_dt",
            "mpm_set_reflection", "mpm_set_penalty_objects", "mpm_set_object_motion", "mpm_set_particle_models",
            "mpm_set_plastic_particles", "mpm_batch_get_grid", "mpm_debug_sort_stall", "mpm_debug_set_sort_epoch",
-           "mpm_debug_set_svd_iterations", "mpm_debug_fail_allocation", "mpm_add_grid_forces"]
+           "mpm_debug_set_svd_iterations", "mpm_debug_fail_allocation", "mpm_debug_g2p_streamed",
+           "mpm_add_grid_forces"]
 
 _lib = None
 
@@ -158,6 +159,7 @@ def load_library(path: str = LIB_PATH):
     L.mpm_debug_set_sort_epoch.argtypes = [P, ctypes.c_uint32]
     L.mpm_debug_set_svd_iterations.argtypes = [ctypes.c_int]
     L.mpm_debug_fail_allocation.argtypes = [P, ctypes.c_int]
+    L.mpm_debug_g2p_streamed.argtypes = [P, ctypes.POINTER(ctypes.c_int)]
     L.mpm_add_grid_forces.argtypes = [P, ctypes.c_double, P, ctypes.c_int, ctypes.c_int]
     L.mpm_count_valid.argtypes = [P, ctypes.POINTER(ctypes.c_int64)]
     L.mpm_set_timing.argtypes = [P, ctypes.c_int]

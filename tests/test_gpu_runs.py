@@ -11,6 +11,8 @@ sizes where they can go wrong, against the C oracle.
 Tolerances: FP64 sums of at most 27 x 60 terms in another order, some 1e-13 of the largest
 value, over ten substeps; FP32 as in test_gpu_parity.py.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -160,7 +162,7 @@ def test_fast_p2g_reports_non_finite(cuda_device, variant, field, bad):
     assert all(np.isfinite(grid[k]).all() for k in grid)
 
 
-@pytest.mark.parametrize("shape", [(3, 128, 1), (2, 64, 1), (1, 256, 1), (3, 64, 1), (0, 128, 2)])
+@pytest.mark.parametrize("shape", [(3, 128, 1), (2, 64, 1), (1, 256, 1), (3, 64, 1), (3, 128, 2), (0, 128, 1)])
 def test_fast_many_items_in_two_scenes(cuda_device, shape):
     """Enough work items that G2P streams them (two and more per CTA), blocks of every fill, a
     scene change on the way, walls with friction, particles that leave the domain: against the
@@ -170,12 +172,14 @@ def test_fast_many_items_in_two_scenes(cuda_device, shape):
     scenes[1] = scenes[1].subset(np.flatnonzero(keep))
     scenes[1].X[:50] = 1.0 - 1e-6
     scenes[1].V[:50] = 10.0
-    assert sum(s.n for s in scenes) > 2 * 2 * 592 * 128
     drv = D().MPM_BATCH(scenes)
     drv.set_launch_shape(*shape)
     drv.set_scene_particles()
     drv.advance(4, 1e-5)
     drv.synchronize()
+    streamed = ctypes.c_int()
+    drv._check(drv.L.mpm_debug_g2p_streamed(drv.h, ctypes.byref(streamed)), "mpm_debug_g2p_streamed")
+    assert streamed.value == 1
     got = drv.split(drv.get_particles())
     drv.close()
     for s, g in zip(scenes, got):
