@@ -2738,7 +2738,9 @@ static const void* g2p_stream_kernel(int threads)
 // 32^3 box (108 items for 592 CTAs) has nothing to prefetch and took 2 % longer per
 // call, the spheres (3.2 per CTA) 2 % less, the 128^3 dam break 11 %.  Not with
 // plasticity, whose items differ in cost: drawn three ahead they leave a longer tail
-// (snow and sand 6 % slower per call).
+// (snow and sand 6 % slower per call).  The host knows the particles, not the items:
+// where blocks are sparse there are more of them than n / part, and some scenes that
+// could stream do not.
 static bool g2p_streams(mpm_handle* h, const FastArgs& a)
 {
     const FastState& f = h->fast;

@@ -54,9 +54,13 @@ template<class T, class FN> __device__ __forceinline__ void for_nodes(const Plai
 }
 
 // Grids of this many nodes and more are passed over by the list of tiles that
-// P2G touched.  64^2 grid (4,900 nodes): every node is the faster way, one
-// launch less; 64^3 (343,000): the list is.
-constexpr int64_t kListedGrid = 1 << 16;
+// P2G touched, which costs a launch and the flags.  Every node / the list, ms per call: 2D
+// block, 100 substeps, 4,900 nodes 1.74 / 1.94, 39,204 1.87 / 2.15, 68,644 1.95 / 2.16;
+// plain FP64 spheres, 64 substeps, 54,872 nodes 2.87 / 2.92, 74,088 2.97 / 3.01, 97,336 3.12
+// / 3.09, 157,464 3.52 / 3.35, 343,000 5.6 / 4.65, 1,061,208 14.0 / 9.5; implicit substep 74,088
+// 2.66 / 2.55, 343,000 3.32 / 3.07.  The line goes by the grid's size alone: bodies that
+// fill the grid gain nothing from the list and pay 2 to 3 % for it (44^3 to 64^3).
+constexpr int64_t kListedGrid = 90000;
 
 inline bool list_tiles(const mpm_handle* h) { return !h->reflect.enabled && h->plain.gn >= kListedGrid; }
 
