@@ -1118,15 +1118,16 @@ __global__ void __launch_bounds__(256) k_grid(FastArgs a)
             int64_t q = node_index(sc, qx, qy, qz);
             float4* const sums = a.acc + a.sums * q;
             double m = 0, P[3] = {0, 0, 0};
-            bool held = false;
-            auto take = [&](const float4& c) {
+            unsigned held = 0;                    // bit s: sum s is not zero
+            auto take = [&](int s) {
+                const float4 c = sums[s];
                 m += c.w; P[0] += c.x; P[1] += c.y; P[2] += c.z;
-                held |= c.x != 0.f || c.y != 0.f || c.z != 0.f || c.w != 0.f;
+                held |= (c.x != 0.f || c.y != 0.f || c.z != 0.f || c.w != 0.f ? 1u : 0u) << s;
             };
             if(a.sums == kSums) {
 #pragma unroll
-                for(int s = 0; s < kSums; s++) take(sums[s]);
-            } else take(sums[0]);
+                for(int s = 0; s < kSums; s++) take(s);
+            } else take(0);
             float4 o0 = make_float4(0, 0, 0, 0), o1 = make_float4(0, 0, 0, 0);
             bool differs = false;
             if(m != 0) {
@@ -1150,8 +1151,9 @@ __global__ void __launch_bounds__(256) k_grid(FastArgs a)
                 o1 = make_float4(vf[1], vf[2], (float)m, 0.f);
             }
             // the force of a massless particle goes to massless nodes too; it is not kept
-            if(held)
-                for(int s = 0; s < a.sums; s++) sums[s] = make_float4(0, 0, 0, 0);
+#pragma unroll
+            for(int s = 0; s < kSums; s++)
+                if((held >> s) & 1u) sums[s] = make_float4(0, 0, 0, 0);
             a.vel[2 * q] = o0;
             a.vel[2 * q + 1] = o1;
             if(a.nb_differs) {                                     // half a node block per warp
