@@ -922,12 +922,13 @@ __global__ void k_penalty_kick(FastArgs a)
 // particles share theirs, and CTA barriers only order the binning and the
 // factors (two per item).
 //
-// What bounds it (4.33 M particles, 128^3 dam break, corotated): 36 issue slots
-// per particle, of which the preparation is two thirds, at 24 warps per SM; the
-// factor reads take a quarter of the shared-memory pipe.  It replaced a 6^3
-// fixed-point tile of shared integer atomics (216 per particle, 74 issue slots
-// and seven barriers per item; for the precision of its sums see node_sum):
-// 540 -> 323 us there, 52 -> 32 us on the 242,752 particles of the spheres.
+// What bounds it (4.33 M particles, 128^3 dam break, corotated, under ncu): the LSU data
+// path (80 % of its peak: the factor reads and the reductions), with 52 warp
+// instructions per particle and two thirds of the issue slots taken at 24 warps per SM;
+// on the 242,752 particles of the spheres, three items per CTA, latency (LSU 49 %, issue
+// 47 %).  It replaced a 6^3 fixed-point tile of shared integer atomics (216 per particle,
+// seven barriers per item; for the precision of its sums see node_sum): 540 -> 311 us
+// and 52 -> 31 us.
 // 128 threads and particles per item: 256 and 256 took 348 and 33 us (fewer
 // CTAs to fill each other's barriers), 64 and 64 331 and 33 us.
 // ---------------------------------------------------------------------------
@@ -1747,7 +1748,8 @@ __device__ __forceinline__ uint32_t g2p_differs(const FastArgs& a, const SceneDe
 // fetched one ahead.  One barrier per item orders all of it (an item's move counts
 // alternate between two rows, so that they can be flushed behind the barrier).
 // 128^3 dam break (4.33 M particles) 9.77 -> 8.71 ms per call of 12 substeps, 256
-// scenes 11.91 -> 10.84 (8 substeps), the spheres 4.83 -> 4.74 (64).
+// scenes 11.91 -> 10.84 (8 substeps), the spheres 4.83 -> 4.74 (64), with one sum per node
+// in P2G on both sides.
 template<int THREADS> __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_g2p_stream(FastArgs a)
 {
     chain_begin();
@@ -3260,7 +3262,8 @@ __global__ void k_particle_totals(FastArgs a, double* acc, unsigned long long* m
 // Compute_Dt's bound alone: max |V| + |B| 6 sqrt(d) / dx, the max_affine_speed of
 // the totals.  Those sum eleven more values with an atomic per warp each: 165 us of a
 // 290 us adaptive substep at 444,528 particles; a maximum per CTA instead, this pass
-// reads 13 floats per particle, and the frame of 25 such substeps takes 3.1 ms, not 6.9.
+// reads 13 floats per particle in 15 us, and a frame of 20 such substeps takes 2.7 ms, not
+// 6.9.
 __global__ void __launch_bounds__(256) k_affine_speed(FastArgs a, unsigned long long* state, double* host)
 {
     double amax = 0;

@@ -10,8 +10,9 @@
 // with NEWTONS_METHOD's default flags as MPM_DRIVER sets them.  The device
 // does every grid and particle pass (the force and Hessian scatters are those
 // of MPM_FINITE_ELEMENTS, Add_Forces / Add_Hessian_Times, l.84-132); the host
-// runs the Newton / CG / line-search control flow, reading back one or two
-// reduced scalars per step (deterministic two-stage reductions in FP64).  The
+// runs the Newton / CG / line-search control flow, reading back the up to three
+// sums of an evaluation or the two of a CG iteration (FP64, in a fixed order, in the
+// launch that forms their terms: grid_sum).  The
 // node passes visit the tiles of the grid that P2G touched.
 //
 // Collision objects are the static boxes, planes and spheres of the explicit
