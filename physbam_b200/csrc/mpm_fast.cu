@@ -818,8 +818,8 @@ __device__ __forceinline__ float particle_factors(const FastArgs& a, const Scene
 
 // P2G's sums of a node: a.sums float4 (momentum + dt force, mass), by the column of the
 // stencil a contribution comes from (its x offset central or not, its y offset central or
-// not), added up in FP64 by k_grid.  A node receives some 65 run sums in FP32 from all
-// around it; in one float4 their rounding was the largest part of what the run sums lost
+// not), added up in FP64 by k_grid.  At 8 particles per cell and items of 128 a node
+// receives some 65 run sums in FP32 from all around it; in one float4 their rounding was the largest part of what the run sums lost
 // against a tile of 46-bit integers per item, which left 7 per node.  The central column
 // holds over half of a node's mass in a ninth of its run sums, so apart from the rest both
 // round less.  Error of B against 64 bits, tile / one sum / four sums and the division in

@@ -321,8 +321,8 @@ template<class T, int d> __device__ __forceinline__ void keep_particle(const Pla
 //   sum w v_fric (Z - X)^T + dt/2 [sum w (v_fric v^T - v v_fric^T) - (V_fric V^T - V V_fric^T)],
 // equal to it and without the cancellation of terms in Z against terms in X.
 // FP64, 242,752 particles (8 substeps): 2.38 -> 2.21 ms per call; errors against the
-// formulas in plain FP64 100 times smaller in FP64 (1.8e-12 -> 1.5e-14), unchanged in an FP32
-// gradient (2.9e-6, 2.8e-6).
+// formulas in plain FP64 100 times smaller in FP64 (1.8e-12 -> 1.5e-14); an FP32 gradient's is set
+// by entries at cell boundaries (2.9e-6 and 2.8e-6 on one state, 3.2e-4 and 9.2e-6 on another).
 template<class T, int d> __global__ void k_g2p(PlainArgs<T> a)
 {
     chain_begin();
